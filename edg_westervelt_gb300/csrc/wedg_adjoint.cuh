@@ -45,7 +45,7 @@ struct AdjArgs {
   AdjIO A;
   double *gc2, *gal, *gbe;
 };
-using MultiAdj = Multi<AdjArgs, 28>;
+using MultiAdj = Multi<AdjArgs, 19>;
 
 // The weighted slot sums of an interior face point, from the scaled slot weights of the "+"
 // element (hP: A, D, F) and of the "-" element (hM), with c² and α of both sides (a continuous
@@ -186,7 +186,8 @@ __device__ __forceinline__ void adj_mass_body(const Basis<NU, NV> &B, const Fiel
     }
   }
   __syncwarp(tmask);
-  team_K<NU, NV, 1>(B, F, Eu, e, u, tmask, Phs, PhWs, xs, zs, zd, acc);
+  team_K<NU, NV, 1>(B, [&](int r, int s2) { return F.G[(r + QH * s2) * Eu + e]; }, u, tmask, Phs, PhWs, xs, zs, zd,
+                    acc);
 #pragma unroll
   for (int j = 0; j < J; ++j) {
     const int k = u + U * j;

@@ -407,8 +407,8 @@ void drain_events(wedg_ws *ws) {
 int enqueue_stage(wedg_ws *ws, const StageIO &S, const Fields *Fo = nullptr, cudaEvent_t after_stage = nullptr,
                   bool prep_done = false) {
   const Fields &F = Fo ? *Fo : ws->F;
-  const int tp = ws->prep_threads, bp = (ws->E + tp - 1) / tp;
-  const int ts = stage_threads(ws->nu, ws->nv, ws->fast), bs = (ws->E + ts - 1) / ts;
+  const int tp = ws->prep_threads, ep = prep_tile(ws->nu, tp), bp = (ws->E + ep - 1) / ep;
+  const int ts = STAGE_THREADS, tile = stage_tile(ws->nu), bs = (ws->E + tile - 1) / tile;
   const int bm = 1;   // the mass kernels size their own grid
   StageIO Sp = S;
   Sp.parity = ws->parity;
@@ -419,6 +419,7 @@ int enqueue_stage(wedg_ws *ws, const StageIO &S, const Fields *Fo = nullptr, cud
     cudaEventRecord(e0, ws->stream);
   }
   if (!prep_done) CK(ws, ws->L.prep(ws->basis.data(), F, Sp, bp, tp, ws->stream, 0));
+  CK(ws, ws->L.bnd(ws->basis.data(), F, Sp, 1, BND_THREADS, ws->stream));
   if (ws->timing) cudaEventRecord(e1, ws->stream);
   CK(ws, ws->L.stage(ws->basis.data(), F, Sp, bs, ts, ws->stream));
   if (after_stage) CK(ws, cudaEventRecord(after_stage, ws->stream));
@@ -428,7 +429,7 @@ int enqueue_stage(wedg_ws *ws, const StageIO &S, const Fields *Fo = nullptr, cud
     cudaEventRecord(e3, ws->stream);
     ws->ev_pending.push_back({e0, e1, e2, e3});
   }
-  ws->stats.kernel_launches += prep_done ? 2 : 3;
+  ws->stats.kernel_launches += prep_done ? 3 : 4;
   ws->stats.element_stages += ws->E;
   CK(ws, cudaGetLastError());
   return WEDG_OK;
@@ -539,7 +540,7 @@ int adjoint_buffers(wedg_ws *ws) {
 // the per-element coefficients are added to it.
 int enqueue_adjoint_core(wedg_ws *ws, const Fields &Fs, const StageIO &S, const double *lam_u, const double *lam_v,
                          double *gu, double *gv, double *gpar) {
-  const int ts = stage_threads(ws->nu, ws->nv, ws->fast), bs = (ws->E + ts - 1) / ts;
+  const int ts = STAGE_THREADS, tile = stage_tile(ws->nu), bs = (ws->E + tile - 1) / tile;
   // μ = M(v)⁻¹ λ_v, on the Chebyshev data of the state
   Fields Fm = Fs;
   Fm.mrhs = const_cast<double *>(lam_v);
@@ -604,7 +605,7 @@ Fields kept_fields(const wedg_ws *ws, const wedg_ws::StageData &d) {
 // bytes of the kept data of one stage
 size_t stage_data_bytes(const wedg_ws *ws) {
   const size_t E = ws->E;
-  return sizeof(double) * E * ((size_t)ws->nu * ws->nu + ws->nv * ws->nv + 12 * ws->nq + ws->qh * ws->qh + 2) +
+  return sizeof(double) * E * ((size_t)ws->nu * ws->nu + ws->nv * ws->nv + 12 * ws->nq + ws->qh * ws->qh + 4) +
          sizeof(int) * (E * (1 + NBIN) + 2 * NBIN + 4);
 }
 
@@ -673,15 +674,18 @@ int argument_error(wedg_ws *ws, const std::string &msg) {
 }
 
 // ---- multi-instance launches of one kernel over many instances' arguments, in chunks of the
-//      launch's capacity (wedg_kernels.cuh); kind 0: k_prep (tile = threads), 1: k_stage
-//      (tile = stage_threads), 2: the mass solve (tile = teams of `threads`). grid_of maps the
-//      virtual blocks of a chunk to its physical grid (persistent launches).
-enum { MK_PREP = 0, MK_STAGE = 1, MK_MASS = 2 };
+//      launch's capacity (wedg_kernels.cuh): k_prep (tile = prep_tile), k_bnd (tile = bnd_tile of the
+//      4N sides), k_stage (tile = stage_tile), the mass solve (tile = teams of `threads`). grid_of
+//      maps the virtual blocks of a chunk to its physical grid (persistent launches).
+enum { MK_PREP = 0, MK_BND = 1, MK_STAGE = 2, MK_MASS = 3 };
 template <class GridOf>
 cudaError_t multi_stage_launch(const Launchers &L, const void *basis, int nu, int nv, bool fast, int kind,
                                const std::vector<StageArgs> &args, int threads, cudaStream_t st, GridOf grid_of) {
   const int TPW = 32 / (qhigh(nu, nv) / 2 + (qhigh(nu, nv) & 1));
-  const int tile = kind == MK_PREP ? threads : kind == MK_STAGE ? stage_threads(nu, nv, fast) : (threads / 32) * TPW;
+  const int tile = kind == MK_PREP    ? prep_tile(nu, threads)
+                   : kind == MK_BND   ? bnd_tile(nu)
+                   : kind == MK_STAGE ? stage_tile(nu)
+                                      : (threads / 32) * TPW;
   const int n = (int)args.size();
   for (int c0 = 0; c0 < n; c0 += MultiStage::cap) {
     const int m = std::min(n - c0, MultiStage::cap);
@@ -691,11 +695,12 @@ cudaError_t multi_stage_launch(const Launchers &L, const void *basis, int nu, in
     P.first[0] = 0;
     for (int x = 0; x < m; ++x) {
       P.a[x] = args[c0 + x];
-      P.first[x + 1] = P.first[x] + (P.a[x].F.E + tile - 1) / tile;
+      P.first[x + 1] = P.first[x] + ((kind == MK_BND ? 4 * P.a[x].F.N : P.a[x].F.E) + tile - 1) / tile;
     }
     const int grid = grid_of(kind, P.first[m]);
     const cudaError_t e = kind == MK_PREP    ? L.prep_m(basis, P, grid, threads, st)
-                          : kind == MK_STAGE ? L.stage_m(basis, P, grid, stage_threads(nu, nv, fast), st)
+                          : kind == MK_BND   ? L.bnd_m(basis, P, grid, threads, st)
+                          : kind == MK_STAGE ? L.stage_m(basis, P, grid, STAGE_THREADS, st)
                                              : L.mass_m(basis, P, grid, threads, st);
     if (e != cudaSuccess) return e;
   }
@@ -777,12 +782,12 @@ int group_stage(const std::vector<wedg_ws *> &G, const std::vector<StageIO> &S, 
     args[i].S = S[i];
     args[i].S.parity = G[i]->parity;
     G[i]->parity = 1 - G[i]->parity;
-    G[i]->stats.kernel_launches += 3;
+    G[i]->stats.kernel_launches += 4;
     G[i]->stats.element_stages += G[i]->E;
   }
   wedg_ws *w = G[0];
   auto all = [](int, int total) { return total; };
-  for (int kind : {MK_PREP, MK_STAGE, MK_MASS}) {
+  for (int kind : {MK_PREP, MK_BND, MK_STAGE, MK_MASS}) {
     const cudaError_t e = multi_stage_launch(w->L, w->basis.data(), w->nu, w->nv, w->fast, kind, args,
                                              kind == MK_PREP ? w->prep_threads : w->mass_threads, w->stream, all);
     if (e != cudaSuccess) return cuda_fail(w, e, "multi-instance launch");
@@ -1087,7 +1092,7 @@ int adjoint_reverse_group(const std::vector<wedg_ws *> &G, const double *const *
     if ((rc = reset_flags(ws))) return rc;
     if (keep) {
       const size_t E = ws->E;
-      const size_t nd = (size_t)ws->nu * ws->nu + ws->nv * ws->nv + 12 * ws->nq + ws->qh * ws->qh + 2;
+      const size_t nd = (size_t)ws->nu * ws->nu + ws->nv * ws->nv + 12 * ws->nq + ws->qh * ws->qh + 4;
       while ((int64_t)ws->rk_keep.size() < nset * 4 * seg) {
         wedg_ws::StageData d;
         double *bd;
@@ -1096,7 +1101,7 @@ int adjoint_reverse_group(const std::vector<wedg_ws *> &G, const double *const *
         d.k = bd;
         d.tr = d.k + nn[i];
         d.G = d.tr + 12 * (size_t)ws->nq * E;
-        d.th = d.G + (size_t)ws->qh * ws->qh * E;
+        d.th = d.G + ((size_t)ws->qh * ws->qh + 2) * E;
         d.de = d.th + E;
         d.nst = ib;
         d.bins = ib + E;
@@ -1508,9 +1513,6 @@ int enqueue_bucket_step(wedg_batch *b, BatchBucket &k, double *const *u, double 
 int enqueue_merged_step(wedg_batch *b, BatchBucket &k, double *const *u, double *const *v, const double *t,
                         const double *dt, int stop_nonfinite, bool tables, long long tf_n) {
   const int n = (int)k.ids.size();
-  const int BT = stage_threads(k.nu, k.nv, k.fast);
-  const int TPW = 32 / (qhigh(k.nu, k.nv) / 2 + (qhigh(k.nu, k.nv) & 1));
-  const int mass_tile = (k.mass_threads / 32) * TPW;
   std::vector<StageArgs> args(n);
   for (int s = 0; s < 4; ++s) {
     for (int x = 0; x < n; ++x) {
@@ -1522,31 +1524,17 @@ int enqueue_merged_step(wedg_batch *b, BatchBucket &k, double *const *u, double 
       w->parity = 1 - w->parity;
       args[x].F = w->F;
       args[x].S = S;
-      w->stats.kernel_launches += 3;
+      w->stats.kernel_launches += 4;
       w->stats.element_stages += w->E;
     }
-    for (int kind = 0; kind < 3; ++kind) {
-      const int tile = kind == 0 ? k.prep_threads : kind == 1 ? BT : mass_tile;
-      for (int c0 = 0; c0 < n; c0 += MultiStage::cap) {
-        const int m = std::min(n - c0, MultiStage::cap);
-        MultiStage P;
-        P.n = m;
-        P.tile = tile;
-        P.first[0] = 0;
-        for (int x = 0; x < m; ++x) {
-          P.a[x] = args[c0 + x];
-          P.first[x + 1] = P.first[x] + (P.a[x].F.E + tile - 1) / tile;
-        }
-        const int total = P.first[m];
-        cudaError_t e;
-        if (kind == 0)
-          e = k.L.prep_m(k.basis.data(), P, bucket_grid(b, k, total, 3, k.prep_threads), k.prep_threads, k.st);
-        else if (kind == 1)
-          e = k.L.stage_m(k.basis.data(), P, bucket_grid(b, k, total, 2, 128), BT, k.st);
-        else
-          e = k.L.mass_m(k.basis.data(), P, bucket_grid(b, k, total, 3, k.mass_threads), k.mass_threads, k.st);
-        if (e != cudaSuccess) return cuda_fail(b->ws[k.ids[0]], e, "multi-instance launch");
-      }
+    for (int kind : {MK_PREP, MK_BND, MK_STAGE, MK_MASS}) {
+      const int threads = kind == MK_PREP ? k.prep_threads : kind == MK_MASS ? k.mass_threads : STAGE_THREADS;
+      auto grid = [&](int kd, int total) {
+        return kd == MK_BND ? total : bucket_grid(b, k, total, kd == MK_STAGE ? 2 : 3, threads);
+      };
+      const cudaError_t e =
+          multi_stage_launch(k.L, k.basis.data(), k.nu, k.nv, k.fast, kind, args, threads, k.st, grid);
+      if (e != cudaSuccess) return cuda_fail(b->ws[k.ids[0]], e, "multi-instance launch");
     }
   }
   if (k.cg) {
@@ -1749,8 +1737,8 @@ int create_finish(wedg_ws *ws) {
   Fields &F = ws->F;
   int rc;
   const size_t nU = (size_t)nu * nu * E, nV = (size_t)nv * nv * E;
-  if ((rc = dalloc(ws, &F.tr, (size_t)12 * nq * E)) || (rc = dalloc(ws, &F.G, (size_t)qh * qh * E)) ||
-      (rc = dalloc(ws, &F.th, Es)) || (rc = dalloc(ws, &F.de, Es)) || (rc = dalloc(ws, &F.nst, Es)) ||
+  if ((rc = dalloc(ws, &F.tr, (size_t)12 * nq * E)) || (rc = dalloc(ws, &F.G, ((size_t)qh * qh + 2) * E)) ||
+      (rc = dalloc(ws, &F.bslots, (size_t)4 * N * (2 * nv + nu))) || (rc = dalloc(ws, &F.th, Es)) || (rc = dalloc(ws, &F.de, Es)) || (rc = dalloc(ws, &F.nst, Es)) ||
       (rc = dalloc(ws, &F.nmax, 3)) || (rc = dalloc(ws, &F.nsum, 1)) || (rc = dalloc(ws, &F.err, 1)) ||
       (rc = dalloc(ws, &F.cg_nfail, 1)) ||
       (rc = dalloc(ws, &F.nonfinite, 1)) || (rc = dalloc(ws, &ws->steps_done, 1)) ||
@@ -1789,9 +1777,7 @@ int create_finish(wedg_ws *ws) {
     F.gam[s] = cfg->gamma_abc[s]; F.eta[s] = cfg->eta_abc[s]; F.sig[s] = cfg->sigma[s];
     F.kb[s] = cfg->kb[s]; F.kap[s] = cfg->kappa[s];
   }
-  // the dynamic shared-memory opt-in of k_stage on this device (a launch of zero blocks does nothing else)
-  cudaError_t ce = ws->L.stage(ws->basis.data(), F, StageIO{}, 0, 0, nullptr);
-  if (ce == cudaSuccess) ce = cudaMemset(F.bin_count, 0, 2 * NBIN * sizeof(int));
+  cudaError_t ce = cudaMemset(F.bin_count, 0, 2 * NBIN * sizeof(int));
   if (ce != cudaSuccess) {
     int r = cuda_fail(ws, ce, "wedg_create");
     wedg_destroy(ws);
@@ -2323,7 +2309,7 @@ int wedg_rk4_steps(wedg_ws *ws, double *u, double *v, double t0, double dt, int6
   // with host state and a step to take, the state comes in by ranges of elements on the copy stream
   // and the first stage's k_prep runs on each range as it arrives (k_prep reads only its own
   // element's state)
-  const int tp = ws->prep_threads;
+  const int tp = ws->prep_threads, ep = prep_tile(ws->nu, tp);
   const int nchunk = host && nsteps > 0 && !ws->timing && ws->E >= kCopyChunks * 4 * tp ? kCopyChunks : 0;
   if ((rc = reset_flags(ws))) return rc;
   if (host) {
@@ -2336,12 +2322,12 @@ int wedg_rk4_steps(wedg_ws *ws, double *u, double *v, double t0, double dt, int6
       const StageIO S0 = rk4_stage_io(ws, du, dv, 0, t0, dt, nullptr, 0, nullptr, nullptr);
       StageIO Sp = S0;
       Sp.parity = ws->parity;
-      const int nb = (ws->E + tp - 1) / tp, per = (nb + nchunk - 1) / nchunk;
+      const int nb = (ws->E + ep - 1) / ep, per = (nb + nchunk - 1) / nchunk;
       const size_t row = sizeof(double) * ws->E;
       for (int c = 0; c < nchunk; ++c) {
         const int b0 = c * per, b1 = std::min(nb, b0 + per);
         if (b0 >= b1) break;
-        const int e0 = b0 * tp, e1 = std::min(ws->E, b1 * tp);
+        const int e0 = b0 * ep, e1 = std::min(ws->E, b1 * ep);
         const size_t w = sizeof(double) * (size_t)(e1 - e0);
         CK(ws, cudaMemcpy2DAsync(ws->d_u + e0, row, u + e0, row, w, (size_t)ws->nu * ws->nu, cudaMemcpyHostToDevice,
                                  ws->copy_stream));

@@ -40,21 +40,21 @@ typedef void (*adj_face_fn)(const void *basis, const Fields &F, const StageIO &S
 
 // Multi-instance launches (wedg_kernels.cuh): `grid` blocks (0: one per virtual block) of
 // `threads` threads; the caller sets P.tile to the kernel's elements per block (k_prep: threads,
-// k_stage: stage_threads, the mass solves: (threads / 32) teams per warp)
+// k_bnd: bnd_tile sides, k_stage: stage_tile, the mass solves: (threads / 32) teams per warp)
 typedef cudaError_t (*multi_fn)(const void *basis, const MultiStage &P, int grid, int threads,
                                 cudaStream_t st);
 typedef cudaError_t (*multi_adj_fn)(const void *basis, const MultiAdj &P, int grid, cudaStream_t st);
 
-// k_prep over the elements [e0, e0 + blocks × threads) (clipped to the mesh)
+// k_prep over the elements [e0, e0 + blocks × prep_tile) (clipped to the mesh)
 typedef cudaError_t (*prep_fn)(const void *basis, const Fields &F, const StageIO &S, int blocks, int threads,
                                cudaStream_t st, int e0);
 
 struct Launchers {
   prep_fn prep = nullptr;
-  launch_fn stage = nullptr, mass = nullptr;
+  launch_fn bnd = nullptr, stage = nullptr, mass = nullptr;
   adj_fn adj_hats = nullptr, adj_mass = nullptr;
   adj_face_fn adj_face = nullptr;
-  multi_fn prep_m = nullptr, stage_m = nullptr, mass_m = nullptr;
+  multi_fn prep_m = nullptr, bnd_m = nullptr, stage_m = nullptr, mass_m = nullptr;
   multi_adj_fn adj_hats_m = nullptr, adj_mass_m = nullptr, adj_face_m = nullptr;
   pack_fn pack = nullptr;
   size_t basis_size = 0;
@@ -77,17 +77,93 @@ void pack_basis(const BasisHost &h, void *out) {
   for (int d = 0; d < NU; ++d) {
     b.El[d] = h.El[d]; b.Er[d] = h.Er[d]; b.E1l[d] = h.E1l[d]; b.E1r[d] = h.E1r[d];
     b.E1F[d] = h.E1F[d];
-    for (int c = 0; c < NU; ++c) { b.K1[d][c] = h.K1[d][c]; b.Q[d][c] = h.Q[d][c]; b.ilam2[d][c] = h.ilam2[d][c]; }
-  }
-  for (int i = 0; i < NU; ++i) {
-    double x = 0.0;
-    for (int a = 0; a < NU; ++a) x += h.Q[a][i] * h.E1F[a];
-    b.QE[i] = x;
+    for (int c = 0; c < NU; ++c) { b.K1[d][c] = h.K1[d][c]; }
   }
   for (int r = 0; r < QH; ++r) {
     b.wh[r] = h.wh[r];
     for (int d = 0; d < NV; ++d) { b.Ph[r][d] = h.Ph[r][d]; b.PhW[r][d] = h.PhW[r][d]; }
   }
+  // fixed-point forms: Ph is contracted over its modes (row sums), PhW over its points (column sums)
+  auto big = [](double &m, double x) { m = x > m ? x : m; };
+  double sP = 0, bP = 0, sW = 0, bW = 0;
+  for (int r = 0; r < QH; ++r) {
+    double s = 0;
+    for (int d = 0; d < NV; ++d) { s += fabs(b.Ph[r][d]); big(bP, fabs(b.Ph[r][d])); big(bW, fabs(b.PhW[r][d])); }
+    big(sP, s);
+  }
+  for (int d = 0; d < NV; ++d) {
+    double s = 0;
+    for (int r = 0; r < QH; ++r) s += fabs(b.PhW[r][d]);
+    big(sW, s);
+  }
+  b.gPh = fx_exponent(sP, bP);
+  b.gPhW = fx_exponent(sW, bW);
+  for (int d = 0; d < NV; ++d) {
+    double c = 0;
+    for (int r = 0; r < QH; ++r) big(c, fabs(b.Ph[r][d]));
+    b.cPh[d] = (int)ceil(ldexp(c, 8));
+  }
+  {
+    double c = 0;                  // the largest Euclidean norm of a row of Ph
+    for (int r = 0; r < QH; ++r) {
+      double s = 0;
+      for (int d = 0; d < NV; ++d) s += b.Ph[r][d] * b.Ph[r][d];
+      big(c, sqrt(s));
+    }
+    int lg;
+    frexp(NV * c, &lg);
+    const int up = 2 * (61 - b.gPh) + (61 - b.gPhW) - lg;
+    b.nrow = up > 0 ? up : 0;
+  }
+  // the constant-coefficient kernels' operators: the end values two to a sum (A and D of a side), K1
+  // by its rows (columns in one sum with them), Q by rows or columns beside the constant mode
+  double eL = 0, e1 = 0, sK = 0, bK = 0, sQ = 0, bQ = 0, bL = 0, bE = 0, QE[NU];
+  for (int i = 0; i < NU; ++i) {
+    big(eL, fabs(h.El[i]));
+    big(e1, fabs(h.E1l[i]));
+    double k = 0, r = 0, c = 0;
+    QE[i] = 0;
+    for (int a = 0; a < NU; ++a) {
+      QE[i] += h.Q[a][i] * h.E1F[a];
+      k += fabs(ldexp(h.K1[i][a], -k1_bits<NU>(a)));
+      big(bK, fabs(ldexp(h.K1[i][a], -k1_bits<NU>(a))));
+      if (i == 0 || a == 0) continue;
+      r += fabs(h.Q[i][a]);
+      c += fabs(h.Q[a][i]);
+      big(bQ, fabs(h.Q[i][a]));
+    }
+    big(sK, 2 * k);
+    big(sQ, r);
+    big(sQ, c);
+    for (int a = 0; a < NU; ++a)
+      if (i + a > 0) big(bL, fabs(h.ilam2[i][a]));
+  }
+  for (int i = 0; i < NU; ++i)
+    for (int a = 0; a < NU; ++a)
+      if (i + a > 0) big(bE, fabs(QE[i] * h.ilam2[i][a]));
+  b.gEl = fx_exponent(2 * eL, eL);
+  b.gE1 = fx_exponent(2 * e1, e1);
+  b.gK1 = fx_exponent(sK, bK);
+  b.gQ = fx_exponent(sQ, bQ);
+  b.gL = fx_exponent(bL, bL);
+  b.gM = fx_exponent(2 * bE, bE);
+  for (int i = 0; i < NU; ++i) {
+    b.fEl[i] = fx_const(h.El[i], b.gEl);
+    b.fE1[i] = fx_const(h.E1l[i], b.gE1);
+    b.kK1[i] = k1_bits<NU>(i);
+    for (int a = 0; a < NU; ++a) {
+      b.fK1[i][a] = fx_const(ldexp(h.K1[i][a], -k1_bits<NU>(a)), b.gK1);
+      b.fQ[i][a] = fx_const(i == 0 || a == 0 ? 0.0 : h.Q[i][a], b.gQ);
+      b.fL[i][a] = fx_const(i + a == 0 ? 0.0 : h.ilam2[i][a], b.gL);
+      b.fM[i][a][0] = fx_const(i + a == 0 ? 0.0 : QE[i] * h.ilam2[i][a], b.gM);
+      b.fM[i][a][1] = fx_const(i + a == 0 ? 0.0 : QE[a] * h.ilam2[i][a], b.gM);
+    }
+  }
+  for (int r = 0; r < QH; ++r)
+    for (int d = 0; d < NV; ++d) {
+      b.fPh[r][d] = fx_const(b.Ph[r][d], b.gPh);
+      b.fPhW[r][d] = fx_const(b.PhW[r][d], b.gPhW);
+    }
 }
 
 template <int NU, int NV>
@@ -97,37 +173,20 @@ cudaError_t launch_prep(const void *basis, const Fields &F, const StageIO &S, in
   return cudaSuccess;
 }
 
-// The opt-in to more than 48 KB of dynamic shared memory for kernel K, once per device: a
-// function attribute belongs to the context of the device that is current when it is set, so
-// every device that launches the kernel needs its own (std::call_once per device index, so
-// that threads that launch at once on one device set it once)
-template <class Tag, class K>
-cudaError_t smem_opt_in(K kernel, size_t smem) {
-  static std::once_flag once[MAX_DEVICES];
-  static cudaError_t result[MAX_DEVICES];
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= MAX_DEVICES)
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  std::call_once(once[dev], [&] {
-    result[dev] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  });
-  return result[dev];
+// k_bnd over the 4N physical sides (the grid follows from F.N)
+template <int NU, int NV>
+cudaError_t launch_bnd(const void *basis, const Fields &F, const StageIO &S, int, int, cudaStream_t st) {
+  k_bnd<NU, NV><<<(4 * F.N + bnd_tile(NU) - 1) / bnd_tile(NU), BND_THREADS, 0, st>>>(
+      *static_cast<const Basis<NU, NV> *>(basis), F, S);
+  return cudaSuccess;
 }
 
-// k_stage keeps the element blocks in dynamic shared memory (up to 227 KB per block);
-// `threads` must be stage_threads(NU, NV, FAST). blocks = 0 only sets the attribute.
-template <int NU, int NV, bool FAST>
-struct StageTag {};
+// k_stage: `blocks` blocks of STAGE_THREADS, stage_tile elements each
 template <int NU, int NV, bool FAST>
 cudaError_t launch_stage(const void *basis, const Fields &F, const StageIO &S, int blocks, int threads,
                          cudaStream_t st) {
-  constexpr size_t smem = stage_smem(NU, NV, FAST);
-  const cudaError_t e = smem_opt_in<StageTag<NU, NV, FAST>>(k_stage<NU, NV, FAST>, smem);
-  if (e != cudaSuccess) return e;
   if (blocks <= 0) return cudaSuccess;
-  k_stage<NU, NV, FAST><<<blocks, threads, smem, st>>>(*static_cast<const Basis<NU, NV> *>(basis), F, S);
+  k_stage<NU, NV, FAST><<<blocks, threads, 0, st>>>(*static_cast<const Basis<NU, NV> *>(basis), F, S);
   return cudaSuccess;
 }
 
@@ -176,16 +235,19 @@ cudaError_t launch_prep_m(const void *basis, const MultiStage &P, int grid, int 
   return cudaSuccess;
 }
 
-template <int NU, int NV, bool FAST>
-struct StageMultiTag {};
-template <int NU, int NV, bool FAST>
-cudaError_t launch_stage_m(const void *basis, const MultiStage &P, int grid, int, cudaStream_t st) {
-  constexpr size_t smem = stage_smem(NU, NV, FAST);
-  const cudaError_t e = smem_opt_in<StageMultiTag<NU, NV, FAST>>(k_stage_m<NU, NV, FAST>, smem);
-  if (e != cudaSuccess) return e;
+template <int NU, int NV>
+cudaError_t launch_bnd_m(const void *basis, const MultiStage &P, int grid, int, cudaStream_t st) {
   const int total = P.first[P.n];
   if (total <= 0) return cudaSuccess;
-  k_stage_m<NU, NV, FAST><<<multi_grid(grid, total), stage_threads(NU, NV, FAST), smem, st>>>(
+  k_bnd_m<NU, NV><<<multi_grid(grid, total), BND_THREADS, 0, st>>>(*static_cast<const Basis<NU, NV> *>(basis), P);
+  return cudaSuccess;
+}
+
+template <int NU, int NV, bool FAST>
+cudaError_t launch_stage_m(const void *basis, const MultiStage &P, int grid, int, cudaStream_t st) {
+  const int total = P.first[P.n];
+  if (total <= 0) return cudaSuccess;
+  k_stage_m<NU, NV, FAST><<<multi_grid(grid, total), STAGE_THREADS, 0, st>>>(
       *static_cast<const Basis<NU, NV> *>(basis), P);
   return cudaSuccess;
 }
@@ -233,6 +295,7 @@ template <int NU, int NV>
 Launchers make_launchers(bool fast) {
   Launchers L;
   L.prep_m = launch_prep_m<NU, NV>;
+  L.bnd_m = launch_bnd_m<NU, NV>;
   L.stage_m = fast ? launch_stage_m<NU, NV, true> : launch_stage_m<NU, NV, false>;
   L.mass_m = launch_mass_m<NU, NV>;
   L.adj_hats_m = launch_adj_hats_m<NU, NV>;
@@ -242,6 +305,7 @@ Launchers make_launchers(bool fast) {
   L.adj_mass = launch_adj_mass<NU, NV>;
   L.adj_face = launch_adj_face<NU, NV>;
   L.prep = launch_prep<NU, NV>;
+  L.bnd = launch_bnd<NU, NV>;
   L.mass = launch_mass<NU, NV>;
   L.stage = fast ? launch_stage<NU, NV, true> : launch_stage<NU, NV, false>;
   L.pack = pack_basis<NU, NV>;

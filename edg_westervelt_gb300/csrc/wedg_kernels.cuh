@@ -43,7 +43,10 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <limits.h>
+#include <math.h>
 #include <stdint.h>
+
+#include "wedg_fixed.cuh"
 
 namespace wedg {
 
@@ -57,19 +60,9 @@ __host__ __device__ constexpr int qhigh(int nu, int nv) {
   return ((3 * (nv - 1) + 1) / 2 + 1) > nu ? ((3 * (nv - 1) + 1) / 2 + 1) : nu;
 }
 
-// Shared memory of k_stage per thread: b and R_v (NU² + NV² doubles); the general kernels give
-// R_v NU² doubles, because the packed-inverse u-solve writes its result there once R_v is spent.
-// Both read U and V from HBM.
-__host__ __device__ constexpr int stage_doubles(int nu, int nv, bool fast) {
-  return fast ? nu * nu + nv * nv : 2 * nu * nu;
-}
-// Threads per block of k_stage: two blocks per SM (228 KB per SM, 1 KB of it per block reserved)
-__host__ __device__ constexpr int stage_threads(int nu, int nv, bool fast) {
-  return 2 * (128 * stage_doubles(nu, nv, fast) * 8 + 1024) <= 233472 ? 128 : 96;
-}
-__host__ __device__ constexpr size_t stage_smem(int nu, int nv, bool fast) {
-  return (size_t)stage_threads(nu, nv, fast) * stage_doubles(nu, nv, fast) * sizeof(double);
-}
+// k_stage: a team of NU threads per element in blocks of 128
+constexpr int STAGE_THREADS = 128;
+__host__ __device__ constexpr int stage_tile(int nu) { return (32 / nu) * (STAGE_THREADS / 32); }   // elements per block
 
 template <int NU, int NV>
 struct Basis {
@@ -85,9 +78,15 @@ struct Basis {
   double PhW[QH][NV];            // w_h[r] P_h_v[r, d], with W2d_h = w_h w_h^T
   double wh[QH];                 // w_h
   double K1[NU][NU];             // 1D stiffness S^T diag(w) S
-  double Q[NU][NU];              // its eigenvectors, Q[row][col]; Q[.][0] = e_0
-  double ilam2[NU][NU];          // 1 / (λ_i + λ_j), and 1 at (0, 0)
-  double QE[NU];                 // Q^T E1F: the u-slots' lift factor in the eigenbasis of K1
+  // fixed-point forms (wedg_fixed.cuh): Ph, PhW; for the constant-coefficient kernels the end values,
+  // K1[a][c] 2^-kK1[c], K1's eigenvectors Q (Q[row][col]; Q[.][0] = e_0), L = 1 / (λ_i + λ_j) (0 at
+  // (0, 0)) and the pairs QE[i] L[i][j], QE[j] L[i][j] (QE = Q^T E1F: the u-slots' lift factor in the
+  // eigenbasis)
+  FxC fPh[QH][NV], fPhW[QH][NV], fEl[NU], fE1[NU], fK1[NU][NU], fQ[NU][NU], fL[NU][NU], fM[NU][NU][2];
+  int gPh, gPhW, gEl, gE1, gK1, gQ, gL, gM;   // their exponents
+  int kK1[NU];
+  int nrow;                      // bits that team_K_fx shifts the grid rows up by
+  int cPh[NV];                   // 2^8 max|Ph[.][a]|, rounded up
 };
 
 struct Fields {
@@ -101,7 +100,13 @@ struct Fields {
   const double *bsp[4], *bspn[4];
   const double *PiSP, *PiBSP2, *PiCdiv, *PiDdiv, *srcP;
   const double *beta2;        // 2β at the high-order points, [(r + QH s) E + e]
-  double *tr, *G, *th, *de;   // G = 2βv at the high-order points
+  // G = 2βv at the high-order points: for k_cheb as integers of one exponent per element, which row
+  // QH² holds with a normalising shift (GPack); k_cg and k_adj_mass keep doubles of their own there.
+  // Row QH² + 1: the largest high words of U and V beside the constant mode (k_stage's exponents)
+  double *tr, *G, *th, *de;
+  // the flux slots of the physical sides projected on the face modes: [(q 4 + s) N + m], q over the
+  // modes of A, D and F, m along side s
+  double *bslots;
   double *mrhs;               // right-hand side of the mass system, [(a + NV b) E + e]
   int *nst;
   int *nmax;                  // largest Chebyshev count: [parity] of a stage (the common count of
@@ -189,7 +194,7 @@ struct Multi {
 };
 
 // CAP is what fits the kernel parameter limit (32 764 bytes) beside the largest Basis
-using MultiStage = Multi<StageArgs, 31>;
+using MultiStage = Multi<StageArgs, 22>;
 
 // The instance of virtual block vb. The kernels read that instance's arguments where they lie, in
 // the parameter block: the index is the same for the whole block, so the reads are uniform
@@ -202,17 +207,6 @@ __device__ __forceinline__ int multi_begin(const Multi<Args, CAP> &P, int vb) {
   __syncthreads();
   return inst;
 }
-
-// A thread-private n×n block in shared memory: X(a, b) at base[(a + n b) BT + tid]
-template <int n, int BT>
-struct Blk {
-  double *p;
-  __device__ __forceinline__ double &operator()(int a, int b) const { return p[(a + n * b) * BT]; }
-};
-
-// Nonzero pattern of the eigenbasis Q of the 1D stiffness K1 (built so on the host): Q[a][i]
-// vanishes for a + i odd and in row and column 0 outside (0, 0)
-__host__ __device__ constexpr bool qnz(int a, int i) { return ((a + i) & 1) == 0 && ((a == 0) == (i == 0)); }
 
 // ----------------------------------------------------------------------------
 // Mirror-parity contractions. The points of both quadratures are Gauss-Legendre
@@ -299,6 +293,18 @@ __device__ __forceinline__ void ph_row_mid(const double (&Ph)[QH][NV], const X &
 // k_prep: traces, boundary weight check, Chebyshev interval data
 // ----------------------------------------------------------------------------
 
+// Row QH² of G: the exponent sG of the element's integers G (G = integer 2^sG) and the shift ng that
+// takes their largest to [2^59, 2^60)
+struct GPack {
+  int sG, ng;
+  __device__ GPack(int s, i64 lo, i64 hi) : sG(s) {
+    const i64 top = max(hi, -lo);
+    ng = top > 0 ? __clzll(top) - 4 : 0;
+  }
+  __device__ explicit GPack(i64 w) : sG((int)(w >> 32)), ng((int)w) {}
+  __device__ i64 word() const { return (i64)sG << 32 | (unsigned)ng; }
+};
+
 // Traces of an n×n block X on the four sides (src/rhs.jl:388-410):
 //   oB[i] = Σ_b P[i,b] Σ_a El[a] X[a][b],  oT with Er,
 //   oL[i] = Σ_b P[i,b] Σ_a El[a] X[b][a],  oR with Er,
@@ -372,161 +378,6 @@ __device__ __forceinline__ void load_regs(double (&X)[n][n], const double *x, in
     for (int a = 0; a < n; ++a) X[a][b] = x[e + (size_t)E * (a + n * b)];
 }
 
-// k_prep's work for element e (first: the instance's first block, which clears the bin counts)
-template <int NU, int NV>
-__device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &F, const StageIO &S, int e,
-                                          bool first) {
-  constexpr int NQ = NU, QH = Basis<NU, NV>::QH;
-  const int E = F.E, N = F.N;
-  // the bin counts and the largest count of the next stage start at zero: all NBIN bins, whatever
-  // the element count
-  if (first && F.sorted)
-    for (int b = threadIdx.x; b < NBIN; b += blockDim.x) F.bin_count[(1 - S.parity) * NBIN + b] = 0;
-  if (first && threadIdx.x == 0) F.nmax[1 - S.parity] = 0;
-  if (e >= E) return;
-  if (err_word(F) != ERR_NONE) return;
-  const int j = e % N, k = e / N;
-  const bool modal = F.modal != 0;
-  {
-    double U[NU][NU];
-    load_regs<NU>(U, S.xu, E, e);
-    trace4<NQ, NU, NU, true>(U, B.P, B.E1l, F.tr, 0, E, e, 1.0, modal);
-  }
-  double V[NV][NV];
-  load_regs<NV>(V, S.xv, E, e);
-  trace4<NQ, NU, NV, false>(V, B.P, B.El, F.tr, 1, E, e, 1.0, modal);
-  trace4<NQ, NU, NV, true>(V, B.P, B.E1l, F.tr, 2, E, e, 1.0, modal);
-
-  const TimeF tf = time_factors(S);
-  // weight check 1 - kβv > 0 for the trace and the data on physical sides
-  // (src/rhs.jl:109-110, 751-757); key of src/rhs.jl:732
-  const bool onb[4] = {j == 0, j == N - 1, k == 0, k == N - 1};
-#pragma unroll 1
-  for (int s = 0; s < 4; ++s) {
-    if (!onb[s] || F.kind[s] == 3) continue;
-    const int m = s < 2 ? k : j;
-    unsigned long long key = ERR_NONE;
-#pragma unroll 1
-    for (int i = 0; i < NQ; ++i) {
-      const double bf = s < 2 ? F.hbf[(s == 0 ? 0 : N) + (size_t)(N + 1) * (k + (size_t)N * i)]
-                              : F.vbf[j + (size_t)N * ((s == 2 ? 0 : N) + (size_t)(N + 1) * i)];
-      const double v_fp = modal ? modal_at<NQ, NU, NV>(B.P, F.tr, 1, s, i, E, e)
-                                : F.tr[((1 * 4 + s) * NQ + i) * (size_t)E + e];
-      const double v_ex = -F.omega * tf.st * F.bsp[s][m + (size_t)N * i];
-      const int check = (1.0 - F.kb[s] * bf * v_fp <= 0.0) ? 1 : (1.0 - F.kb[s] * bf * v_ex <= 0.0) ? 2 : 0;
-      if (check) {
-        const unsigned long long kk =
-            2ull * ((unsigned long long)s * NQ * N + i + (unsigned long long)m * NQ) + check;
-        key = kk < key ? kk : key;
-      }
-    }
-    if (key != ERR_NONE) atomicMin(F.err, key);
-  }
-
-  if (F.cg) return;
-  // Chebyshev interval of the element: v_q = P_h V P_h^T, G = 2βv_q, a± = 1 - extrema(G);
-  // the rows of the point grid in mirrored pairs. The extrema and the NaN test run on the
-  // integer pipe (order-preserving integer keys of the doubles), so that a point costs one
-  // FP64 multiply besides the contractions.
-  long long kmin = LLONG_MAX, kmax = LLONG_MIN;
-  bool nan = false;
-  auto vx = [&](int a, int b) { return V[a][b]; };
-  auto point = [&](double y, int r, int s2) {
-    const size_t gi = (r + QH * s2) * (size_t)E + e;
-    const double g = y * F.beta2[gi];
-    F.G[gi] = g;
-    const long long bits = __double_as_longlong(g);
-    nan |= (bits & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
-    const long long key = bits ^ ((bits >> 63) & 0x7fffffffffffffffLL);
-    kmin = min(kmin, key);
-    kmax = max(kmax, key);
-  };
-  // the points of row r: v_q = Σ_b T[b] Ph[s2][b], mirrored columns s2 and QH-1-s2 together
-  auto points = [&](const double (&T)[NV], int r) {
-#pragma unroll
-    for (int s2 = 0; s2 < QH / 2; ++s2) {
-      double ev = 0.0, od = 0.0;
-#pragma unroll
-      for (int b = 0; b < NV; b += 2) ev = fma(T[b], B.Ph[s2][b], ev);
-#pragma unroll
-      for (int b = 1; b < NV; b += 2) od = fma(T[b], B.Ph[s2][b], od);
-      point(ev + od, r, s2);
-      point(ev - od, r, QH - 1 - s2);
-    }
-    if constexpr ((QH & 1) != 0) {
-      double ev = 0.0;
-#pragma unroll
-      for (int b = 0; b < NV; b += 2) ev = fma(T[b], B.Ph[QH / 2][b], ev);
-      point(ev, r, QH / 2);
-    }
-  };
-#pragma unroll 1
-  for (int r = 0; r < QH / 2; ++r) {
-    double Tp[NV], Tm[NV];
-    ph_row_pair<QH, NV>(B.Ph, r, vx, Tp, Tm);
-    points(Tp, r);
-    points(Tm, QH - 1 - r);
-  }
-  if constexpr ((QH & 1) != 0) {
-    double T[NV];
-    ph_row_mid<QH, NV>(B.Ph, vx, T);
-    points(T, QH / 2);
-  }
-  const double gmin = __longlong_as_double(kmin ^ ((kmin >> 63) & 0x7fffffffffffffffLL));
-  const double gmax = __longlong_as_double(kmax ^ ((kmax >> 63) & 0x7fffffffffffffffLL));
-  const double amin = 1.0 - gmax, amax = 1.0 - gmin;
-  if (nan || !(amin > 0.0)) {
-    atomicMin(F.err, (1ull << ERR_CLASS_SHIFT) | (unsigned long long)(e + 1));
-    return;
-  }
-  const double th = 0.5 * (amax + amin);
-  const double de = fmax(0.5 * (amax - amin), 1e-15 * th);
-  F.th[e] = th;
-  F.de[e] = de;
-  const int n = (int)ceil(F.Lcheb / acosh(th / de));
-  F.nst[e] = n;
-  // largest count and the sum of the counts: one atomic each per warp
-  const unsigned mask = __activemask();
-  const int nw = __reduce_max_sync(mask, n);
-  const unsigned ns = __reduce_add_sync(mask, (unsigned)n);
-  const int lane = threadIdx.x & 31;
-  if (lane == __ffs(mask) - 1) {
-    atomicMax(&F.nmax[S.parity], nw);
-    atomicMax(&F.nmax[2], nw);
-    atomicAdd(F.nsum, (unsigned long long)ns);
-  }
-  if (F.sorted) {
-    // append e to the list of its count, one atomic per group of lanes with the same count
-    const int bin = (n < NBIN ? n : NBIN) - 1;
-    const unsigned same = __match_any_sync(mask, bin);
-    const int leader = __ffs(same) - 1;
-    const int rank = __popc(same & ((1u << lane) - 1));
-    int base = 0;
-    if (lane == leader) base = atomicAdd(&F.bin_count[S.parity * NBIN + bin], __popc(same));
-    base = __shfl_sync(same, base, leader);
-    F.bins[(size_t)bin * E + base + rank] = e;
-  }
-}
-
-template <int NU, int NV>
-__global__ void __launch_bounds__(128, 3) k_prep(const __grid_constant__ Basis<NU, NV> B,
-                                              const __grid_constant__ Fields F,
-                                              const __grid_constant__ StageIO S, int e0) {
-  // elements e0 + (block, thread): a launch may cover a range of the elements (the first range
-  // clears the next stage's counts)
-  prep_body<NU, NV>(B, F, S, e0 + (int)(blockIdx.x * blockDim.x + threadIdx.x), blockIdx.x == 0 && e0 == 0);
-}
-
-template <int NU, int NV>
-__global__ void __launch_bounds__(128, 3) k_prep_m(const __grid_constant__ Basis<NU, NV> B,
-                                                const __grid_constant__ MultiStage P) {
-  for (int vb = blockIdx.x; vb < P.first[P.n]; vb += gridDim.x) {
-    const int inst = multi_begin(P, vb);
-    const int e0 = (vb - P.first[inst]) * P.tile;
-    prep_body<NU, NV>(B, P.a[inst].F, P.a[inst].S, e0 + (int)threadIdx.x, e0 == 0);
-  }
-}
-
 // ----------------------------------------------------------------------------
 // k_stage helpers
 // ----------------------------------------------------------------------------
@@ -579,53 +430,58 @@ __device__ __forceinline__ void interior_flux(const Fields &F, const FaceCoef &c
   }
 }
 
-// Numerical flux slots A, D, F at point i of side s of the element
-// (src/rhs.jl:620-700 for interior faces, :65-103 and :738-763 for physical sides).
+// Numerical flux slots A, D, F at point i of physical side s of the element (src/rhs.jl:65-103, 738-763)
 template <int NU, int NV>
-__device__ __forceinline__ void side_point(const Basis<NU, NV> &B, const Fields &F, const TimeF &S, int s,
-                                           bool boundary, int j, int k, int e, int i, double &A, double &D,
+__device__ __forceinline__ void boundary_point(const Basis<NU, NV> &B, const Fields &F, const TimeF &S, int s, int j,
+                                               int k, int e, int i, double &A, double &D, double &Fs) {
+  constexpr int NQ = NU;
+  const int N = F.N, E = F.E;
+  const double *tr = F.tr;
+  auto T = [&](int fam, int side, int el) { return tr[((fam * 4 + side) * NQ + i) * (size_t)E + el]; };
+  const int m = s < 2 ? k : j;
+  const double sgn = (s == 0 || s == 2) ? -1.0 : 1.0;
+  size_t fi;
+  const double *c2a, *afa, *cfa, *bfa;
+  if (s < 2) { fi = (s == 0 ? 0 : N) + (size_t)(N + 1) * (k + (size_t)N * i); c2a = F.hc2; afa = F.haf; cfa = F.hcf; bfa = F.hbf; }
+  else { fi = j + (size_t)N * ((s == 2 ? 0 : N) + (size_t)(N + 1) * i); c2a = F.vc2; afa = F.vaf; cfa = F.vcf; bfa = F.vbf; }
+  const double c2f = c2a[fi], af = afa[fi], cf = cfa[fi];
+  const bool modal = F.modal != 0;
+  const double v_fp = modal ? modal_at<NQ, NU, NV>(B.P, tr, 1, s, i, E, e) : T(1, s, e);
+  const double gun = sgn * (F.two_h * (modal ? modal_at<NQ, NU, NU>(B.P, tr, 0, s, i, E, e) : T(0, s, e)));
+  const double gvn = sgn * (F.two_h * (modal ? modal_at<NQ, NU, NV>(B.P, tr, 2, s, i, E, e) : T(2, s, e)));
+  const double spn = F.bspn[s][m + (size_t)N * i], sp = F.bsp[s][m + (size_t)N * i];
+  const double gu_ex = sgn * (S.ct * spn - spn);
+  const double gv_ex = sgn * (-F.omega * S.st * spn);
+  const double v_ex = -F.omega * S.st * sp;
+  double F1, dv;
+  if (F.kind[s] == 3) {
+    const double g2 = c2f * gu_ex + af * gv_ex;
+    const double rho_w = c2f * gun + af * gvn - g2;
+    dv = -(F.kap[s] / cf) * rho_w;
+    F1 = g2;
+  } else {
+    const double bf = bfa[fi];
+    const double g = F.gam[s], et = F.eta[s], sg = F.sig[s], kb = F.kb[s];
+    const double sqf = sqrt(1.0 - kb * bf * v_fp);
+    const double rho_num = et * (c2f * gun + af * gvn) + g * cf * sqf * v_fp;
+    const double rho_ex = et * (c2f * gu_ex + af * gv_ex) + g * cf * sqrt(1.0 - kb * bf * v_ex) * v_ex;
+    const double rho = rho_num - rho_ex;
+    F1 = c2f * gun + af * gvn - (et + sg * g) * rho;
+    dv = -(g - sg * et) / (cf * sqf) * rho;
+  }
+  A = F1;
+  D = sgn * (af * dv);
+  Fs = -sgn * (c2f * dv);
+}
+
+// Numerical flux slots A, D, F at point i of interior side s of the element (src/rhs.jl:620-700)
+template <int NU, int NV>
+__device__ __forceinline__ void side_point(const Fields &F, int s, int j, int k, int e, int i, double &A, double &D,
                                            double &Fs) {
   constexpr int NQ = NU;
   const int N = F.N, E = F.E;
   const double *tr = F.tr;
   auto T = [&](int fam, int side, int el) { return tr[((fam * 4 + side) * NQ + i) * (size_t)E + el]; };
-  if (boundary) {
-    const int m = s < 2 ? k : j;
-    const double sgn = (s == 0 || s == 2) ? -1.0 : 1.0;
-    size_t fi;
-    const double *c2a, *afa, *cfa, *bfa;
-    if (s < 2) { fi = (s == 0 ? 0 : N) + (size_t)(N + 1) * (k + (size_t)N * i); c2a = F.hc2; afa = F.haf; cfa = F.hcf; bfa = F.hbf; }
-    else { fi = j + (size_t)N * ((s == 2 ? 0 : N) + (size_t)(N + 1) * i); c2a = F.vc2; afa = F.vaf; cfa = F.vcf; bfa = F.vbf; }
-    const double c2f = c2a[fi], af = afa[fi], cf = cfa[fi];
-    const bool modal = F.modal != 0;
-    const double v_fp = modal ? modal_at<NQ, NU, NV>(B.P, tr, 1, s, i, E, e) : T(1, s, e);
-    const double gun = sgn * (F.two_h * (modal ? modal_at<NQ, NU, NU>(B.P, tr, 0, s, i, E, e) : T(0, s, e)));
-    const double gvn = sgn * (F.two_h * (modal ? modal_at<NQ, NU, NV>(B.P, tr, 2, s, i, E, e) : T(2, s, e)));
-    const double spn = F.bspn[s][m + (size_t)N * i], sp = F.bsp[s][m + (size_t)N * i];
-    const double gu_ex = sgn * (S.ct * spn - spn);
-    const double gv_ex = sgn * (-F.omega * S.st * spn);
-    const double v_ex = -F.omega * S.st * sp;
-    double F1, dv;
-    if (F.kind[s] == 3) {
-      const double g2 = c2f * gu_ex + af * gv_ex;
-      const double rho_w = c2f * gun + af * gvn - g2;
-      dv = -(F.kap[s] / cf) * rho_w;
-      F1 = g2;
-    } else {
-      const double bf = bfa[fi];
-      const double g = F.gam[s], et = F.eta[s], sg = F.sig[s], kb = F.kb[s];
-      const double sqf = sqrt(1.0 - kb * bf * v_fp);
-      const double rho_num = et * (c2f * gun + af * gvn) + g * cf * sqf * v_fp;
-      const double rho_ex = et * (c2f * gu_ex + af * gv_ex) + g * cf * sqrt(1.0 - kb * bf * v_ex) * v_ex;
-      const double rho = rho_num - rho_ex;
-      F1 = c2f * gun + af * gvn - (et + sg * g) * rho;
-      dv = -(g - sg * et) / (cf * sqf) * rho;
-    }
-    A = F1;
-    D = sgn * (af * dv);
-    Fs = -sgn * (c2f * dv);
-    return;
-  }
   // interior: the element is "+" on its B and L sides, "-" on T and R
   const bool plus = (s == 0 || s == 2);
   const int nb = s == 0 ? e - 1 : s == 1 ? e + 1 : s == 2 ? e - N : e + N;
@@ -647,673 +503,363 @@ __device__ __forceinline__ void side_point(const Basis<NU, NV> &B, const Fields 
   interior_flux(F, cf, plus, dum, dup, vm, vp, dvm, dvp, A, D, Fs);
 }
 
-// The projections Y_A, Y_D (b < NV) and Y_F (b < NU) of the flux slots of interior side s, with
-// the traces held as modal end sums (Fields::modal). The face coefficients are one value along the
-// face, so every slot is a linear combination of the six traces and the jump term K with the same
-// weights at every point, and its projection Σ_i w_i P[i][b] (.)_i is that combination of the
-// traces' modes b and of K's projection on mode b (hJCm, vJCm): the face rule integrates the
-// product of two modes exactly and the modes are orthonormal. The same results as the point form
-// of side_point and the projections, to rounding.
+// k_bnd: the physical sides, a team of NQ lanes per side: lane i evaluates the flux slots at
+// point i, then projects them on mode i (Y[b] = Σ_q w_q P[q][b] (.)_q), and k_stage reads the
+// projections. A point costs about 150 FP64 operations (two square roots and the divisions); in its
+// element's thread of k_stage a side held the 31 others of the warp up for 7 points on end, in every
+// fourth warp at N = 256 and in every one below N = 64, and the columns of the left and right sides
+// were whole warps of it. Spread over the chip the 4N sides take some 6 us.
+constexpr int BND_THREADS = 32;
+__host__ __device__ constexpr int bnd_tile(int nu) { return BND_THREADS / nu; }
 template <int NU, int NV>
-__device__ __forceinline__ void modal_side(const Fields &F, int s, int j, int k, int e, double (&YA)[NV],
-                                           double (&YD)[NV], double (&YF)[NU]) {
+__device__ __forceinline__ void bnd_body(const Basis<NU, NV> &B, const Fields &F, const StageIO &S, int side0) {
   constexpr int NQ = NU;
-  const int N = F.N;
-  const size_t E = F.E;
-  const bool plus = (s == 0 || s == 2);
-  const int nb = s == 0 ? e - 1 : s == 1 ? e + 1 : s == 2 ? e - N : e + N;
-  const int sm = s < 2 ? 1 : 3, spp = s < 2 ? 0 : 2;      // trace sides of the "-" and "+" elements
-  const int em = plus ? nb : e, ep = plus ? e : nb;
-  size_t fi;
-  const double *c2p_a, *afp_a, *c2m_a, *afm_a, *jc_a, *jcm;
-  if (s < 2) {
-    fi = (s == 0 ? j : j + 1) + (size_t)(N + 1) * k;
-    c2p_a = F.hc2; afp_a = F.haf; c2m_a = F.hc2m; afm_a = F.hafm; jc_a = F.hJC; jcm = F.hJCm;
-  } else {
-    fi = j + (size_t)N * (s == 2 ? k : k + 1);
-    c2p_a = F.vc2; afp_a = F.vaf; c2m_a = F.vc2m; afm_a = F.vafm; jc_a = F.vJC; jcm = F.vJCm;
-  }
-  const FaceCoef cf = face_coef(F, c2p_a, afp_a, c2m_a, afm_a, jc_a, fi);   // point 0 of the face
-  // the slots of interior_flux as linear forms with the face's weights (continuous faces: the
-  // one-sided form with equal values on both sides): G = Σ g·traces, J = Σ j·traces + K,
-  // s = v⁻ - v⁺; "+": A = pen s - G - (1-θ)K, w = θ s - τJ, D = -α⁺ w, F = c²⁺ w;
-  // "-": A = G - pen s - θK, w = -(1-θ) s - τJ, D = α⁻ w, F = -c²⁻ w
-  const double th = F.theta, tau = F.tau, two_h = F.two_h;
-  const double c2m = F.one_sided ? cf.c2m : cf.c2p, afm = F.one_sided ? cf.afm : cf.afp;
-  const double c2p = cf.c2p, afp = cf.afp;
-  const double g_um = two_h * ((1 - th) * c2m), g_up = two_h * (th * c2p);
-  const double g_vm = two_h * ((1 - th) * afm), g_vp = two_h * (th * afp);
-  const double j_um = two_h * c2m, j_up = -(two_h * c2p), j_vm = two_h * afm, j_vp = -(two_h * afp);
-  const double pen = (0.5 * (c2m + c2p)) * F.lu + (0.5 * (afm + afp)) * F.lv;
-  const double sw = plus ? th : -(1 - th);                 // w = sw s - τJ
-  const double kA = plus ? -(1 - th) : -th;                // A = ±(pen s - G) + kA K
-  const double dD = plus ? -afp : afm, dF = plus ? c2p : -c2m;
-  const size_t fstride = (size_t)(N + 1) * N;              // from point (mode) b to b + 1
-  const double *tr = F.tr;
-  // mode b of trace family fam on side `side` of element el
-  auto T = [&](int fam, int side, int el, int b) { return tr[((fam * 4 + side) * NQ + b) * E + el]; };
+  const int N = F.N, E = F.E, lane = threadIdx.x & 31, tw = lane / NQ, i = lane - tw * NQ;
+  const int x = side0 + tw;
+  if (tw >= bnd_tile(NU) || x >= 4 * N) return;
+  if (err_word(F) != ERR_NONE) return;
+  const unsigned mask = ((1u << NQ) - 1u) << (tw * NQ);
+  const TimeF tf = time_factors(S);
+  const int s = x / N, m = x - s * N;
+  const int j = s == 0 ? 0 : s == 1 ? N - 1 : m, k = s == 2 ? 0 : s == 3 ? N - 1 : m, e = j + N * k;
+  double A, D, Fs;
+  boundary_point<NU, NV>(B, F, tf, s, j, k, e, i, A, D, Fs);
+  double ya = 0.0, yd = 0.0, yf = 0.0;
 #pragma unroll
-  for (int b = 0; b < NU; ++b) {
-    const double dum = T(0, sm, em, b), dup = T(0, spp, ep, b);
-    double G = fma(g_um, dum, g_up * dup), J = fma(j_um, dum, j_up * dup), sj = 0.0;
-    if (b < NV) {
-      const double vm = T(1, sm, em, b), vp = T(1, spp, ep, b);
-      const double dvm = T(2, sm, em, b), dvp = T(2, spp, ep, b);
-      G = fma(g_vp, dvp, fma(g_vm, dvm, G));
-      J = fma(j_vp, dvp, fma(j_vm, dvm, J));
-      sj = vm - vp;
-    }
-    const double K = jcm ? jcm[fi + fstride * b] : 0.0;
-    J += K;
-    const double w = fma(sw, sj, -tau * J);
-    if (b < NV) {
-      const double a = fma(pen, sj, -G);
-      YA[b] = fma(kA, K, plus ? a : -a);
-      YD[b] = dD * w;
-    }
-    YF[b] = dF * w;
+  for (int q = 0; q < NQ; ++q) {
+    const double p = B.Pw[q][i];
+    ya = fma(p, __shfl_sync(mask, A, tw * NQ + q), ya);
+    yd = fma(p, __shfl_sync(mask, D, tw * NQ + q), yd);
+    yf = fma(p, __shfl_sync(mask, Fs, tw * NQ + q), yf);
+  }
+  double *o = F.bslots + x;
+  const size_t st = (size_t)4 * N;
+  if (i < NV) {
+    o[i * st] = ya;
+    o[(NV + i) * st] = yd;
+  }
+  o[(2 * NV + i) * st] = yf;
+}
+template <int NU, int NV>
+__global__ void __launch_bounds__(BND_THREADS) k_bnd(const __grid_constant__ Basis<NU, NV> B,
+                                                     const __grid_constant__ Fields F,
+                                                     const __grid_constant__ StageIO S) {
+  bnd_body<NU, NV>(B, F, S, blockIdx.x * bnd_tile(NU));
+}
+// tile = bnd_tile(NU) sides per virtual block, of the 4N of an instance
+template <int NU, int NV>
+__global__ void __launch_bounds__(BND_THREADS) k_bnd_m(const __grid_constant__ Basis<NU, NV> B,
+                                                       const __grid_constant__ MultiStage P) {
+  for (int vb = blockIdx.x; vb < P.first[P.n]; vb += gridDim.x) {
+    const int inst = multi_begin(P, vb);
+    bnd_body<NU, NV>(B, P.a[inst].F, P.a[inst].S, (vb - P.first[inst]) * P.tile);
   }
 }
 
-// ----------------------------------------------------------------------------
-// k_stage: fluxes, lifts, volume, source, u-equation; the mass right-hand side to HBM
-// ----------------------------------------------------------------------------
-// k_stage's work for element e, whose blocks live in the shared-memory slot tid of the block
-template <int NU, int NV, bool FAST>
-__device__ __forceinline__ void stage_body(const Basis<NU, NV> &B, const Fields &F, const StageIO &S, int e,
-                                           int tid) {
-  constexpr int NQ = NU, BT = stage_threads(NU, NV, FAST);
-  extern __shared__ double smem[];
-  const int E = F.E, N = F.N;
+// Count of Chebyshev steps for the interval θ ± δ: ceil(L / acosh(θ/δ)), from FP32 where that is not within its
+// rounding of a whole number (acosh costs some 100 FP64 operations)
+__device__ __forceinline__ int cheb_count(double L, double th, double de) {
+  const float x = (float)L / acoshf((float)th / (float)de), r = rintf(x);
+  if (x < 1e6f && fabsf(x - r) > 1e-4f * x + 1e-4f) return (int)ceilf(x);
+  return (int)ceil(L / acosh(th / de));
+}
+
+// k_prep: a team of NU threads per element. Thread r takes the sums over the normal modes at mode r of
+// the four sides (column r and row r of the blocks), the r-th face point, column r of P_h V and the
+// point rows r, r + NU, ... With a thread per element a warp held the chip's FP64 pipes for the
+// whole of its 378 trace operations and two blocks of state per thread; the team fills them from more
+// warps and spreads small meshes over the chip.
+template <int NU, int NV>
+struct PrepTeam {
+  static constexpr int QH = qhigh(NU, NV), TPW = 32 / NU;
+  static constexpr int S0 = NU * NU + NV * NV, S1 = 12 * NU, S2 = QH * NV;
+  static constexpr int SLOT = (S0 > S1 ? (S0 > S2 ? S0 : S2) : S1 > S2 ? S1 : S2) | 1;   // odd: bank conflicts
+};
+__host__ __device__ constexpr int prep_tile(int nu, int threads) { return (threads / 32) * (32 / nu); }
+
+// The block's elements from e0 on (first: the instance's first block, which clears the bin counts)
+template <int NU, int NV>
+__device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &F, const StageIO &S, int e0,
+                                          bool first) {
+  using T = PrepTeam<NU, NV>;
+  constexpr int NQ = NU, QH = T::QH;
+  __shared__ double sh[T::TPW * 4 * T::SLOT];
+  __shared__ double Ps[NQ * NU];
+  const int E = F.E;
+  // the bin counts and the largest count of the next stage start at zero: all NBIN bins, whatever
+  // the element count
+  if (first && F.sorted)
+    for (int b = threadIdx.x; b < NBIN; b += blockDim.x) F.bin_count[(1 - S.parity) * NBIN + b] = 0;
+  if (first && threadIdx.x == 0) F.nmax[1 - S.parity] = 0;
+  for (int i = threadIdx.x; i < NQ * NU; i += blockDim.x) Ps[i] = B.P[i / NU][i % NU];
+  __syncthreads();
+  const int lane = threadIdx.x & 31, tw = lane / NU;
+  if (tw >= T::TPW) return;
+  const int r = lane - tw * NU, slot = (threadIdx.x >> 5) * T::TPW + tw, e = e0 + slot;
   if (e >= E) return;
   if (err_word(F) != ERR_NONE) return;
-  const int j = e % N, k = e / N;
-  const double two_h = F.two_h, four_hh = F.four_hh;
-  const TimeF tf = time_factors(S);
-  // thread-private blocks: b (NU², the u-equation right-hand side, then UT) and R_v (NV², the
-  // v-equation right-hand side; in the general kernels its space, NU², then takes UT)
-  Blk<NU, BT> bb{smem + tid};
-  Blk<NV, BT> Rv{smem + NU * NU * BT + tid};
-
-  // ---- faces and lifts (src/rhs.jl:421-473): Rv (v-equation), b = -Fu (u-equation).
-  //      The numerical flux slots A, D, F of a side are projected on the modes, Y[b] =
-  //      Σ_i w_i P[i][b] (.)_i, from the sums (even b) and differences (odd b) of mirrored points,
-  //      and the two sides of an axis are lifted together: the right-end factors are the
-  //      left-end ones times ±(-1)^a, so both sides need one rank-one update per slot.
-#pragma unroll 1
-  for (int a = 0; a < NV; ++a)
-#pragma unroll
-    for (int b = 0; b < NV; ++b) Rv(a, b) = 0.0;
-#pragma unroll 1
-  for (int a = 0; a < NU; ++a)
-#pragma unroll
-    for (int b = 0; b < NU; ++b) bb(a, b) = S.mode == OUT_ADJ_USOLVE ? S.xu[e + (size_t)E * (a + NU * b)] : 0.0;
-  const bool adjoint = S.mode >= OUT_ADJ_USOLVE;
-  // the forward modes of the constant-coefficient kernels build the u-equation's right-hand side
-  // in the eigenbasis of K1 (the adjoint's volume mode needs the plain basis)
-  const bool eig = FAST && !adjoint;
-#pragma unroll 1
-  for (int ax = 0; ax < 2 && !adjoint; ++ax) {
-    double A0[NV], D0[NV], F0[NU];          // the projections of the axis' first side (B or L)
-    double YA[NV], YD[NV], YF[NU];
-#pragma unroll 1
-    for (int t = 0; t < 2; ++t) {
-      const int s = 2 * ax + t;
-      const bool boundary = (s == 0 && j == 0) || (s == 1 && j == N - 1) || (s == 2 && k == 0) || (s == 3 && k == N - 1);
-#pragma unroll
-      for (int b = 0; b < NU; ++b) {
-        if (b < NV) { YA[b] = 0.0; YD[b] = 0.0; }
-        YF[b] = 0.0;
-      }
-      if (F.modal && !boundary) {
-        modal_side<NU, NV>(F, s, j, k, e, YA, YD, YF);
-      } else {
-#pragma unroll 1
-        for (int i = 0; i < NQ / 2; ++i) {
-          double A1, D1, F1, A2, D2, F2;
-          side_point<NU, NV>(B, F, tf, s, boundary, j, k, e, i, A1, D1, F1);
-          side_point<NU, NV>(B, F, tf, s, boundary, j, k, e, NQ - 1 - i, A2, D2, F2);
-          const double as = A1 + A2, ad = A1 - A2, ds = D1 + D2, dd = D1 - D2, fs = F1 + F2, fd = F1 - F2;
-#pragma unroll
-          for (int b = 0; b < NU; ++b) {
-            const double p = B.Pw[i][b];
-            if (b < NV) {
-              YA[b] = fma(p, (b & 1) ? ad : as, YA[b]);
-              YD[b] = fma(p, (b & 1) ? dd : ds, YD[b]);
-            }
-            YF[b] = fma(p, (b & 1) ? fd : fs, YF[b]);
-          }
-        }
-        if constexpr ((NQ & 1) != 0) {         // the middle point: the odd modes vanish there
-          double A1, D1, F1;
-          side_point<NU, NV>(B, F, tf, s, boundary, j, k, e, NQ / 2, A1, D1, F1);
-#pragma unroll
-          for (int b = 0; b < NU; b += 2) {
-            const double p = B.Pw[NQ / 2][b];
-            if (b < NV) {
-              YA[b] = fma(p, A1, YA[b]);
-              YD[b] = fma(p, D1, YD[b]);
-            }
-            YF[b] = fma(p, F1, YF[b]);
-          }
-        }
-      }
-      if (t == 0) {
-#pragma unroll
-        for (int b = 0; b < NU; ++b) {
-          if (b < NV) { A0[b] = YA[b]; D0[b] = YD[b]; }
-          F0[b] = YF[b];
-        }
-      }
-    }
-    // lifts of both sides: with σ_a = (-1)^a, El = the left-end values, E1l the left-end
-    // derivatives, Rv += El ⊗ (2/h)(A_0 + σ A_1) + E1l ⊗ (4/h²)(D_0 - σ D_1) and
-    // b -= E1l ⊗ (F_0 - σ F_1) (B/T: the row index carries E; L/R: the column index)
-#pragma unroll
-    for (int b = 0; b < NU; ++b) {
-      if (b < NV) {
-        const double ap = A0[b] + YA[b], am = A0[b] - YA[b], dp = D0[b] + YD[b], dm = D0[b] - YD[b];
-        // even-σ and odd-σ combinations, with the mesh factors of the v-slots
-        A0[b] = two_h * ap; YA[b] = two_h * am; D0[b] = four_hh * dm; YD[b] = four_hh * dp;
-      }
-      const double fp = F0[b] + YF[b], fm = F0[b] - YF[b];
-      F0[b] = fm; YF[b] = fp;
-    }
-    if (eig) {
-      // the u-slots' lifts straight into the eigenbasis of K1: Q^T (E1F_even ⊗ F_0 + E1F_odd ⊗ F_1) Q
-      // = QE_even ⊗ Q^T F_0 + QE_odd ⊗ Q^T F_1 (QE = Q^T E1F keeps the parity of its index)
-      double t0[NU], t1[NU];
-#pragma unroll
-      for (int i = 0; i < NU; ++i) { t0[i] = 0.0; t1[i] = 0.0; }
-#pragma unroll
-      for (int a = 0; a < NU; ++a)
-#pragma unroll
-        for (int i = 0; i < NU; ++i)
-          if (qnz(a, i)) { t0[i] = fma(B.Q[a][i], F0[a], t0[i]); t1[i] = fma(B.Q[a][i], YF[a], t1[i]); }
-#pragma unroll
-      for (int i = 0; i < NU; ++i) { F0[i] = t0[i]; YF[i] = t1[i]; }
-    }
-    const double *LF = eig ? B.QE : B.E1F;
-    if (ax == 0) {
-#pragma unroll 1
-      for (int a = 0; a < NV; ++a) {
-        const double ca = B.El[a], cd = B.E1l[a];
-        const bool od = a & 1;
-#pragma unroll
-        for (int b = 0; b < NV; ++b)
-          Rv(a, b) = fma(cd, od ? YD[b] : D0[b], fma(ca, od ? YA[b] : A0[b], Rv(a, b)));
-      }
-#pragma unroll 1
-      for (int a = 0; a < NU; ++a) {
-        const double ce = LF[a];
-        const bool od = a & 1;
-#pragma unroll
-        for (int b = 0; b < NU; ++b) bb(a, b) = fma(ce, od ? YF[b] : F0[b], bb(a, b));
-      }
-    } else {
-#pragma unroll
-      for (int a = 0; a < NV; ++a) {
-#pragma unroll
-        for (int b = 0; b < NV; ++b)
-          Rv(a, b) = fma(B.E1l[b], (b & 1) ? YD[a] : D0[a], fma(B.El[b], (b & 1) ? YA[a] : A0[a], Rv(a, b)));
-      }
-#pragma unroll
-      for (int a = 0; a < NU; ++a) {
-#pragma unroll
-        for (int b = 0; b < NU; ++b) bb(a, b) = fma(LF[b], (b & 1) ? YF[a] : F0[a], bb(a, b));
-      }
-    }
-  }
-
-  // ---- the state of the stage is read from HBM (by rows of modes in the general kernels, by
-  //      columns and by rows in the constant-coefficient kernels)
+  const unsigned mask = ((1u << NU) - 1u) << (tw * NU);
   const size_t Eu = (size_t)E;
-  if (S.mode != OUT_ADJ_USOLVE) {
-
-  // ---- volume terms (src/rhs.jl:309-333): Rv += -4/h² [(c²∇φ_v,∇u_h) + (α∇φ_v,∇v_h)],
-  //      b += (c²∇φ_u, ∇v_h)
-  if constexpr (FAST) {
-    // constant c², α on the element: Cw = c² W, Aw = α W, so that with the
-    // 1D stiffness K1 = S^T diag(w) S and the orthonormality of the basis
-    //   (c²∇φ_v,∇u_h) + (α∇φ_v,∇v_h) = (K1 W + W K1)[v-block] / (-4/h²),  W = -4/h² (c² U + α V)
-    //   (c²∇φ_u, ∇v_h) = c² (K1[:, v] V + V K1[v, :])
-    // (V padded with zeros to NU × NU; row and column 0 of K1 vanish, and K1 couples only modes
-    // of equal parity). The products with K1 from the left take the columns of U and V, those
-    // from the right their rows: both are read from HBM (L2), so that U and V need no shared
-    // memory.
-    const double c2 = F.c2e[e], al = F.ae[e];
-    const double mc2 = -four_hh * c2, mal = -four_hh * al;
-    const double *xu = S.xu + e, *xv = S.xv + e;
-#pragma unroll 1
-    for (int b = 0; b < NV; ++b) {                  // columns: K1 W and K1[:, v] V
-      double w[NU], vc[NV];
-#pragma unroll
-      for (int c = 1; c < NU; ++c) {
-        const double uc = xu[Eu * (c + NU * b)];
-        if (c < NV) {
-          const double x = xv[Eu * (c + NV * b)];
-          w[c] = fma(mal, x, mc2 * uc);
-          vc[c] = c2 * x;
-        } else {
-          w[c] = mc2 * uc;
-        }
-      }
-#pragma unroll
-      for (int a = 1; a < NU; ++a) {
-        if (a < NV) {
-          double acc = Rv(a, b);
-#pragma unroll
-          for (int c = 2 - (a & 1); c < NU; c += 2) acc = fma(B.K1[a][c], w[c], acc);
-          Rv(a, b) = acc;
-        }
-        if (!eig) {
-          double acc = bb(a, b);
-#pragma unroll
-          for (int c = 2 - (a & 1); c < NV; c += 2) acc = fma(B.K1[a][c], vc[c], acc);
-          bb(a, b) = acc;
-        }
-      }
-    }
-#pragma unroll 1
-    for (int a = 0; a < NV; ++a) {                  // rows: W K1 and V K1[v, :]
-      double w[NU], vr[NV];
-#pragma unroll
-      for (int c = 1; c < NU; ++c) {
-        const double uc = xu[Eu * (a + NU * c)];
-        if (c < NV) {
-          const double x = xv[Eu * (a + NV * c)];
-          w[c] = fma(mal, x, mc2 * uc);
-          vr[c] = c2 * x;
-        } else {
-          w[c] = mc2 * uc;
-        }
-      }
-#pragma unroll
-      for (int b = 1; b < NU; ++b) {
-        if (b < NV) {
-          double acc = Rv(a, b);
-#pragma unroll
-          for (int c = 2 - (b & 1); c < NU; c += 2) acc = fma(w[c], B.K1[c][b], acc);
-          Rv(a, b) = acc;
-        }
-        if (!eig) {
-          double acc = bb(a, b);
-#pragma unroll
-          for (int c = 2 - (b & 1); c < NV; c += 2) acc = fma(vr[c], B.K1[c][b], acc);
-          bb(a, b) = acc;
-        }
-      }
-    }
-  } else {
-#pragma unroll 1
-    for (int r = 0; r < NQ; ++r) {
-      // row r of G1 = S U P^T, G2 = P U S^T and of the same for V
-      double tu1[NU], tu2[NU], tv1[NV], tv2[NV];
-#pragma unroll
-      for (int b = 0; b < NU; ++b) { tu1[b] = 0; tu2[b] = 0; }
-#pragma unroll
-      for (int b = 0; b < NV; ++b) { tv1[b] = 0; tv2[b] = 0; }
-#pragma unroll 1
-      for (int a = 0; a < NU; ++a) {
-        const double sa = B.S[r][a], pa = B.P[r][a];
-#pragma unroll
-        for (int b = 0; b < NU; ++b) {
-          const double x = S.xu[e + Eu * (a + NU * b)];
-          tu1[b] = fma(sa, x, tu1[b]);
-          tu2[b] = fma(pa, x, tu2[b]);
-        }
-        if (a < NV) {
-#pragma unroll
-          for (int b = 0; b < NV; ++b) {
-            const double x = S.xv[e + Eu * (a + NV * b)];
-            tv1[b] = fma(sa, x, tv1[b]);
-            tv2[b] = fma(pa, x, tv2[b]);
-          }
-        }
-      }
-      // the row at the points: g1[s] = Σ_b tu1[b] P[s][b], g2[s] = Σ_b tu2[b] S[s][b], ... from the
-      // even and odd modes: P[m][b] = (-1)^b P[s][b] and S[m][b] = -(-1)^b S[s][b] at the mirror
-      // point m = NQ-1-s, so the point and its mirror are a sum and a difference
-      double g1[NQ], g2[NQ], gv1[NQ], gv2[NQ];
-#pragma unroll
-      for (int s2 = 0; s2 < (NQ + 1) / 2; ++s2) {
-        double pe = 0, po = 0, se = 0, so = 0, qe = 0, qo = 0, te = 0, to = 0;
-#pragma unroll
-        for (int b = 0; b < NU; ++b) {
-          const double pb = B.P[s2][b], sb = B.S[s2][b];
-          if (b & 1) {
-            po = fma(tu1[b], pb, po); so = fma(tu2[b], sb, so);
-            if (b < NV) { qo = fma(tv1[b], pb, qo); to = fma(tv2[b], sb, to); }
-          } else {
-            pe = fma(tu1[b], pb, pe); se = fma(tu2[b], sb, se);
-            if (b < NV) { qe = fma(tv1[b], pb, qe); te = fma(tv2[b], sb, te); }
-          }
-        }
-        g1[s2] = pe + po; g2[s2] = se + so; gv1[s2] = qe + qo; gv2[s2] = te + to;
-        if (2 * s2 + 1 != NQ) {
-          const int m = NQ - 1 - s2;
-          g1[m] = pe - po; g2[m] = so - se; gv1[m] = qe - qo; gv2[m] = to - te;
-        }
-      }
-      // weighted by the coefficients, back to the modes: z1[b] = Σ_s h1[s] P[s][b], ... from the
-      // sums and differences of mirrored points
-      double h1[NQ], h2[NQ], b1[NQ], b2[NQ];
-#pragma unroll
-      for (int s2 = 0; s2 < NQ; ++s2) {
-        const size_t ci = (r + NQ * s2) * Eu + e;
-        const double cw = F.Cw[ci], aw = F.Aw[ci];
-        h1[s2] = fma(aw, gv1[s2], cw * g1[s2]);
-        h2[s2] = fma(aw, gv2[s2], cw * g2[s2]);
-        b1[s2] = cw * gv1[s2];
-        b2[s2] = cw * gv2[s2];
-      }
-      double z1[NV], z2[NV], y1[NU], y2[NU];
-#pragma unroll
-      for (int b = 0; b < NV; ++b) { z1[b] = 0; z2[b] = 0; }
-#pragma unroll
-      for (int b = 0; b < NU; ++b) { y1[b] = 0; y2[b] = 0; }
-#pragma unroll
-      for (int s2 = 0; s2 < (NQ + 1) / 2; ++s2) {
-        const bool mid = 2 * s2 + 1 == NQ;
-        const int m = NQ - 1 - s2;
-        // P-weighted: even modes take the sum, odd the difference; S-weighted: the opposite
-        const double h1s = mid ? h1[s2] : h1[s2] + h1[m], h1d = mid ? 0.0 : h1[s2] - h1[m];
-        const double h2s = mid ? h2[s2] : h2[s2] + h2[m], h2d = mid ? 0.0 : h2[s2] - h2[m];
-        const double b1s = mid ? b1[s2] : b1[s2] + b1[m], b1d = mid ? 0.0 : b1[s2] - b1[m];
-        const double b2s = mid ? b2[s2] : b2[s2] + b2[m], b2d = mid ? 0.0 : b2[s2] - b2[m];
-#pragma unroll
-        for (int b = 0; b < NU; ++b) {
-          const double pb = B.P[s2][b], sb = B.S[s2][b];
-          const bool odd = b & 1;
-          if (b < NV) {
-            z1[b] = fma(odd ? h1d : h1s, pb, z1[b]);
-            z2[b] = fma(odd ? h2s : h2d, sb, z2[b]);
-          }
-          y1[b] = fma(odd ? b1d : b1s, pb, y1[b]);
-          y2[b] = fma(odd ? b2s : b2d, sb, y2[b]);
-        }
-      }
-#pragma unroll
-      for (int b = 0; b < NV; ++b) { z1[b] *= -four_hh; z2[b] *= -four_hh; }
-#pragma unroll 1
-      for (int a = 0; a < NV; ++a) {
-        const double sa = B.S[r][a], pa = B.P[r][a];
-#pragma unroll
-        for (int b = 0; b < NV; ++b) Rv(a, b) = fma(sa, z1[b], fma(pa, z2[b], Rv(a, b)));
-      }
-#pragma unroll 1
-      for (int a = 0; a < NU; ++a) {
-        const double sa = B.S[r][a], pa = B.P[r][a];
-#pragma unroll
-        for (int b = 0; b < NU; ++b) bb(a, b) = fma(sa, y1[b], fma(pa, y2[b], bb(a, b)));
-      }
-    }
-  }
-
-  }   // volume terms
-
-  if (S.mode == OUT_ADJ_VOLUME) {
-#pragma unroll 1
-    for (int b = 0; b < NV; ++b)
-#pragma unroll
-      for (int a = 0; a < NV; ++a) S.vt[e + Eu * (a + NV * b)] = Rv(a, b);
-#pragma unroll 1
-    for (int b = 0; b < NU; ++b)
-#pragma unroll
-      for (int a = 0; a < NU; ++a) S.ut[e + Eu * (a + NU * b)] = bb(a, b);
-    return;
-  }
-
-  // ---- source (src/rhs.jl:340-350), and the mass right-hand side to HBM
-#pragma unroll 1
-  for (int b = 0; b < NV && !adjoint; ++b)
-#pragma unroll
-    for (int a = 0; a < NV; ++a) {
-      const size_t l = (a + NV * b) * Eu + e;
-      double x = Rv(a, b);
-      if (F.mms_on) {
-        x = fma(tf.cSP, F.PiSP[l], x);
-        x = fma(tf.cB, F.PiBSP2[l], x);
-        x = fma(tf.cC, F.PiCdiv[l], x);
-        x = fma(tf.cD, F.PiDdiv[l], x);
-      } else if (!F.src_on) {
-        x += F.PiCdiv[l];
-      }
-      if (F.src_on) x = fma(tf.srct, F.srcP[l], x);
-      F.mrhs[l] = x;
-    }
-
-  // ---- u-equation (src/rhs.jl:352-382): A_e UT = VB - Fu + e_1 V[0][0]
-  if (!adjoint) {
-    bb(0, 0) += S.xv[e];
-  }
-  // UT: in place of b (constant-coefficient kernels), in the space of R_v (general kernels: R_v is
-  // spent once the mass right-hand side is written)
-  Blk<NU, BT> UT = FAST ? bb : Blk<NU, BT>{smem + NU * NU * BT + tid};
-  if constexpr (FAST) {
-    // A_e = c² (K1 ⊗ I + I ⊗ K1) + e_0 e_0^T is diagonal in the eigenbasis Q ⊗ Q of K1 (whose
-    // first eigenvector is e_0 with λ_0 = 0): UT = Q [ (Q^T b Q) ∘ L ] Q^T, L = 1/(c²(λ_i+λ_j)), 1 at (0,0).
-    // Q[a][i] vanishes for a + i odd and in row and column 0 outside (0, 0): qnz skips those
-    // terms at compile time. The four products run in place: a product with Q from the left
-    // changes each column on its own, one from the right each row.
-    const double ic2 = F.ic2e[e];
-    if (eig) {
-      if constexpr (NU != NV) {
-      // as below, Ṽ accumulated column by column of V (padded with zeros to NU × NU): with
-      // t = Q^T V[:, c], X += t ⊗ Q[c, :] (R_v's space is too small for Q^T V here)
-#pragma unroll 1
-      for (int i = 0; i < NU; ++i)
-#pragma unroll
-        for (int jj = 0; jj < NU; ++jj)
-          if (i != 0 || jj != 0) bb(i, jj) = bb(i, jj) * (B.ilam2[i][jj] * ic2);
-#pragma unroll 1
-      for (int c = 0; c < NV; ++c) {
-        double t[NU], x[NV];
-#pragma unroll
-        for (int a = 0; a < NV; ++a) x[a] = S.xv[e + Eu * (a + NV * c)];
-#pragma unroll
-        for (int i = 0; i < NU; ++i) t[i] = 0;
-#pragma unroll
-        for (int a = 0; a < NV; ++a)
-#pragma unroll
-          for (int i = 0; i < NU; ++i)
-            if (qnz(a, i)) t[i] = fma(B.Q[a][i], x[a], t[i]);
-#pragma unroll
-        for (int i = 0; i < NU; ++i)
-#pragma unroll
-          for (int jj = 0; jj < NU; ++jj)
-            if (qnz(c, jj) && (i != 0 || jj != 0)) bb(i, jj) = fma(t[i], B.Q[c][jj], bb(i, jj));
-      }
-      } else {
-      // b is in the eigenbasis except for its volume part c²(K1 V + V K1), whose transform
-      // c²(Λ Ṽ + Ṽ Λ), Ṽ = Q^T V Q, divided by c²(λ_i + λ_j) is Ṽ itself (zero at (0, 0)):
-      // X = Ṽ + (Q^T b' Q) ∘ L. T1 = Q^T V by columns into the space of R_v (written out above),
-      // then X = T1 Q + b' ∘ L by rows.
-      Blk<NV, BT> T1 = Rv;
-#pragma unroll 1
-      for (int c = 0; c < NU; ++c) {
-        double t[NU], x[NU];
-#pragma unroll
-        for (int a = 0; a < NU; ++a) x[a] = S.xv[e + Eu * (a + NU * c)];
-#pragma unroll
-        for (int i = 0; i < NU; ++i) t[i] = 0;
-#pragma unroll
-        for (int a = 0; a < NU; ++a)
-#pragma unroll
-          for (int i = 0; i < NU; ++i)
-            if (qnz(a, i)) t[i] = fma(B.Q[a][i], x[a], t[i]);
-#pragma unroll
-        for (int i = 0; i < NU; ++i) T1(i, c) = t[i];
-      }
-#pragma unroll 1
-      for (int i = 0; i < NU; ++i) {
-        double t[NU];
-#pragma unroll
-        for (int jj = 0; jj < NU; ++jj) t[jj] = 0;
-#pragma unroll
-        for (int c = 0; c < NU; ++c) {
-          const double x = T1(i, c);
-#pragma unroll
-          for (int jj = 0; jj < NU; ++jj)
-            if (qnz(c, jj)) t[jj] = fma(x, B.Q[c][jj], t[jj]);
-        }
-#pragma unroll
-        for (int jj = 0; jj < NU; ++jj)
-          bb(i, jj) = (i == 0 && jj == 0) ? bb(0, 0) : fma(bb(i, jj), B.ilam2[i][jj] * ic2, t[jj]);
-      }
-      }
-    } else {
-#pragma unroll 1
-    for (int c = 0; c < NU; ++c) {                 // T1 = Q^T b, by columns
-      double t[NU];
-#pragma unroll
-      for (int i = 0; i < NU; ++i) t[i] = 0;
-#pragma unroll
-      for (int a = 0; a < NU; ++a) {
-        const double x = bb(a, c);
-#pragma unroll
-        for (int i = 0; i < NU; ++i)
-          if (qnz(a, i)) t[i] = fma(B.Q[a][i], x, t[i]);
-      }
-#pragma unroll
-      for (int i = 0; i < NU; ++i) bb(i, c) = t[i];
-    }
-#pragma unroll 1
-    for (int i = 0; i < NU; ++i) {                 // T2 = (T1 Q) ∘ L, by rows
-      double t[NU];
-#pragma unroll
-      for (int jj = 0; jj < NU; ++jj) t[jj] = 0;
-#pragma unroll
-      for (int c = 0; c < NU; ++c) {
-        const double x = bb(i, c);
-#pragma unroll
-        for (int jj = 0; jj < NU; ++jj)
-          if (qnz(c, jj)) t[jj] = fma(x, B.Q[c][jj], t[jj]);
-      }
-#pragma unroll
-      for (int jj = 0; jj < NU; ++jj) bb(i, jj) = (i == 0 && jj == 0) ? t[jj] : t[jj] * (B.ilam2[i][jj] * ic2);
-    }
-    }
-#pragma unroll 1
-    for (int jj = 0; jj < NU; ++jj) {              // T3 = Q T2, by columns
-      double t[NU];
-#pragma unroll
-      for (int a = 0; a < NU; ++a) t[a] = 0;
-#pragma unroll
-      for (int i = 0; i < NU; ++i) {
-        const double x = bb(i, jj);
-#pragma unroll
-        for (int a = 0; a < NU; ++a)
-          if (qnz(a, i)) t[a] = fma(B.Q[a][i], x, t[a]);
-      }
-#pragma unroll
-      for (int a = 0; a < NU; ++a) bb(a, jj) = t[a];
-    }
-#pragma unroll 1
-    for (int a = 0; a < NU; ++a) {                 // UT = T3 Q^T, by rows
-      double t[NU];
-#pragma unroll
-      for (int c = 0; c < NU; ++c) t[c] = 0;
-#pragma unroll
-      for (int jj = 0; jj < NU; ++jj) {
-        const double x = bb(a, jj);
-#pragma unroll
-        for (int c = 0; c < NU; ++c)
-          if (qnz(c, jj)) t[c] = fma(x, B.Q[c][jj], t[c]);
-      }
-#pragma unroll
-      for (int c = 0; c < NU; ++c) bb(a, c) = t[c];
-    }
-  } else {
-    // packed upper triangle of the symmetric inverse, by columns: entry (i, j), i ≤ j, in row j(j+1)/2 + i
-    constexpr int n = NU * NU;
-    double *X = &UT(0, 0), *bv = &bb(0, 0);       // UT and b as vectors a + NU c
-#pragma unroll 1
-    for (int i = 0; i < n; ++i) X[i * BT] = 0.0;
-    // two columns jj, jj + 1 per pass: one read-modify-write of X[i] for both, twice the
-    // independent loads of Ainv in flight
-#pragma unroll 1
-    for (int jj = 0; jj + 1 < n; jj += 2) {
-      const double bj = bv[jj * BT], bk = bv[(jj + 1) * BT];
-      const double *Aj = F.Ainv + (size_t)(jj * (jj + 1) / 2) * Eu + e;
-      const double *Ak = Aj + (size_t)(jj + 1) * Eu;
-      double sj = 0, sk = 0;
-#pragma unroll 8
-      for (int i = 0; i < jj; ++i) {
-        const double a = Aj[(size_t)i * Eu], c = Ak[(size_t)i * Eu];
-        const double bi = bv[i * BT];
-        X[i * BT] = fma(c, bk, fma(a, bj, X[i * BT]));
-        sj = fma(a, bi, sj);
-        sk = fma(c, bi, sk);
-      }
-      // the 2 × 2 corner: (jj, jj), (jj, jj + 1), (jj + 1, jj + 1)
-      const double ajj = Aj[(size_t)jj * Eu], ajk = Ak[(size_t)jj * Eu], akk = Ak[(size_t)(jj + 1) * Eu];
-      X[jj * BT] = fma(ajk, bk, fma(ajj, bj, X[jj * BT] + sj));
-      X[(jj + 1) * BT] = fma(akk, bk, fma(ajk, bj, X[(jj + 1) * BT] + sk));
-    }
-    if constexpr ((n & 1) != 0) {
-      const int jj = n - 1;
-      const double bj = bv[jj * BT];
-      const double *Aj = F.Ainv + (size_t)(jj * (jj + 1) / 2) * Eu + e;
-      double sj = 0;
-#pragma unroll 4
-      for (int i = 0; i < jj; ++i) {
-        const double a = Aj[(size_t)i * Eu];
-        X[i * BT] = fma(a, bj, X[i * BT]);
-        sj = fma(a, bv[i * BT], sj);
-      }
-      X[jj * BT] = fma(Aj[(size_t)jj * Eu], bj, X[jj * BT] + sj);
-    }
-  }
-
-  // ---- u outputs: RK4 (src/solver.jl:289-321): acc = k1 + 2 k2 + 2 k3 in this order, the next
-  //      stage state u + c k, the last stage u + (dt/6)(acc + k4) with the finite check
-  bool fin = true;
-#pragma unroll 1
-  for (int b = 0; b < NU; ++b)
+  const bool has_v = r < NV, modal = F.modal != 0;
+  double *Us = sh + slot * T::SLOT, *Vs = Us + NU * NU;
+  // ---- traces (src/rhs.jl:388-410): the sums over the normal modes, at mode r: family x (du, v, dv) of the
+  //      low and the high side of both axes; El, Er are the values or derivatives of the modes at the
+  //      two ends, Er[a] = ±(-1)^a El[a], so both ends come from the even and odd parts of one sum
+  double V[NV];
+  double lo[3][2], hi[3][2];
+  int hu = 0, hv = 0;                                    // the largest high words beside the constant mode
+  auto ends = [&](double xe, double xo, bool der, double &l, double &h) {
+    l = xe + xo;
+    h = der ? xo - xe : xe - xo;
+  };
+  {
+    double U[NU];
 #pragma unroll
     for (int a = 0; a < NU; ++a) {
-      const size_t l = e + Eu * (a + NU * b);
-      const double kk = UT(a, b);
-      if (S.mode == OUT_RHS || S.mode == OUT_ADJ_USOLVE) {
-        S.ut[l] = kk;
-      } else if (S.mode == OUT_RK4_STAGE) {
-        S.accu[l] = S.first ? kk : S.accu[l] + 2.0 * kk;
-        S.su[l] = S.u0[l] + S.c * kk;
-      } else if (S.mode == OUT_RK4_LAST) {
-        // Chebyshev mode only: no error can arise after k_prep, so u is updated in place now
-        const double x = S.u0[l] + S.c * (S.accu[l] + kk);
-        S.uo[l] = x;
-        fin = fin && isfinite(x);
-      } else {
-        S.accu[l] = S.accu[l] + kk;
-      }
+      U[a] = S.xu[e + Eu * (a + NU * r)];
+      Us[a + NU * r] = U[a];
+      if (a + r > 0) hu = max(hu, fx_abs_hi(U[a]));
     }
-  if (S.mode == OUT_RK4_LAST && !fin) atomicOr(F.nonfinite, 1u);
+#pragma unroll
+    for (int a = 0; a < NV; ++a) {
+      V[a] = has_v ? S.xv[e + Eu * (a + NV * r)] : 0.0;
+      if (has_v) Vs[a + NV * r] = V[a];
+      if (a + r > 0) hv = max(hv, fx_abs_hi(V[a]));
+    }
+    __syncwarp(mask);
+#pragma unroll
+    for (int ax = 0; ax < 2; ++ax) {
+      double ue = 0, uo = 0, ve = 0, vo = 0, de = 0, d_o = 0;
+#pragma unroll
+      for (int a = 0; a < NU; ++a) {
+        const double x = ax == 0 ? U[a] : Us[r + NU * a];
+        if (a & 1) uo = fma(B.E1l[a], x, uo); else ue = fma(B.E1l[a], x, ue);
+        if (a < NV) {
+          const double y = ax == 0 ? V[a] : has_v ? Vs[r + NV * a] : 0.0;
+          if (a & 1) { vo = fma(B.El[a], y, vo); d_o = fma(B.E1l[a], y, d_o); }
+          else { ve = fma(B.El[a], y, ve); de = fma(B.E1l[a], y, de); }
+        }
+      }
+      ends(ue, uo, true, lo[0][ax], hi[0][ax]);
+      ends(ve, vo, false, lo[1][ax], hi[1][ax]);
+      ends(de, d_o, true, lo[2][ax], hi[2][ax]);
+    }
+  }
+  hu = __reduce_max_sync(mask, hu);
+  hv = __reduce_max_sync(mask, hv);
+  i64 *Gi = reinterpret_cast<i64 *>(F.G);
+  if (r == 0) Gi[(size_t)(QH * QH + 1) * E + e] = (i64)hu << 32 | hv;
+  const int N = F.N, j = e % N, k = e / N;
+  const bool onb[4] = {j == 0, j == N - 1, k == 0, k == N - 1};
+  const bool check = (onb[0] && F.kind[0] != 3) || (onb[1] && F.kind[1] != 3) || (onb[2] && F.kind[2] != 3) ||
+                     (onb[3] && F.kind[3] != 3);
+  __syncwarp(mask);                                      // U, V in shared memory are spent
+  double *ss = Us;                                       // the sums, [(fam 4 + side) NU + mode]
+  if (!modal || check) {
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+#pragma unroll
+      for (int ax = 0; ax < 2; ++ax) {
+        ss[(f * 4 + 2 * ax) * NU + r] = lo[f][ax];
+        ss[(f * 4 + 2 * ax + 1) * NU + r] = hi[f][ax];
+      }
+    __syncwarp(mask);
+  }
+  // the sum over the face modes at point r
+  auto at = [&](int f, int s) {
+    double x = 0.0;
+#pragma unroll
+    for (int b = 0; b < NU; ++b)
+      if (f == 0 || b < NV) x = fma(Ps[r * NU + b], ss[(f * 4 + s) * NU + b], x);
+    return x;
+  };
+  if (modal) {             // the end sums themselves, mode r in the slot of point r
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+#pragma unroll
+      for (int ax = 0; ax < 2; ++ax)
+        if (f == 0 || has_v) {
+          F.tr[((f * 4 + 2 * ax) * NQ + r) * Eu + e] = lo[f][ax];
+          F.tr[((f * 4 + 2 * ax + 1) * NQ + r) * Eu + e] = hi[f][ax];
+        }
+  } else {
+#pragma unroll 1
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int f = 0; f < 3; ++f) F.tr[((f * 4 + s) * NQ + r) * Eu + e] = at(f, s);
+  }
+  // weight check 1 - kβv > 0 for the trace and the data on physical sides at point r
+  // (src/rhs.jl:109-110, 751-757); key of src/rhs.jl:732
+  if (check) {
+    const double st = time_factors(S).st;
+#pragma unroll 1
+    for (int s = 0; s < 4; ++s) {
+      if (!onb[s] || F.kind[s] == 3) continue;
+      const int m = s < 2 ? k : j;
+      const double bf = s < 2 ? F.hbf[(s == 0 ? 0 : N) + (size_t)(N + 1) * (k + (size_t)N * r)]
+                              : F.vbf[j + (size_t)N * ((s == 2 ? 0 : N) + (size_t)(N + 1) * r)];
+      const double v_fp = at(1, s), v_ex = -F.omega * st * F.bsp[s][m + (size_t)N * r];
+      const int bad = (1.0 - F.kb[s] * bf * v_fp <= 0.0) ? 1 : (1.0 - F.kb[s] * bf * v_ex <= 0.0) ? 2 : 0;
+      if (bad) atomicMin(F.err, 2ull * ((unsigned long long)s * NQ * N + r + (unsigned long long)m * NQ) + bad);
+    }
+  }
+  if (F.cg) return;
+
+  // ---- Chebyshev interval of the element: v_q = P_h V P_h^T, G = 2βv_q, a± = 1 - extrema(G), in fixed
+  //      point (the integers of V and 2β share an exponent over the element)
+  int hb = 0;
+#pragma unroll 1
+  for (int q = r; q < QH; q += NU)
+#pragma unroll
+    for (int s2 = 0; s2 < QH; ++s2) hb = max(hb, fx_abs_hi(F.beta2[(q + QH * s2) * Eu + e]));
+  hb = __reduce_max_sync(mask, hb);
+  hv = max(hv, __reduce_max_sync(mask, r == 0 ? fx_abs_hi(V[0]) : 0));
+  const bool nan = !fx_finite(hv) || !fx_finite(hb);
+  const int ev = fx_exp(hv), eb = fx_exp(hb) + 2;
+  Fx2 x[NV];
+  int top = 0;
+#pragma unroll
+  for (int a = 0; a < NV; ++a) {
+    const i64 y = fx_from(V[a], ev);
+    x[a] = fx_split(y);
+    top += (B.cPh[a] * ((fx_hi(y) >> 12) + 1)) >> 8;
+  }
+  // the rows T = Ph V go up by nt, the room that Σ_a max|Ph[.][a]| |V[a][b]| leaves in every column, so that
+  // v_q has the bits which the levels' headroom for any V would take (top 2^12 bounds the high words
+  // of T 2^(61 - gPh))
+  const int nt = max(__clz(__reduce_max_sync(mask, top)) - 3 - 12 + (61 - B.gPh), 0);
+  const int sG = (ev - FX_BIAS) + 2 * (61 - B.gPh) - nt + (eb - FX_BIAS) + 61;   // G = (integer) 2^sG
+  Fx2 *Ts = reinterpret_cast<Fx2 *>(Us);                 // T[q][b] at Ts[q NV + b]
+  __syncwarp(mask);                                      // the sums are spent
+  if (has_v) {
+    auto xa = [&](int a) { return x[a]; };
+#pragma unroll
+    for (int q = 0; q < (QH + 1) / 2; ++q) {
+      auto c = [&](int a) -> const FxC & { return B.fPh[q][a]; };
+      const i64 t0 = fx_dot<0, 2, NV>(xa, c), t1 = fx_dot<1, 2, NV>(xa, c);
+      Ts[q * NV + r] = fx_split((t0 + t1) << nt);
+      if (2 * q + 1 != QH) Ts[(QH - 1 - q) * NV + r] = fx_split((t0 - t1) << nt);
+    }
+  }
+  __syncwarp(mask);
+  i64 kmin = LLONG_MAX, kmax = LLONG_MIN;
+#pragma unroll 1
+  for (int q = r; q < QH; q += NU) {
+#pragma unroll
+    for (int b = 0; b < NV; ++b) x[b] = Ts[q * NV + b];
+    auto tb = [&](int b) { return x[b]; };
+    auto point = [&](i64 y, int s2) {
+      const size_t gi = (q + QH * s2) * Eu + e;
+      const i64 g = fx_mul(fx_split(y), fx_split(fx_from(F.beta2[gi], eb)));
+      Gi[gi] = g;
+      kmin = min(kmin, g);
+      kmax = max(kmax, g);
+    };
+    // v_q = Σ_b T[b] Ph[s2][b], mirrored columns s2 and QH-1-s2 together
+#pragma unroll
+    for (int s2 = 0; s2 < QH / 2; ++s2) {
+      auto c = [&](int b) -> const FxC & { return B.fPh[s2][b]; };
+      const i64 t0 = fx_dot<0, 2, NV>(tb, c), t1 = fx_dot<1, 2, NV>(tb, c);
+      point(t0 + t1, s2);
+      point(t0 - t1, QH - 1 - s2);
+    }
+    if constexpr ((QH & 1) != 0)
+      point(fx_dot<0, 2, NV>(tb, [&](int b) -> const FxC & { return B.fPh[QH / 2][b]; }), QH / 2);
+  }
+  // the extrema over the team: the high words, then the low words of those that have it
+  {
+    const int h1 = __reduce_max_sync(mask, (int)(kmax >> 32)), h0 = __reduce_min_sync(mask, (int)(kmin >> 32));
+    const unsigned l1 = __reduce_max_sync(mask, (int)(kmax >> 32) == h1 ? (unsigned)kmax : 0u);
+    const unsigned l0 = __reduce_min_sync(mask, (int)(kmin >> 32) == h0 ? (unsigned)kmin : ~0u);
+    kmax = (i64)((u64)(unsigned)h1 << 32 | l1);
+    kmin = (i64)((u64)(unsigned)h0 << 32 | l0);
+  }
+  if (r != 0) return;
+  Gi[(size_t)QH * QH * E + e] = GPack(sG, kmin, kmax).word();
+  const double gmin = ldexp((double)kmin, sG), gmax = ldexp((double)kmax, sG);
+  const double amin = 1.0 - gmax, amax = 1.0 - gmin;
+  if (nan || !(amin > 0.0)) {
+    atomicMin(F.err, (1ull << ERR_CLASS_SHIFT) | (unsigned long long)(e + 1));
+    return;
+  }
+  const double th = 0.5 * (amax + amin);
+  const double de = fmax(0.5 * (amax - amin), 1e-15 * th);
+  F.th[e] = th;
+  F.de[e] = de;
+  const int n = cheb_count(F.Lcheb, th, de);
+  F.nst[e] = n;
+  // largest count and the sum of the counts: one atomic each per warp
+  const unsigned am = __activemask();
+  const int nw = __reduce_max_sync(am, n);
+  const unsigned ns = __reduce_add_sync(am, (unsigned)n);
+  if (lane == __ffs(am) - 1) {
+    atomicMax(&F.nmax[S.parity], nw);
+    atomicMax(&F.nmax[2], nw);
+    atomicAdd(F.nsum, (unsigned long long)ns);
+  }
+  if (F.sorted) {
+    // append e to the list of its count, one atomic per group of lanes with the same count
+    const int bin = (n < NBIN ? n : NBIN) - 1;
+    const unsigned same = __match_any_sync(am, bin);
+    const int leader = __ffs(same) - 1;
+    const int rank = __popc(same & ((1u << lane) - 1));
+    int first_slot = 0;
+    if (lane == leader) first_slot = atomicAdd(&F.bin_count[S.parity * NBIN + bin], __popc(same));
+    first_slot = __shfl_sync(same, first_slot, leader);
+    F.bins[(size_t)bin * E + first_slot + rank] = e;
+  }
 }
 
-// Blocks per SM asked of k_stage: at low degrees the registers allow more than two blocks of
-// 128 elements (the shared memory does), and the compiler keeps the kernel within them without
-// spilling; from q_u = 4 on, two
-__host__ __device__ constexpr int stage_m_blocks(int nu) { return nu <= 2 ? 5 : nu == 3 ? 4 : nu == 4 ? 3 : 2; }
+template <int NU, int NV>
+__global__ void __launch_bounds__(128, 4) k_prep(const __grid_constant__ Basis<NU, NV> B,
+                                              const __grid_constant__ Fields F,
+                                              const __grid_constant__ StageIO S, int e0) {
+  // elements from e0 on: a launch may cover a range of the elements (the first range clears the next
+  // stage's counts)
+  prep_body<NU, NV>(B, F, S, e0 + (int)blockIdx.x * prep_tile(NU, blockDim.x), blockIdx.x == 0 && e0 == 0);
+}
+
+// tile = prep_tile(NU, threads) elements per virtual block
+template <int NU, int NV>
+__global__ void __launch_bounds__(128, 4) k_prep_m(const __grid_constant__ Basis<NU, NV> B,
+                                                const __grid_constant__ MultiStage P) {
+  for (int vb = blockIdx.x; vb < P.first[P.n]; vb += gridDim.x) {
+    const int inst = multi_begin(P, vb);
+    const int e0 = (vb - P.first[inst]) * P.tile;
+    prep_body<NU, NV>(B, P.a[inst].F, P.a[inst].S, e0, e0 == 0);
+  }
+}
+
+}  // namespace wedg
+
+#include "wedg_stage_fx.cuh"
+#include "wedg_stage_gen.cuh"
+
+namespace wedg {
+
+// Blocks per SM asked of k_stage: the constant-coefficient kernels four (128 registers), the general ones
+// three (168)
+__host__ __device__ constexpr int stage_m_blocks(int, bool fast) { return fast ? 4 : 3; }
 
 template <int NU, int NV, bool FAST>
-__global__ void __launch_bounds__(stage_threads(NU, NV, FAST), stage_m_blocks(NU))
+__global__ void __launch_bounds__(STAGE_THREADS, stage_m_blocks(NU, FAST))
     k_stage(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ Fields F,
             const __grid_constant__ StageIO S) {
-  constexpr int BT = stage_threads(NU, NV, FAST);
-  stage_body<NU, NV, FAST>(B, F, S, blockIdx.x * BT + (int)threadIdx.x, threadIdx.x);
+  const int e0 = blockIdx.x * stage_tile(NU);
+  if constexpr (FAST) stage_fast_body<NU, NV>(B, F, S, e0);
+  else stage_gen_body<NU, NV>(B, F, S, e0);
 }
 
 
-// tile = stage_threads(NU, NV, FAST) elements per virtual block
+// tile = stage_tile(NU) elements per virtual block
 template <int NU, int NV, bool FAST>
-__global__ void __launch_bounds__(stage_threads(NU, NV, FAST), stage_m_blocks(NU))
+__global__ void __launch_bounds__(STAGE_THREADS, stage_m_blocks(NU, FAST))
     k_stage_m(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ MultiStage P) {
   for (int vb = blockIdx.x; vb < P.first[P.n]; vb += gridDim.x) {
     const int inst = multi_begin(P, vb);
-    stage_body<NU, NV, FAST>(B, P.a[inst].F, P.a[inst].S, (vb - P.first[inst]) * P.tile + (int)threadIdx.x,
-                             threadIdx.x);
+    const int e0 = (vb - P.first[inst]) * P.tile;
+    if constexpr (FAST) stage_fast_body<NU, NV>(B, P.a[inst].F, P.a[inst].S, e0);
+    else stage_gen_body<NU, NV>(B, P.a[inst].F, P.a[inst].S, e0);
   }
 }
 
@@ -1370,6 +916,7 @@ struct ChebTeam {
   static constexpr int NE = NV * NV;
   static constexpr int J = (NE + U - 1) / U;            // modal entries per thread
   static constexpr int SLOT = NE + 2 * U * NV;          // x, then the row sums and differences
+  static constexpr int GSLOT = QH * QH | 1;             // the weights of k_cheb (odd: fewer bank conflicts)
 };
 
 // The shared setup of a team kernel: Ph and PhW in shared memory, the team of this thread, its
@@ -1402,10 +949,11 @@ __device__ __forceinline__ double team_sum(double x, unsigned mask) {
 // acc[j] ± (K x)[k_j] on the thread's entries k_j = u + U j (+ with SIGN = 1, - with -1), for x in
 // the team's shared slot xs (complete, after a __syncwarp). zs, zd hold the units' row results
 // until the next __syncwarp of the caller.
-template <int NU, int NV, int SIGN>
-__device__ __forceinline__ void team_K(const Basis<NU, NV> &B, const Fields &F, size_t Eu, int e, int u,
-                                       unsigned mask, const double *Phs, const double *PhWs, const double *xs,
-                                       double *zs, double *zd, double (&acc)[ChebTeam<NU, NV>::J]) {
+// G(r, s) gives the weight at a point.
+template <int NU, int NV, int SIGN, class GAt>
+__device__ __forceinline__ void team_K(const Basis<NU, NV> &B, const GAt &G, int u, unsigned mask,
+                                       const double *Phs, const double *PhWs, const double *xs, double *zs,
+                                       double *zd, double (&acc)[ChebTeam<NU, NV>::J]) {
   using T = ChebTeam<NU, NV>;
   constexpr int QH = T::QH, U = T::U, NE = T::NE, J = T::J;
   const int r1 = u, r2 = QH - 1 - u;                    // the unit's rows (r1 = r2 for the middle row)
@@ -1413,7 +961,7 @@ __device__ __forceinline__ void team_K(const Basis<NU, NV> &B, const Fields &F, 
     double Y[QH];
     ph_to_points<QH, NV>(B.Ph, Tv, Y);
 #pragma unroll
-    for (int s2 = 0; s2 < QH; ++s2) Y[s2] *= F.G[(r + QH * s2) * Eu + e];
+    for (int s2 = 0; s2 < QH; ++s2) Y[s2] *= G(r, s2);
     ph_from_points<QH, NV>(B.PhW, Y, Z);
   };
   // phase 1: rows r1, r2 of P_h x, at the points, weighted, back to the modes
@@ -1460,10 +1008,13 @@ __device__ __forceinline__ void team_K(const Basis<NU, NV> &B, const Fields &F, 
   constexpr int U = T::U, NE = T::NE, J = T::J;                                                 \
   __shared__ double sh[T::TPB * T::SLOT];                                                       \
   __shared__ double Phs[T::QH * NV], PhWs[T::QH * NV];                                          \
+  __shared__ Fx2 Phf[T::QH * NV], PhWf[T::QH * NV];                                             \
   __shared__ int pref[NBIN];                                                                    \
   for (int i = threadIdx.x; i < T::QH * NV; i += blockDim.x) {                                 \
     Phs[i] = B.Ph[i / NV][i % NV];                                                              \
     PhWs[i] = B.PhW[i / NV][i % NV];                                                            \
+    Phf[i] = Fx2{B.fPh[i / NV][i % NV].h, B.fPh[i / NV][i % NV].l};                             \
+    PhWf[i] = Fx2{B.fPhW[i / NV][i % NV].h, B.fPhW[i / NV][i % NV].l};                          \
   }                                                                                             \
   if (F.sorted && threadIdx.x == 0) {                                                           \
     int acc_ = 0;                                                                               \
@@ -1481,60 +1032,280 @@ __device__ __forceinline__ void team_K(const Basis<NU, NV> &B, const Fields &F, 
   double *xs = sh + tp.slot * T::SLOT, *zs = xs + NE, *zd = zs + U * NV;                        \
   (void)Eu;
 
+// The thread's part of r -= (M/θ) d in fixed point (k_cheb), M = I - P_h^T W G P_h, for d in the team's
+// shared slot xs as d 2^nd (complete, after a __syncwarp) and G in Gs. The levels of the sum
+// factorisation keep the exponents fixed by the operators; 2^kd takes the last one to the integers
+// of d 2^nd. ith: 1/θ as an integer of 2^-56.
+template <int NU, int NV>
+__device__ __forceinline__ void team_M_fx(const Basis<NU, NV> &B, const Fx2 *Gs, int kd, Fx2 ith, int nd, int u,
+                                          unsigned mask, const Fx2 *Phs, const Fx2 *PhWs, const Fx2 *xs, Fx2 *zs,
+                                          Fx2 *zd, i64 (&r)[ChebTeam<NU, NV>::J]) {
+  using T = ChebTeam<NU, NV>;
+  constexpr int QH = T::QH, U = T::U, NE = T::NE, J = T::J;
+  // The levels leave headroom for sums that K does not reach: its rows of the grid stay below
+  // max|G| |d| max_r |Ph[r]| (Euclidean norms) and K d below max|G| |d|. The rows go up by nrow bits, and
+  // the modes by the rest, so that little is lost to the rounding of the levels; T goes up to the top
+  // of its range for the points, by the thread's own nt.
+  const int nrow = B.nrow, zsh = 2 * (61 - B.gPh) + 2 * (61 - B.gPhW) - nrow;
+  {
+    // rows u and QH-1-u (the same one in the middle) of P_h d: even plus and minus odd modes
+    i64 Te[NV], To[NV];
+    {
+      FxC p[NV];
+#pragma unroll
+      for (int a = 0; a < NV; ++a) {
+        const Fx2 q = Phs[u * NV + a];
+        p[a] = FxC{q.h, q.l, q.h << 3};
+      }
+      auto c = [&](int a) -> const FxC & { return p[a]; };
+#pragma unroll
+      for (int b = 0; b < NV; ++b) {
+        auto x = [&](int a) { return xs[a + NV * b]; };
+        Te[b] = fx_dot<0, 2, NV>(x, c);
+        To[b] = fx_dot<1, 2, NV>(x, c);
+      }
+    }
+    int nt = 0;
+#pragma unroll
+    for (int b = 0; b < NV; ++b) nt = max(nt, max(fx_hi(Te[b]), fx_hi(To[b])));
+    nt = max(fx_room(nt) - 1, 0);
+#pragma unroll
+    for (int b = 0; b < NV; ++b) {
+      Te[b] <<= nt;
+      To[b] <<= nt;
+    }
+    const i64 half = nt > nrow ? (i64)1 << (nt - nrow - 1) : 0;
+#pragma unroll 1
+    for (int t = 0; t < 2; ++t) {
+      // row r of the grid: the points, weighted, back to the modes
+      const int r = t == 0 ? u : QH - 1 - u;
+      const i64 sg = -t;
+      if (t == 1 && r == u) break;        // the middle row: zd is not read (PhW vanishes for odd modes)
+      Fx2 Tv[NV];
+#pragma unroll
+      for (int b = 0; b < NV; ++b) Tv[b] = fx_split(Te[b] + ((To[b] ^ sg) - sg));
+      auto tv = [&](int b) { return Tv[b]; };
+      Fx2 ys[QH / 2 + 1], yd[QH / 2 + 1];
+      auto weigh = [&](i64 y0, int s2) {
+        const Fx2 y = fx_split(y0), g = Gs[r + QH * s2];
+        const i64 m = fx_mad(y.h, g.l, fx_mad(y.l, g.h, 1 << 28));
+        return (fx_mad(y.h, g.h, 0) << 3) + (m >> 29);
+      };
+#pragma unroll
+      for (int s2 = 0; s2 < QH / 2; ++s2) {
+        auto c = [&](int b) -> const FxC & { return B.fPh[s2][b]; };
+        const i64 e0 = fx_dot<0, 2, NV>(tv, c), o0 = fx_dot<1, 2, NV>(tv, c);
+        const i64 p = weigh(e0 + o0, s2), m = weigh(e0 - o0, QH - 1 - s2);
+        ys[s2] = fx_split(p + m);
+        yd[s2] = fx_split(p - m);
+      }
+      if constexpr ((QH & 1) != 0)
+        ys[QH / 2] = fx_split(
+            weigh(fx_dot<0, 2, NV>(tv, [&](int b) -> const FxC & { return B.fPh[QH / 2][b]; }), QH / 2));
+#pragma unroll
+      for (int b = 0; b < NV; ++b) {
+        auto c = [&](int s2) -> const FxC & { return B.fPhW[s2][b]; };
+        i64 z;
+        if (b & 1) z = fx_dot<0, 1, QH / 2>([&](int s2) { return yd[s2]; }, c);
+        else z = fx_dot<0, 1, (QH + 1) / 2>([&](int s2) { return ys[s2]; }, c);
+        // the sum and the difference of the two rows' results; the first row's waits in the slots
+        z = nt > nrow ? (z + half) >> (nt - nrow) : z << (nrow - nt);
+        const i64 z0 = t == 0 ? 0 : fx_join(zs[u * NV + b]);
+        zs[u * NV + b] = fx_split(z0 + z);
+        zd[u * NV + b] = fx_split(t == 0 ? z : z0 - z);
+      }
+    }
+  }
+  __syncwarp(mask);
+  const int up = max(kd - nd, 0), down = min(max(nd - kd, 0), 62);
+  const i64 half = down ? (i64)1 << (down - 1) : 0;
+#pragma unroll
+  for (int j = 0; j < J; ++j) {
+    const int k = u + U * j;
+    if (k < NE) {
+      const int a = k % NV, b = k / NV;
+      const Fx2 *z = ((a & 1) ? zd : zs) + b;
+      // (with the products of the low halves: the result goes up by zsh)
+      i64 m = 0, h = 0, l = 0;
+#pragma unroll
+      for (int v = 0; v < U; ++v) {
+        const Fx2 p = PhWs[v * NV + a], y = z[v * NV];
+        l += fx_mad(y.l, p.l, 0) >> 32;
+        m = fx_mad(y.h, p.l, m);
+        m = fx_mad(y.l, p.h, m);
+        h = fx_mad(y.h, p.h, h);
+      }
+      m += l;
+      const i64 Kd = ((((h << zsh) + (m >> (32 - zsh))) << up) + half) >> down;
+      const Fx2 t = fx_split((fx_join(xs[k]) >> nd) - Kd);
+      m = fx_mad(t.h, ith.l, fx_mad(t.l, ith.h, (fx_mad(t.l, ith.l, 0) >> 32) + (1 << 23)));
+      r[j] -= (fx_mad(t.h, ith.h, 0) << 8) + (m >> 24);
+    }
+  }
+}
+
 // k_cheb: the Chebyshev mass solve (Saad Alg. 12.1, src/rhs.jl:920-939). Elements are visited in
 // decreasing order of their step counts (k_prep lists them by count), so the longest solves start
 // first. The team keeps the residual r, the iterate X and the direction d of its entries in
 // registers and d in its shared slot.
+//
+// The iteration runs in fixed point on the system scaled by the middle θ of the spectral interval,
+// (M/θ) X' = R with X' = θX, whose spectrum is 1 ± ε, ε = δ/θ: the integers of r, X' and d keep the
+// exponent of R through all steps (the solution grows by at most 1/(1 - ε), for which R gets
+// headroom), and d goes into the products with M as d 2^nd, at the top of its range. Elements with
+// ε > 31/32, θ < 1/8 or max|G| > 7 and right-hand sides that are not finite take it in FP64.
 template <int NU, int NV>
 __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &F, const StageIO &S, int g0) {
   WEDG_TEAM_SETUP(g0);
+  constexpr int QH = T::QH;
   const int e = mass_element(F, S, g, pref);
   const double th = F.th[e], de = F.de[e];
   const double s1 = th / de;
   const int n = F.cheb_common ? F.nmax[S.parity] : F.nst[e];
   const double ith = 1.0 / th;
-  double rr[J], xx[J], dd[J];
+  const i64 *G = reinterpret_cast<const i64 *>(F.G) + e;
+  const GPack gp(G[(size_t)QH * QH * Eu]);
+  double R[J];
+  int hr = 0;
 #pragma unroll
   for (int j = 0; j < J; ++j) {
     const int k = u + U * j;
-    rr[j] = xx[j] = dd[j] = 0.0;
-    if (k < NE) {
-      const double x = F.mrhs[k * Eu + e];
-      rr[j] = x;
-      dd[j] = x * ith;
-      xs[k] = dd[j];
-    }
+    R[j] = k < NE ? F.mrhs[k * Eu + e] : 0.0;
+    hr = max(hr, fx_abs_hi(R[j]));
   }
-  __syncwarp(tmask);
-  double rho = 1.0 / s1;
-#pragma unroll 1
-  for (int step = 1; step <= n; ++step) {
+  hr = __reduce_max_sync(tmask, hr);
+  bool fin = true;
+  __shared__ i64 Xsh[T::TPB * NE];
+  // max|G| from the ends of the interval
+  const double gmax = fmax(fabs(1.0 - (th + de)), fabs(1.0 - (th - de)));
+  if (fx_finite(hr) && s1 >= 32.0 / 31.0 && th >= 0.125 && gmax <= 7.0) {
+    // R with headroom: the entries of X' and d stay below |R|max + 2 ε/(1 - ε) |R| and those of M d below
+    // that with |R| (1 + max|G|) (the Euclidean norm, from the entries' high words in FP32, with a
+    // little to spare)
+    float r2 = 0.0f;
 #pragma unroll
     for (int j = 0; j < J; ++j) {
-      xx[j] += dd[j];
-      rr[j] -= dd[j];
+      const int x = fx_abs_hi(R[j]) - (hr & 0x7ff00000) + (127 << 20);   // |R| over the largest's power of two
+      const float f = x > 0 ? __int_as_float(x << 3) : 0.0f;
+      r2 = fmaf(f, f, r2);
     }
-    if (step == n) break;
-    team_K<NU, NV, 1>(B, F, Eu, e, u, tmask, Phs, PhWs, xs, zs, zd, rr);   // r += K d
-    const double rhon = 1.0 / (2.0 * s1 - rho);
-    const double c1 = rhon * rho, c2 = 2.0 * rhon / de;
+    r2 = (float)__reduce_add_sync(tmask, (unsigned)(r2 * 1024.0f) + 1) * (1.0f / 1024.0f);
+    const float eps = (float)(de / th);
+    const float grow = 1.0f + 0.51f * (1.0f + (float)gmax) * fmaxf(1.0f, 2.0f * eps / (1.0f - eps)) * sqrtf(r2);
+    const int hb = (__float_as_int(grow) >> 23) - 126;
+    const int er = fx_exp(hr) + hb;
+    Fx2 *xf = reinterpret_cast<Fx2 *>(xs);
+    // r in registers, X' and d (as d 2^nd, what K takes) in shared memory
+    i64 *X = Xsh + tp.slot * NE;
+    i64 rr[J];
 #pragma unroll
     for (int j = 0; j < J; ++j) {
       const int k = u + U * j;
+      rr[j] = fx_from(R[j], er);
       if (k < NE) {
-        dd[j] = fma(c1, dd[j], c2 * rr[j]);
-        xs[k] = dd[j];
+        X[k] = 0;
+        xf[k] = fx_split(rr[j] << hb);
       }
     }
-    rho = rhon;
     __syncwarp(tmask);
-  }
-
-  bool fin = true;
+    int nd = hb;                                   // d 2^nd, just below 2^61, is what K takes
+    // the unit's rows of G 2^ng, just below 2^60
+    __shared__ Fx2 Gsh[T::TPB * T::GSLOT];
+    Fx2 *Gs = Gsh + tp.slot * T::GSLOT;
+    if (n > 1)
+#pragma unroll 1
+      for (int t = 0; t < 2; ++t) {
+        const int r = t == 0 ? u : QH - 1 - u;
 #pragma unroll
-  for (int j = 0; j < J; ++j) {
-    const int k = u + U * j;
-    if (k < NE) store_v(S, e + Eu * k, xx[j], fin);
+        for (int s2 = 0; s2 < QH; ++s2) Gs[r + QH * s2] = fx_split(G[(r + QH * s2) * Eu] << gp.ng);
+      }
+    const int kd = max(gp.sG - gp.ng + 64, -62);   // (team_M_fx's zsh takes the levels' exponents up to this one)
+    const Fx2 ithf = fx_split(fx_scalar(ith, FX_BIAS - 56));
+    double rho = 1.0 / s1;
+#pragma unroll 1
+    for (int step = 1; step <= n; ++step) {
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const int k = u + U * j;
+        if (k < NE) {
+          X[k] += fx_join(xf[k]) >> nd;
+        }
+      }
+      if (step == n) break;
+      team_M_fx<NU, NV>(B, Gs, kd, ithf, nd, u, tmask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs),
+                        reinterpret_cast<Fx2 *>(zd), rr);
+      // d = c1 d + c2 r, c1 = ρ' ρ < 1 and c2 = 2 ρ' θ/δ ≤ 2 as integers of 2^-59
+      const double rhon = 1.0 / (2.0 * s1 - rho);
+      const Fx2 c1 = fx_split(fx_from(rhon * rho, 1024)), c2 = fx_split(fx_from(2.0 * rhon * s1, 1024));
+      rho = rhon;
+      int hd = 0;
+      i64 dd[J];
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const int k = u + U * j;
+        const Fx2 d = fx_split(k < NE ? fx_join(xf[k]) >> nd : 0), r = fx_split(rr[j]);
+        const i64 m = fx_mad(d.h, c1.l, fx_mad(d.l, c1.h, fx_mad(r.h, c2.l, fx_mad(r.l, c2.h, 1 << 26))));
+        dd[j] = (fx_mad(d.h, c1.h, fx_mad(r.h, c2.h, 0)) << 5) + (m >> 27);
+        hd = max(hd, fx_hi(dd[j]));
+      }
+      nd = fx_room(__reduce_max_sync(tmask, hd));
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const int k = u + U * j;
+        if (k < NE) xf[k] = fx_split(dd[j] << nd);
+      }
+      __syncwarp(tmask);
+    }
+    const double sc = fx_pow2(er - FX_BIAS) * ith;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const int k = u + U * j;
+      if (k < NE) store_v(S, e + Eu * k, __dmul_rn((double)X[k], sc), fin);
+    }
+  } else {
+    const double gs = ldexp(1.0, gp.sG);
+    auto Gd = [&](int r, int s2) { return (double)G[(r + QH * s2) * Eu] * gs; };
+    double *X = reinterpret_cast<double *>(Xsh) + tp.slot * NE;
+    double rr[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const int k = u + U * j;
+      rr[j] = R[j];
+      if (k < NE) {
+        X[k] = 0.0;
+        xs[k] = R[j] * ith;
+      }
+    }
+    __syncwarp(tmask);
+    double rho = 1.0 / s1;
+#pragma unroll 1
+    for (int step = 1; step <= n; ++step) {
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const int k = u + U * j;
+        if (k < NE) {
+          const double d = xs[k];
+          X[k] += d;
+          rr[j] -= d;
+        }
+      }
+      if (step == n) break;
+      team_K<NU, NV, 1>(B, Gd, u, tmask, Phs, PhWs, xs, zs, zd, rr);   // r += K d
+      const double rhon = 1.0 / (2.0 * s1 - rho);
+      const double c1 = rhon * rho, c2 = 2.0 * rhon / de;
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const int k = u + U * j;
+        if (k < NE) xs[k] = fma(c1, xs[k], c2 * rr[j]);
+      }
+      rho = rhon;
+      __syncwarp(tmask);
+    }
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const int k = u + U * j;
+      if (k < NE) store_v(S, e + Eu * k, X[k], fin);
+    }
   }
   if (S.mode == OUT_RK4_LAST && !fin) atomicOr(F.nonfinite, 1u);
 }
@@ -1566,6 +1337,7 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
     gput(Tp, r1);
     if (r2 != r1) gput(Tm, r2);
   }
+  auto G = [&](int r, int s2) { return F.G[(r + QH * s2) * Eu + e]; };
   double X[J], r[J], p[J], Ap[J];
   double r0 = 0;
 #pragma unroll
@@ -1581,7 +1353,7 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
   }
   r0 = sqrt(team_sum<U>(r0, tmask));
   __syncwarp(tmask);
-  team_K<NU, NV, 1>(B, F, Eu, e, u, tmask, Phs, PhWs, xs, zs, zd, r);    // r = R - M X = K R for X = R
+  team_K<NU, NV, 1>(B, G, u, tmask, Phs, PhWs, xs, zs, zd, r);    // r = R - M X = K R for X = R
   double rr = 0;
 #pragma unroll
   for (int j = 0; j < J; ++j) {
@@ -1603,7 +1375,7 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
     __syncwarp(tmask);
 #pragma unroll
     for (int j = 0; j < J; ++j) Ap[j] = p[j];
-    team_K<NU, NV, -1>(B, F, Eu, e, u, tmask, Phs, PhWs, xs, zs, zd, Ap);  // A p = p - K p
+    team_K<NU, NV, -1>(B, G, u, tmask, Phs, PhWs, xs, zs, zd, Ap);  // A p = p - K p
     double pAp = 0;
 #pragma unroll
     for (int j = 0; j < J; ++j) pAp = fma(p[j], Ap[j], pAp);
@@ -1647,14 +1419,14 @@ __device__ __forceinline__ int team_tile() {
 }
 
 template <int NU, int NV>
-__global__ void __launch_bounds__(CHEB_THREADS, 3)
+__global__ void __launch_bounds__(CHEB_THREADS, 4)
     k_cheb(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ Fields F,
            const __grid_constant__ StageIO S) {
   cheb_body<NU, NV>(B, F, S, blockIdx.x * team_tile<NU, NV>());
 }
 
 template <int NU, int NV>
-__global__ void __launch_bounds__(CHEB_THREADS, 3)
+__global__ void __launch_bounds__(CHEB_THREADS, 4)
     k_cg(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ Fields F,
          const __grid_constant__ StageIO S) {
   cg_body<NU, NV>(B, F, S, blockIdx.x * team_tile<NU, NV>());
@@ -1662,7 +1434,7 @@ __global__ void __launch_bounds__(CHEB_THREADS, 3)
 
 // tile = team_tile elements per virtual block; CG selects k_cg's body
 template <int NU, int NV, bool CG>
-__global__ void __launch_bounds__(CHEB_THREADS, 3)
+__global__ void __launch_bounds__(CHEB_THREADS, CG ? 3 : 4)
     k_mass_m(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ MultiStage P) {
   for (int vb = blockIdx.x; vb < P.first[P.n]; vb += gridDim.x) {
     const int inst = multi_begin(P, vb);

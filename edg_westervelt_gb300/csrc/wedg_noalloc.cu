@@ -129,7 +129,8 @@ extern "C" int wedg_rhs_noalloc(const wedg_config *cfg, const wedg_pre *pre, con
     return fail(msg, msg_len, WEDG_ERR_ARGUMENT, "Ainv_u is needed: the coefficients are not constant per element");
   const Launchers Lch = get_launchers(nu, nv, fast);
   if (!Lch.prep) return fail(msg, msg_len, WEDG_ERR_ARGUMENT, "unsupported degrees");
-  alignas(16) char basis[8192];
+  alignas(16) char basis[16384];
+  static_assert(sizeof(Basis<MAXN, MAXN>) <= sizeof basis, "the 1D operators exceed their buffer");
   if (Lch.basis_size > sizeof basis) return fail(msg, msg_len, WEDG_ERR_ARGUMENT, "unsupported degrees");
   Lch.pack(bh, basis);
 
@@ -150,7 +151,7 @@ extern "C" int wedg_rhs_noalloc(const wedg_config *cfg, const wedg_pre *pre, con
   const size_t o_pid = cfg->mms_on ? take(np) : 0;
   const size_t o_pic = cfg->src_on ? 0 : take(np), o_src = cfg->src_on ? take(np) : 0;
   const size_t o_beta = take((size_t)qh * qh * E);
-  const size_t o_tr = take((size_t)12 * nq * E), o_G = take((size_t)qh * qh * E);
+  const size_t o_tr = take((size_t)12 * nq * E), o_bs = take((size_t)4 * N * (2 * nv + nq));
   const size_t o_th = take(E), o_de = take(E), o_nst = take(E);
   const size_t o_mrhs = take((size_t)nv * nv * E);
   const size_t o_bins = take(((size_t)NBIN * E + 1) / 2), o_bcnt = take(NBIN);   // ints, two per double
@@ -158,7 +159,9 @@ extern "C" int wedg_rhs_noalloc(const wedg_config *cfg, const wedg_pre *pre, con
   raw_max = raw_max > (size_t)qh * qh * E ? raw_max : (size_t)qh * qh * E;
   raw_max = raw_max > nh ? raw_max : nh;
   raw_max = raw_max > np ? raw_max : np;
-  const size_t o_raw = take(raw_max);
+  // the raw copies of pre come before G is written: one place for both
+  const size_t g_size = ((size_t)qh * qh + 2) * E;
+  const size_t o_raw = take(raw_max > g_size ? raw_max : g_size), o_G = o_raw;
   if (off > NOALLOC_DOUBLES) {
     if (msg && msg_len)
       snprintf(msg, msg_len,
@@ -240,6 +243,7 @@ extern "C" int wedg_rhs_noalloc(const wedg_config *cfg, const wedg_pre *pre, con
   F.beta2 = base + o_beta;
   F.tr = base + o_tr;
   F.G = base + o_G;
+  F.bslots = base + o_bs;
   F.th = base + o_th;
   F.de = base + o_de;
   F.nst = reinterpret_cast<int *>(base + o_nst);
@@ -298,11 +302,12 @@ extern "C" int wedg_rhs_noalloc(const wedg_config *cfg, const wedg_pre *pre, con
     if (msg && msg_len) snprintf(msg, msg_len, "CUDA error: %s", cudaGetErrorString(ce));
     return WEDG_ERR_CUDA;
   }
-  const int tp = 128, ts = stage_threads(nu, nv, fast);
+  const int tp = 128, ep = prep_tile(nu, tp), ts = STAGE_THREADS, tile = stage_tile(nu);
   unsigned long long err = 0;
   unsigned int cgf = 0;
-  if ((ce = Lch.prep(basis, F, S, (iE + tp - 1) / tp, tp, st, 0)) != cudaSuccess ||
-      (ce = Lch.stage(basis, F, S, (iE + ts - 1) / ts, ts, st)) != cudaSuccess ||
+  if ((ce = Lch.prep(basis, F, S, (iE + ep - 1) / ep, tp, st, 0)) != cudaSuccess ||
+      (ce = Lch.bnd(basis, F, S, 1, BND_THREADS, st)) != cudaSuccess ||
+      (ce = Lch.stage(basis, F, S, (iE + tile - 1) / tile, ts, st)) != cudaSuccess ||
       (ce = Lch.mass(basis, F, S, 1, CHEB_THREADS, st)) != cudaSuccess ||
       (ce = cudaGetLastError()) != cudaSuccess ||
       (ce = cudaMemcpyAsync(&err, F.err, sizeof err, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||

@@ -675,17 +675,16 @@ int argument_error(wedg_ws *ws, const std::string &msg) {
 
 // ---- multi-instance launches of one kernel over many instances' arguments, in chunks of the
 //      launch's capacity (wedg_kernels.cuh): k_prep (tile = prep_tile), k_bnd (tile = bnd_tile of the
-//      4N sides), k_stage (tile = stage_tile), the mass solve (tile = teams of `threads`). grid_of
+//      4N sides), k_stage (tile = stage_tile), the mass solve (tile = mass_tile). grid_of
 //      maps the virtual blocks of a chunk to its physical grid (persistent launches).
 enum { MK_PREP = 0, MK_BND = 1, MK_STAGE = 2, MK_MASS = 3 };
 template <class GridOf>
 cudaError_t multi_stage_launch(const Launchers &L, const void *basis, int nu, int nv, bool fast, int kind,
                                const std::vector<StageArgs> &args, int threads, cudaStream_t st, GridOf grid_of) {
-  const int TPW = 32 / (qhigh(nu, nv) / 2 + (qhigh(nu, nv) & 1));
   const int tile = kind == MK_PREP    ? prep_tile(nu, threads)
                    : kind == MK_BND   ? bnd_tile(nu)
                    : kind == MK_STAGE ? stage_tile(nu)
-                                      : (threads / 32) * TPW;
+                                      : mass_tile(nu, nv, !args.empty() && args[0].F.cg, threads);
   const int n = (int)args.size();
   for (int c0 = 0; c0 < n; c0 += MultiStage::cap) {
     const int m = std::min(n - c0, MultiStage::cap);

@@ -811,7 +811,7 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
 }
 
 template <int NU, int NV>
-__global__ void __launch_bounds__(128, 4) k_prep(const __grid_constant__ Basis<NU, NV> B,
+__global__ void __launch_bounds__(128, 8) k_prep(const __grid_constant__ Basis<NU, NV> B,
                                               const __grid_constant__ Fields F,
                                               const __grid_constant__ StageIO S, int e0) {
   // elements from e0 on: a launch may cover a range of the elements (the first range clears the next
@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(128, 4) k_prep(const __grid_constant__ Basis<N
 
 // tile = prep_tile(NU, threads) elements per virtual block
 template <int NU, int NV>
-__global__ void __launch_bounds__(128, 4) k_prep_m(const __grid_constant__ Basis<NU, NV> B,
+__global__ void __launch_bounds__(128, 8) k_prep_m(const __grid_constant__ Basis<NU, NV> B,
                                                 const __grid_constant__ MultiStage P) {
   for (int vb = blockIdx.x; vb < P.first[P.n]; vb += gridDim.x) {
     const int inst = multi_begin(P, vb);
@@ -837,9 +837,9 @@ __global__ void __launch_bounds__(128, 4) k_prep_m(const __grid_constant__ Basis
 
 namespace wedg {
 
-// Blocks per SM asked of k_stage: the constant-coefficient kernels four (128 registers), the general ones
+// Blocks per SM asked of k_stage: the constant-coefficient kernels six (80 registers), the general ones
 // three (168)
-__host__ __device__ constexpr int stage_m_blocks(int, bool fast) { return fast ? 4 : 3; }
+__host__ __device__ constexpr int stage_m_blocks(int, bool fast) { return fast ? 6 : 3; }
 
 template <int NU, int NV, bool FAST>
 __global__ void __launch_bounds__(STAGE_THREADS, stage_m_blocks(NU, FAST))
@@ -916,7 +916,6 @@ struct ChebTeam {
   static constexpr int NE = NV * NV;
   static constexpr int J = (NE + U - 1) / U;            // modal entries per thread
   static constexpr int SLOT = NE + 2 * U * NV;          // x, then the row sums and differences
-  static constexpr int GSLOT = QH * QH | 1;             // the weights of k_cheb (odd: fewer bank conflicts)
 };
 
 // The shared setup of a team kernel: Ph and PhW in shared memory, the team of this thread, its
@@ -1008,13 +1007,10 @@ __device__ __forceinline__ void team_K(const Basis<NU, NV> &B, const GAt &G, int
   constexpr int U = T::U, NE = T::NE, J = T::J;                                                 \
   __shared__ double sh[T::TPB * T::SLOT];                                                       \
   __shared__ double Phs[T::QH * NV], PhWs[T::QH * NV];                                          \
-  __shared__ Fx2 Phf[T::QH * NV], PhWf[T::QH * NV];                                             \
   __shared__ int pref[NBIN];                                                                    \
   for (int i = threadIdx.x; i < T::QH * NV; i += blockDim.x) {                                 \
     Phs[i] = B.Ph[i / NV][i % NV];                                                              \
     PhWs[i] = B.PhW[i / NV][i % NV];                                                            \
-    Phf[i] = Fx2{B.fPh[i / NV][i % NV].h, B.fPh[i / NV][i % NV].l};                             \
-    PhWf[i] = Fx2{B.fPhW[i / NV][i % NV].h, B.fPhW[i / NV][i % NV].l};                          \
   }                                                                                             \
   if (F.sorted && threadIdx.x == 0) {                                                           \
     int acc_ = 0;                                                                               \
@@ -1032,103 +1028,132 @@ __device__ __forceinline__ void team_K(const Basis<NU, NV> &B, const GAt &G, int
   double *xs = sh + tp.slot * T::SLOT, *zs = xs + NE, *zd = zs + U * NV;                        \
   (void)Eu;
 
-// The thread's part of r -= (M/θ) d in fixed point (k_cheb), M = I - P_h^T W G P_h, for d in the team's
-// shared slot xs as d 2^nd (complete, after a __syncwarp) and G in Gs. The levels of the sum
-// factorisation keep the exponents fixed by the operators; 2^kd takes the last one to the integers
-// of d 2^nd. ith: 1/θ as an integer of 2^-56.
+// k_cheb: the Chebyshev mass solve (Saad Alg. 12.1, src/rhs.jl:920-939), a team of QH threads per
+// element: thread u takes row u of the point grid and J of the modal entries. Elements are visited in
+// decreasing order of their step counts (k_prep lists them by count), so the longest solves start
+// first.
+//
+// The iteration runs in fixed point on the system scaled by the middle θ of the spectral interval,
+// (M/θ) X' = R with X' = θX, whose spectrum is 1 ± ε, ε = δ/θ: the integers of r, X' and d keep the
+// exponent of R through all steps (the solution grows by at most 1/(1 - ε), for which R gets
+// headroom), and d goes into the products with M as d 2^nd, at the top of its range. Elements with
+// ε > 31/32, θ < 1/8 or max|G| > 7 and right-hand sides that are not finite take it in FP64.
+//
+// What bounds it: one product with M costs about 1 300 multiply-adds an element at q = 6, three integer
+// ones each (4 cycles a warp), and 18 shared-memory words a thread; a thread per row keeps 24 warps an SM
+// where a thread per pair of rows (half the exchanges, 16 warps) left the pipes waiting.
+template <int NU, int NV>
+struct MassTeam {
+  static constexpr int QH = qhigh(NU, NV);
+  static constexpr int HP = (QH + 1) / 2;               // row pairs (and the middle row)
+  static constexpr int TPW = 32 / QH;                   // teams per warp
+  static constexpr int TPB = TPW * (CHEB_THREADS / 32); // elements per block
+  static constexpr int NE = NV * NV;
+  static constexpr int J = (NE + QH - 1) / QH;          // modal entries per thread
+  static constexpr int ZR = 2 * HP * NV;                // the sums and differences of row pairs
+  static constexpr int SLOT = (2 * NE + ZR + QH * QH) | 1;   // d, X', the rows, G; odd: bank conflicts
+};
+__host__ __device__ constexpr int mass_tile(int nu, int nv, bool cg, int threads) {
+  const int qh = qhigh(nu, nv);
+  return (threads / 32) * (32 / (cg ? (qh + 1) / 2 : qh));
+}
+
+// The thread's part of r -= (M/θ) d, M = I - P_h^T W G P_h, for d in xs as d 2^nd (complete, after a
+// __syncwarp) and G in Gs. The levels of the sum factorisation keep the exponents fixed by the
+// operators; 2^kd takes the last one to the integers of d 2^nd. ith: 1/θ as an integer of 2^-56.
 template <int NU, int NV>
 __device__ __forceinline__ void team_M_fx(const Basis<NU, NV> &B, const Fx2 *Gs, int kd, Fx2 ith, int nd, int u,
-                                          unsigned mask, const Fx2 *Phs, const Fx2 *PhWs, const Fx2 *xs, Fx2 *zs,
-                                          Fx2 *zd, i64 (&r)[ChebTeam<NU, NV>::J]) {
-  using T = ChebTeam<NU, NV>;
-  constexpr int QH = T::QH, U = T::U, NE = T::NE, J = T::J;
+                                          int lane0, unsigned mask, const Fx2 *Phs, const Fx2 *PhWs, const Fx2 *xs,
+                                          Fx2 *zs, i64 (&r)[MassTeam<NU, NV>::J]) {
+  using T = MassTeam<NU, NV>;
+  constexpr int QH = T::QH, HP = T::HP, NE = T::NE, J = T::J, NP = (NV + 1) / 2;
   // The levels leave headroom for sums that K does not reach: its rows of the grid stay below
   // max|G| |d| max_r |Ph[r]| (Euclidean norms) and K d below max|G| |d|. The rows go up by nrow bits, and
   // the modes by the rest, so that little is lost to the rounding of the levels; T goes up to the top
   // of its range for the points, by the thread's own nt.
   const int nrow = B.nrow, zsh = 2 * (61 - B.gPh) + 2 * (61 - B.gPhW) - nrow;
+  const bool high = u >= HP;                             // the mirror of a lower row
+  const int low = high ? QH - 1 - u : u, mate = lane0 + (QH - 1 - u);
+  // row u of P_h d: the thread of the lower row sums the even modes, its mirror the odd ones
+  i64 Tv[NV];
   {
-    // rows u and QH-1-u (the same one in the middle) of P_h d: even plus and minus odd modes
-    i64 Te[NV], To[NV];
-    {
-      FxC p[NV];
+    Fx2 p[NP];
+    const int o = high ? 1 : 0;
 #pragma unroll
-      for (int a = 0; a < NV; ++a) {
-        const Fx2 q = Phs[u * NV + a];
-        p[a] = FxC{q.h, q.l, q.h << 3};
-      }
-      auto c = [&](int a) -> const FxC & { return p[a]; };
-#pragma unroll
-      for (int b = 0; b < NV; ++b) {
-        auto x = [&](int a) { return xs[a + NV * b]; };
-        Te[b] = fx_dot<0, 2, NV>(x, c);
-        To[b] = fx_dot<1, 2, NV>(x, c);
-      }
-    }
-    int nt = 0;
-#pragma unroll
-    for (int b = 0; b < NV; ++b) nt = max(nt, max(fx_hi(Te[b]), fx_hi(To[b])));
-    nt = max(fx_room(nt) - 1, 0);
+    for (int i = 0; i < NP; ++i) p[i] = 2 * i + o < NV ? Phs[low * NV + 2 * i + o] : Fx2{0, 0};
 #pragma unroll
     for (int b = 0; b < NV; ++b) {
-      Te[b] <<= nt;
-      To[b] <<= nt;
-    }
-    const i64 half = nt > nrow ? (i64)1 << (nt - nrow - 1) : 0;
-#pragma unroll 1
-    for (int t = 0; t < 2; ++t) {
-      // row r of the grid: the points, weighted, back to the modes
-      const int r = t == 0 ? u : QH - 1 - u;
-      const i64 sg = -t;
-      if (t == 1 && r == u) break;        // the middle row: zd is not read (PhW vanishes for odd modes)
-      Fx2 Tv[NV];
+      i64 m = 1 << 28, h = 0;
 #pragma unroll
-      for (int b = 0; b < NV; ++b) Tv[b] = fx_split(Te[b] + ((To[b] ^ sg) - sg));
-      auto tv = [&](int b) { return Tv[b]; };
-      Fx2 ys[QH / 2 + 1], yd[QH / 2 + 1];
-      auto weigh = [&](i64 y0, int s2) {
-        const Fx2 y = fx_split(y0), g = Gs[r + QH * s2];
-        const i64 m = fx_mad(y.h, g.l, fx_mad(y.l, g.h, 1 << 28));
-        return (fx_mad(y.h, g.h, 0) << 3) + (m >> 29);
-      };
-#pragma unroll
-      for (int s2 = 0; s2 < QH / 2; ++s2) {
-        auto c = [&](int b) -> const FxC & { return B.fPh[s2][b]; };
-        const i64 e0 = fx_dot<0, 2, NV>(tv, c), o0 = fx_dot<1, 2, NV>(tv, c);
-        const i64 p = weigh(e0 + o0, s2), m = weigh(e0 - o0, QH - 1 - s2);
-        ys[s2] = fx_split(p + m);
-        yd[s2] = fx_split(p - m);
+      for (int i = 0; i < NP; ++i) {
+        const Fx2 x = xs[(2 * i + o < NV ? 2 * i + o : 0) + NV * b];
+        m = fx_mad(x.h, p[i].l, fx_mad(x.l, p[i].h, m));
+        h = fx_mad(x.h, p[i].h, h);
       }
-      if constexpr ((QH & 1) != 0)
-        ys[QH / 2] = fx_split(
-            weigh(fx_dot<0, 2, NV>(tv, [&](int b) -> const FxC & { return B.fPh[QH / 2][b]; }), QH / 2));
-#pragma unroll
-      for (int b = 0; b < NV; ++b) {
-        auto c = [&](int s2) -> const FxC & { return B.fPhW[s2][b]; };
-        i64 z;
-        if (b & 1) z = fx_dot<0, 1, QH / 2>([&](int s2) { return yd[s2]; }, c);
-        else z = fx_dot<0, 1, (QH + 1) / 2>([&](int s2) { return ys[s2]; }, c);
-        // the sum and the difference of the two rows' results; the first row's waits in the slots
-        z = nt > nrow ? (z + half) >> (nt - nrow) : z << (nrow - nt);
-        const i64 z0 = t == 0 ? 0 : fx_join(zs[u * NV + b]);
-        zs[u * NV + b] = fx_split(z0 + z);
-        zd[u * NV + b] = fx_split(t == 0 ? z : z0 - z);
-      }
+      const i64 t = (h << 3) + (m >> 29), q = __shfl_sync(mask, t, mate);
+      Tv[b] = 2 * u + 1 == QH ? t : high ? q - t : t + q;   // (the odd modes vanish in the middle row)
     }
+  }
+  int nt = 0;
+#pragma unroll
+  for (int b = 0; b < NV; ++b) nt = max(nt, fx_hi(Tv[b]));
+  nt = fx_room(nt);
+  // the points of the row, weighted, and back to the modes
+  i64 Z[NV];
+  {
+    Fx2 t[NV];
+#pragma unroll
+    for (int b = 0; b < NV; ++b) t[b] = fx_split(Tv[b] << nt);
+    auto tv = [&](int b) { return t[b]; };
+    Fx2 ys[QH / 2 + 1], yd[QH / 2 + 1];
+    auto weigh = [&](i64 y0, int s2) {
+      const Fx2 y = fx_split(y0), g = Gs[u + QH * s2];
+      const i64 m = fx_mad(y.h, g.l, fx_mad(y.l, g.h, 1 << 28));
+      return (fx_mad(y.h, g.h, 0) << 3) + (m >> 29);
+    };
+#pragma unroll
+    for (int s2 = 0; s2 < QH / 2; ++s2) {
+      auto c = [&](int b) -> const FxC & { return B.fPh[s2][b]; };
+      const i64 e0 = fx_dot<0, 2, NV>(tv, c), o0 = fx_dot<1, 2, NV>(tv, c);
+      const i64 p = weigh(e0 + o0, s2), m = weigh(e0 - o0, QH - 1 - s2);
+      ys[s2] = fx_split(p + m);
+      yd[s2] = fx_split(p - m);
+    }
+    if constexpr ((QH & 1) != 0)
+      ys[QH / 2] = fx_split(
+          weigh(fx_dot<0, 2, NV>(tv, [&](int b) -> const FxC & { return B.fPh[QH / 2][b]; }), QH / 2));
+    const int dn = nt - nrow;
+#pragma unroll
+    for (int b = 0; b < NV; ++b) {
+      auto c = [&](int s2) -> const FxC & { return B.fPhW[s2][b]; };
+      i64 z;
+      if (b & 1) z = fx_dot<0, 1, QH / 2>([&](int s2) { return yd[s2]; }, c);
+      else z = fx_dot<0, 1, (QH + 1) / 2>([&](int s2) { return ys[s2]; }, c);
+      Z[b] = dn > 0 ? (z + ((i64)1 << (dn - 1))) >> dn : z << -dn;
+    }
+  }
+  // the sums (lower row's thread) and differences (its mirror) of the row pairs, [row NV + b] each; the
+  // middle row is its own sum, and its difference is not read for anything (P_h's odd modes vanish there)
+#pragma unroll
+  for (int b = 0; b < NV; ++b) {
+    const i64 q = __shfl_sync(mask, Z[b], mate);
+    const i64 z = 2 * u + 1 == QH ? Z[b] : high ? q - Z[b] : Z[b] + q;
+    zs[((high ? HP : 0) + low) * NV + b] = fx_split(z);
+    if (2 * u + 1 == QH) zs[(HP + low) * NV + b] = Fx2{0, 0};
   }
   __syncwarp(mask);
   const int up = max(kd - nd, 0), down = min(max(nd - kd, 0), 62);
   const i64 half = down ? (i64)1 << (down - 1) : 0;
 #pragma unroll
   for (int j = 0; j < J; ++j) {
-    const int k = u + U * j;
+    const int k = u + QH * j;
     if (k < NE) {
       const int a = k % NV, b = k / NV;
-      const Fx2 *z = ((a & 1) ? zd : zs) + b;
+      const Fx2 *z = zs + ((a & 1) ? HP * NV : 0) + b;
       // (with the products of the low halves: the result goes up by zsh)
       i64 m = 0, h = 0, l = 0;
 #pragma unroll
-      for (int v = 0; v < U; ++v) {
+      for (int v = 0; v < HP; ++v) {
         const Fx2 p = PhWs[v * NV + a], y = z[v * NV];
         l += fx_mad(y.l, p.l, 0) >> 32;
         m = fx_mad(y.h, p.l, m);
@@ -1144,41 +1169,150 @@ __device__ __forceinline__ void team_M_fx(const Basis<NU, NV> &B, const Fx2 *Gs,
   }
 }
 
-// k_cheb: the Chebyshev mass solve (Saad Alg. 12.1, src/rhs.jl:920-939). Elements are visited in
-// decreasing order of their step counts (k_prep lists them by count), so the longest solves start
-// first. The team keeps the residual r, the iterate X and the direction d of its entries in
-// registers and d in its shared slot.
-//
-// The iteration runs in fixed point on the system scaled by the middle θ of the spectral interval,
-// (M/θ) X' = R with X' = θX, whose spectrum is 1 ± ε, ε = δ/θ: the integers of r, X' and d keep the
-// exponent of R through all steps (the solution grows by at most 1/(1 - ε), for which R gets
-// headroom), and d goes into the products with M as d 2^nd, at the top of its range. Elements with
-// ε > 31/32, θ < 1/8 or max|G| > 7 and right-hand sides that are not finite take it in FP64.
+// k_cheb's iteration in FP64, for the elements beyond the limits of the fixed-point form
+template <int NU, int NV>
+__device__ __noinline__ void cheb_fp64(const Basis<NU, NV> &B, const StageIO &S, const i64 *G, int sG,
+                                       const double (&R)[MassTeam<NU, NV>::J], double th, double de, int n, int u,
+                                       unsigned mask, size_t Eu, int e, double *xs, double *X, double *zs,
+                                       bool &fin) {
+  using T = MassTeam<NU, NV>;
+  constexpr int QH = T::QH, NE = T::NE, J = T::J;
+  const double gs = ldexp(1.0, sG), s1 = th / de, ith = 1.0 / th;
+  double rr[J];
+#pragma unroll 1
+  for (int j = 0; j < J; ++j) {
+    const int k = u + QH * j;
+    rr[j] = R[j];
+    if (k < NE) {
+      X[k] = 0.0;
+      xs[k] = R[j] * ith;
+    }
+  }
+  __syncwarp(mask);
+  double rho = 1.0 / s1;
+#pragma unroll 1
+  for (int step = 1; step <= n; ++step) {
+#pragma unroll 1
+    for (int j = 0; j < J; ++j) {
+      const int k = u + QH * j;
+      if (k < NE) {
+        X[k] += xs[k];
+        rr[j] -= xs[k];
+      }
+    }
+    if (step == n) break;
+    // r += K d: row u at the points, weighted, and back (zs holds QH rows of NV)
+    double t[NV], z[NV];
+#pragma unroll
+    for (int b = 0; b < NV; ++b) {
+      t[b] = z[b] = 0.0;
+#pragma unroll
+      for (int a = 0; a < NV; ++a) t[b] = fma(B.Ph[u][a], xs[a + NV * b], t[b]);
+    }
+#pragma unroll 1
+    for (int s2 = 0; s2 < QH; ++s2) {
+      double y = 0.0;
+#pragma unroll
+      for (int b = 0; b < NV; ++b) y = fma(t[b], B.Ph[s2][b], y);
+      y *= (double)G[(u + QH * s2) * Eu] * gs;
+#pragma unroll
+      for (int b = 0; b < NV; ++b) z[b] = fma(y, B.PhW[s2][b], z[b]);
+    }
+#pragma unroll
+    for (int b = 0; b < NV; ++b) zs[u * NV + b] = z[b];
+    __syncwarp(mask);
+    const double rhon = 1.0 / (2.0 * s1 - rho);
+    const double c1 = rhon * rho, c2 = 2.0 * rhon / de;
+#pragma unroll 1
+    for (int j = 0; j < J; ++j) {
+      const int k = u + QH * j;
+      if (k < NE) {
+        for (int v = 0; v < QH; ++v) rr[j] = fma(B.PhW[v][k % NV], zs[v * NV + k / NV], rr[j]);
+        xs[k] = fma(c1, xs[k], c2 * rr[j]);
+      }
+    }
+    rho = rhon;
+    __syncwarp(mask);
+  }
+#pragma unroll 1
+  for (int j = 0; j < J; ++j) {
+    const int k = u + QH * j;
+    if (k < NE) store_v(S, e + Eu * k, X[k], fin);
+  }
+}
+
+// 1/D for 1 ≤ D ≤ 2 as integers of 2^-59: FP32's reciprocal and two steps of Newton's method
+__device__ __forceinline__ i64 fx_recip(i64 D) {
+  const float f = __uint_as_float((unsigned)(D >> 36) - (1u << 23) + (127u << 23));   // D ≥ 2^59: its top 24 bits
+  i64 r = (i64)((1.0f / f) * 1073741824.0f) << 29;
+  const Fx2 d = fx_split(D);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const Fx2 q = fx_split(r), t = fx_split(((i64)1 << 60) - (fx_mul(d, q) << 2));     // 2 - D r
+    r = fx_mul(q, t) << 2;
+  }
+  return r;
+}
+
 template <int NU, int NV>
 __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &F, const StageIO &S, int g0) {
-  WEDG_TEAM_SETUP(g0);
-  constexpr int QH = T::QH;
+  using T = MassTeam<NU, NV>;
+  constexpr int QH = T::QH, NE = T::NE, J = T::J, HP = T::HP;
+  __shared__ double sh[T::TPB * T::SLOT];
+  __shared__ Fx2 Phf[HP * NV], PhWf[HP * NV];
+  __shared__ int pref[NBIN];
+  for (int i = threadIdx.x; i < HP * NV; i += blockDim.x) {
+    Phf[i] = Fx2{B.fPh[i / NV][i % NV].h, B.fPh[i / NV][i % NV].l};
+    PhWf[i] = Fx2{B.fPhW[i / NV][i % NV].h, B.fPhW[i / NV][i % NV].l};
+  }
+  if (F.sorted && threadIdx.x < 32) {                    // pref[b]: the elements in the bins above b
+    int carry = 0;
+#pragma unroll
+    for (int b0 = 0; b0 < NBIN; b0 += 32) {
+      const int b = NBIN - 1 - b0 - (int)threadIdx.x, own = b >= 0 ? F.bin_count[S.parity * NBIN + b] : 0;
+      int x = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(~0u, x, o);
+        if ((int)threadIdx.x >= o) x += y;
+      }
+      if (b >= 0) pref[b] = carry + x - own;
+      carry += __shfl_sync(~0u, x, 31);
+    }
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, tw = lane / QH;
+  if (tw >= T::TPW) return;
+  const int u = lane - tw * QH, lane0 = tw * QH, slot = (threadIdx.x >> 5) * T::TPW + tw, g = g0 + slot;
+  if (g >= F.E) return;
+  if (err_word(F) != ERR_NONE) return;
+  const unsigned mask = ((1u << QH) - 1u) << lane0;
+  const size_t Eu = (size_t)F.E;
   const int e = mass_element(F, S, g, pref);
+  double *xs = sh + slot * T::SLOT, *X = xs + NE, *zs = X + NE;
   const double th = F.th[e], de = F.de[e];
-  const double s1 = th / de;
   const int n = F.cheb_common ? F.nmax[S.parity] : F.nst[e];
-  const double ith = 1.0 / th;
   const i64 *G = reinterpret_cast<const i64 *>(F.G) + e;
   const GPack gp(G[(size_t)QH * QH * Eu]);
   double R[J];
   int hr = 0;
 #pragma unroll
   for (int j = 0; j < J; ++j) {
-    const int k = u + U * j;
+    const int k = u + QH * j;
     R[j] = k < NE ? F.mrhs[k * Eu + e] : 0.0;
     hr = max(hr, fx_abs_hi(R[j]));
   }
-  hr = __reduce_max_sync(tmask, hr);
+  // the thread's row of G 2^ng, just below 2^60
+  Fx2 *Gs = reinterpret_cast<Fx2 *>(zs + T::ZR);
+  if (n > 1)
+#pragma unroll
+    for (int s2 = 0; s2 < QH; ++s2) Gs[u + QH * s2] = fx_split(G[(u + QH * s2) * Eu] << gp.ng);
+  hr = __reduce_max_sync(mask, hr);
   bool fin = true;
-  __shared__ i64 Xsh[T::TPB * NE];
+  const double ith = 1.0 / th, eps = de * ith;
   // max|G| from the ends of the interval
   const double gmax = fmax(fabs(1.0 - (th + de)), fabs(1.0 - (th - de)));
-  if (fx_finite(hr) && s1 >= 32.0 / 31.0 && th >= 0.125 && gmax <= 7.0) {
+  if (fx_finite(hr) && eps <= 31.0 / 32.0 && th >= 0.125 && gmax <= 7.0) {
     // R with headroom: the entries of X' and d stay below |R|max + 2 ε/(1 - ε) |R| and those of M d below
     // that with |R| (1 + max|G|) (the Euclidean norm, from the entries' high words in FP32, with a
     // little to spare)
@@ -1189,123 +1323,70 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
       const float f = x > 0 ? __int_as_float(x << 3) : 0.0f;
       r2 = fmaf(f, f, r2);
     }
-    r2 = (float)__reduce_add_sync(tmask, (unsigned)(r2 * 1024.0f) + 1) * (1.0f / 1024.0f);
-    const float eps = (float)(de / th);
-    const float grow = 1.0f + 0.51f * (1.0f + (float)gmax) * fmaxf(1.0f, 2.0f * eps / (1.0f - eps)) * sqrtf(r2);
+    r2 = (float)__reduce_add_sync(mask, (unsigned)(r2 * 1024.0f) + 1) * (1.0f / 1024.0f);
+    const float ef = (float)eps;
+    const float grow = 1.0f + 0.51f * (1.0f + (float)gmax) * fmaxf(1.0f, 2.0f * ef / (1.0f - ef)) * sqrtf(r2);
     const int hb = (__float_as_int(grow) >> 23) - 126;
     const int er = fx_exp(hr) + hb;
+    // r in registers, X' and d (as d 2^nd, what M takes) in shared memory
     Fx2 *xf = reinterpret_cast<Fx2 *>(xs);
-    // r in registers, X' and d (as d 2^nd, what K takes) in shared memory
-    i64 *X = Xsh + tp.slot * NE;
+    i64 *Xf = reinterpret_cast<i64 *>(X);
     i64 rr[J];
 #pragma unroll
     for (int j = 0; j < J; ++j) {
-      const int k = u + U * j;
+      const int k = u + QH * j;
       rr[j] = fx_from(R[j], er);
       if (k < NE) {
-        X[k] = 0;
+        Xf[k] = 0;
         xf[k] = fx_split(rr[j] << hb);
       }
     }
-    __syncwarp(tmask);
-    int nd = hb;                                   // d 2^nd, just below 2^61, is what K takes
-    // the unit's rows of G 2^ng, just below 2^60
-    __shared__ Fx2 Gsh[T::TPB * T::GSLOT];
-    Fx2 *Gs = Gsh + tp.slot * T::GSLOT;
-    if (n > 1)
-#pragma unroll 1
-      for (int t = 0; t < 2; ++t) {
-        const int r = t == 0 ? u : QH - 1 - u;
-#pragma unroll
-        for (int s2 = 0; s2 < QH; ++s2) Gs[r + QH * s2] = fx_split(G[(r + QH * s2) * Eu] << gp.ng);
-      }
+    __syncwarp(mask);
+    int nd = hb;                                   // d 2^nd, just below 2^61, is what M takes
     const int kd = max(gp.sG - gp.ng + 64, -62);   // (team_M_fx's zsh takes the levels' exponents up to this one)
     const Fx2 ithf = fx_split(fx_scalar(ith, FX_BIAS - 56));
-    double rho = 1.0 / s1;
+    // the scalars, as integers of 2^-59: with q = ρ θ/δ the recurrence ρ' = 1/(2 θ/δ - ρ) is q' = 1/(2 - ε² q),
+    // and d' = ρ'ρ d + 2 (ρ'/δ) r in the scaled system is ε² q q' d + 2 q' r
+    const Fx2 e2 = fx_split(fx_scalar(eps * eps, FX_BIAS - 59));
+    i64 q = (i64)1 << 59;                          // ρ = δ/θ: q = 1
 #pragma unroll 1
     for (int step = 1; step <= n; ++step) {
 #pragma unroll
       for (int j = 0; j < J; ++j) {
-        const int k = u + U * j;
-        if (k < NE) {
-          X[k] += fx_join(xf[k]) >> nd;
-        }
+        const int k = u + QH * j;
+        if (k < NE) Xf[k] += fx_join(xf[k]) >> nd;
       }
       if (step == n) break;
-      team_M_fx<NU, NV>(B, Gs, kd, ithf, nd, u, tmask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs),
-                        reinterpret_cast<Fx2 *>(zd), rr);
-      // d = c1 d + c2 r, c1 = ρ' ρ < 1 and c2 = 2 ρ' θ/δ ≤ 2 as integers of 2^-59
-      const double rhon = 1.0 / (2.0 * s1 - rho);
-      const Fx2 c1 = fx_split(fx_from(rhon * rho, 1024)), c2 = fx_split(fx_from(2.0 * rhon * s1, 1024));
-      rho = rhon;
+      team_M_fx<NU, NV>(B, Gs, kd, ithf, nd, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs), rr);
+      const i64 eq = fx_mul(fx_split(q), e2) << 2;                       // ε² q
+      q = fx_recip(((i64)1 << 60) - eq);
+      const Fx2 qs = fx_split(q), c1 = fx_split(fx_mul(qs, fx_split(eq)) << 2), c2 = fx_split(2 * q);
       int hd = 0;
       i64 dd[J];
 #pragma unroll
       for (int j = 0; j < J; ++j) {
-        const int k = u + U * j;
+        const int k = u + QH * j;
         const Fx2 d = fx_split(k < NE ? fx_join(xf[k]) >> nd : 0), r = fx_split(rr[j]);
         const i64 m = fx_mad(d.h, c1.l, fx_mad(d.l, c1.h, fx_mad(r.h, c2.l, fx_mad(r.l, c2.h, 1 << 26))));
         dd[j] = (fx_mad(d.h, c1.h, fx_mad(r.h, c2.h, 0)) << 5) + (m >> 27);
         hd = max(hd, fx_hi(dd[j]));
       }
-      nd = fx_room(__reduce_max_sync(tmask, hd));
+      nd = fx_room(__reduce_max_sync(mask, hd));
 #pragma unroll
       for (int j = 0; j < J; ++j) {
-        const int k = u + U * j;
+        const int k = u + QH * j;
         if (k < NE) xf[k] = fx_split(dd[j] << nd);
       }
-      __syncwarp(tmask);
+      __syncwarp(mask);
     }
     const double sc = fx_pow2(er - FX_BIAS) * ith;
 #pragma unroll
     for (int j = 0; j < J; ++j) {
-      const int k = u + U * j;
-      if (k < NE) store_v(S, e + Eu * k, __dmul_rn((double)X[k], sc), fin);
+      const int k = u + QH * j;
+      if (k < NE) store_v(S, e + Eu * k, __dmul_rn((double)Xf[k], sc), fin);
     }
   } else {
-    const double gs = ldexp(1.0, gp.sG);
-    auto Gd = [&](int r, int s2) { return (double)G[(r + QH * s2) * Eu] * gs; };
-    double *X = reinterpret_cast<double *>(Xsh) + tp.slot * NE;
-    double rr[J];
-#pragma unroll
-    for (int j = 0; j < J; ++j) {
-      const int k = u + U * j;
-      rr[j] = R[j];
-      if (k < NE) {
-        X[k] = 0.0;
-        xs[k] = R[j] * ith;
-      }
-    }
-    __syncwarp(tmask);
-    double rho = 1.0 / s1;
-#pragma unroll 1
-    for (int step = 1; step <= n; ++step) {
-#pragma unroll
-      for (int j = 0; j < J; ++j) {
-        const int k = u + U * j;
-        if (k < NE) {
-          const double d = xs[k];
-          X[k] += d;
-          rr[j] -= d;
-        }
-      }
-      if (step == n) break;
-      team_K<NU, NV, 1>(B, Gd, u, tmask, Phs, PhWs, xs, zs, zd, rr);   // r += K d
-      const double rhon = 1.0 / (2.0 * s1 - rho);
-      const double c1 = rhon * rho, c2 = 2.0 * rhon / de;
-#pragma unroll
-      for (int j = 0; j < J; ++j) {
-        const int k = u + U * j;
-        if (k < NE) xs[k] = fma(c1, xs[k], c2 * rr[j]);
-      }
-      rho = rhon;
-      __syncwarp(tmask);
-    }
-#pragma unroll
-    for (int j = 0; j < J; ++j) {
-      const int k = u + U * j;
-      if (k < NE) store_v(S, e + Eu * k, X[k], fin);
-    }
+    cheb_fp64<NU, NV>(B, S, G, gp.sG, R, th, de, n, u, mask, Eu, e, xs, X, zs, fin);
   }
   if (S.mode == OUT_RK4_LAST && !fin) atomicOr(F.nonfinite, 1u);
 }
@@ -1419,22 +1500,22 @@ __device__ __forceinline__ int team_tile() {
 }
 
 template <int NU, int NV>
-__global__ void __launch_bounds__(CHEB_THREADS, 4)
+__global__ void __launch_bounds__(CHEB_THREADS, 6)
     k_cheb(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ Fields F,
            const __grid_constant__ StageIO S) {
-  cheb_body<NU, NV>(B, F, S, blockIdx.x * team_tile<NU, NV>());
+  cheb_body<NU, NV>(B, F, S, blockIdx.x * mass_tile(NU, NV, false, blockDim.x));
 }
 
 template <int NU, int NV>
-__global__ void __launch_bounds__(CHEB_THREADS, 4)
+__global__ void __launch_bounds__(CHEB_THREADS, 3)
     k_cg(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ Fields F,
          const __grid_constant__ StageIO S) {
   cg_body<NU, NV>(B, F, S, blockIdx.x * team_tile<NU, NV>());
 }
 
-// tile = team_tile elements per virtual block; CG selects k_cg's body
+// tile = mass_tile elements per virtual block; CG selects k_cg's body
 template <int NU, int NV, bool CG>
-__global__ void __launch_bounds__(CHEB_THREADS, CG ? 3 : 4)
+__global__ void __launch_bounds__(CHEB_THREADS, CG ? 3 : 6)
     k_mass_m(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ MultiStage P) {
   for (int vb = blockIdx.x; vb < P.first[P.n]; vb += gridDim.x) {
     const int inst = multi_begin(P, vb);

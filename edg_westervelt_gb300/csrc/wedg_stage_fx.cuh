@@ -460,7 +460,9 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
   // order, the next stage state u + c k, the last stage u + (dt/6)(acc + k4) with the finite check
 #pragma unroll
   for (int i = 0; i < NU; ++i) x[i] = fx_split(X[c + NU * i]);
+  // kk = t f: f the integers' unit, but 1 for the constant mode (thread 0's first entry)
   const double un = (ok ? fx_unit(sX + 2 * dQ) : nan) * (usolve ? F.ic2e[e] : 1.0), u1 = ok ? 1.0 : nan;
+  const double un2 = __dmul_rn(2.0, un), unc = __dmul_rn(S.c, un);
   bool fin = true;
 #pragma unroll
   for (int b = 0; b < NU; ++b) {
@@ -469,13 +471,13 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
     if (b == 0) y = fx_down(fx_join(x[0]), dQ);
     else y = (b & 1) ? fx_dot<1, 2, NU>(xs, q) : fx_dot<2, 2, NU>(xs, q);
     const bool first = b == 0 && c == 0;
-    const double t = first ? x00 : (double)y, f = first ? u1 : un;   // kk = t f
+    const double t = first ? x00 : (double)y, f = first ? u1 : un;
     const size_t l = e + Eu * (c + NU * b);
     if (S.mode == OUT_RHS || usolve) {
       S.ut[l] = __dmul_rn(t, f);
     } else if (S.mode == OUT_RK4_STAGE) {
-      S.accu[l] = S.first ? __dmul_rn(t, f) : fma(t, __dmul_rn(2.0, f), S.accu[l]);
-      S.su[l] = fma(t, __dmul_rn(S.c, f), S.u0[l]);
+      S.accu[l] = S.first ? __dmul_rn(t, f) : fma(t, first ? 2.0 * u1 : un2, S.accu[l]);
+      S.su[l] = fma(t, first ? S.c * u1 : unc, S.u0[l]);
     } else if (S.mode == OUT_RK4_LAST) {
       // Chebyshev mode only: no error can arise after k_prep, so u is updated in place now
       const double x1 = fma(S.c, fma(t, f, S.accu[l]), S.u0[l]);

@@ -684,7 +684,7 @@ cudaError_t multi_stage_launch(const Launchers &L, const void *basis, int nu, in
   const int tile = kind == MK_PREP    ? prep_tile(nu, threads)
                    : kind == MK_BND   ? bnd_tile(nu)
                    : kind == MK_STAGE ? stage_tile(nu)
-                                      : mass_tile(nu, nv, !args.empty() && args[0].F.cg, threads);
+                                      : mass_tile(nu, nv, threads);
   const int n = (int)args.size();
   for (int c0 = 0; c0 < n; c0 += MultiStage::cap) {
     const int m = std::min(n - c0, MultiStage::cap);

@@ -199,7 +199,7 @@ cudaError_t launch_mass(const void *basis, const Fields &F, const StageIO &S, in
   if (blocks <= 0) return cudaSuccess;
   const Basis<NU, NV> &B = *static_cast<const Basis<NU, NV> *>(basis);
   threads = (threads >= 32 && threads <= CHEB_THREADS && threads % 32 == 0) ? threads : CHEB_THREADS;
-  const int tpb = mass_tile(NU, NV, F.cg, threads);
+  const int tpb = mass_tile(NU, NV, threads);
   const int grid = (F.E + tpb - 1) / tpb;
   if (F.cg) k_cg<NU, NV><<<grid, threads, 0, st>>>(B, F, S);
   else k_cheb<NU, NV><<<grid, threads, 0, st>>>(B, F, S);

@@ -100,8 +100,8 @@ struct Fields {
   const double *bsp[4], *bspn[4];
   const double *PiSP, *PiBSP2, *PiCdiv, *PiDdiv, *srcP;
   const double *beta2;        // 2β at the high-order points, [(r + QH s) E + e]
-  // G = 2βv at the high-order points: for k_cheb as integers of one exponent per element, which row
-  // QH² holds with a normalising shift (GPack); k_cg and k_adj_mass keep doubles of their own there.
+  // G = 2βv at the high-order points, as integers of one exponent per element, which row QH² holds with
+  // a normalising shift (GPack); k_adj_mass keeps doubles of its own there.
   // Row QH² + 1: the largest high words of U and V beside the constant mode (k_stage's exponents)
   double *tr, *G, *th, *de;
   // the flux slots of the physical sides projected on the face modes: [(q 4 + s) N + m], q over the
@@ -296,6 +296,7 @@ __device__ __forceinline__ void ph_row_mid(const double (&Ph)[QH][NV], const X &
 // Row QH² of G: the exponent sG of the element's integers G (G = integer 2^sG) and the shift ng that
 // takes their largest to [2^59, 2^60)
 struct GPack {
+  static constexpr int BAD = INT_MIN;                    // sG where V or β is not finite
   int sG, ng;
   __device__ GPack(int s, i64 lo, i64 hi) : sG(s) {
     const i64 top = max(hi, -lo);
@@ -703,7 +704,6 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
       if (bad) atomicMin(F.err, 2ull * ((unsigned long long)s * NQ * N + r + (unsigned long long)m * NQ) + bad);
     }
   }
-  if (F.cg) return;
 
   // ---- Chebyshev interval of the element: v_q = P_h V P_h^T, G = 2βv_q, a± = 1 - extrema(G), in fixed
   //      point (the integers of V and 2β share an exponent over the element)
@@ -775,7 +775,8 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
     kmin = (i64)((u64)(unsigned)h0 << 32 | l0);
   }
   if (r != 0) return;
-  Gi[(size_t)QH * QH * E + e] = GPack(sG, kmin, kmax).word();
+  Gi[(size_t)QH * QH * E + e] = GPack(nan ? GPack::BAD : sG, kmin, kmax).word();
+  if (F.cg) return;                                      // (k_cg finds a matrix that is not positive definite)
   const double gmin = ldexp((double)kmin, sG), gmax = ldexp((double)kmax, sG);
   const double amin = 1.0 - gmax, amax = 1.0 - gmin;
   if (nan || !(amin > 0.0)) {
@@ -1000,34 +1001,6 @@ __device__ __forceinline__ void team_K(const Basis<NU, NV> &B, const GAt &G, int
   }
 }
 
-// Shared memory of a team kernel and its setup: the bin prefix (sorted order) and the bases;
-// g0 is the first element slot of the block (slots in the order of mass_element)
-#define WEDG_TEAM_SETUP(g0)                                                                     \
-  using T = ChebTeam<NU, NV>;                                                                   \
-  constexpr int U = T::U, NE = T::NE, J = T::J;                                                 \
-  __shared__ double sh[T::TPB * T::SLOT];                                                       \
-  __shared__ double Phs[T::QH * NV], PhWs[T::QH * NV];                                          \
-  __shared__ int pref[NBIN];                                                                    \
-  for (int i = threadIdx.x; i < T::QH * NV; i += blockDim.x) {                                 \
-    Phs[i] = B.Ph[i / NV][i % NV];                                                              \
-    PhWs[i] = B.PhW[i / NV][i % NV];                                                            \
-  }                                                                                             \
-  if (F.sorted && threadIdx.x == 0) {                                                           \
-    int acc_ = 0;                                                                               \
-    for (int b = NBIN - 1; b >= 0; --b) { pref[b] = acc_; acc_ += F.bin_count[S.parity * NBIN + b]; } \
-  }                                                                                             \
-  __syncthreads();                                                                              \
-  TeamPos tp;                                                                                   \
-  if (!team_pos<NU, NV>(tp)) return;                                                            \
-  const int g = (g0) + tp.slot;                                                                 \
-  if (g >= F.E) return;                                                                         \
-  if (err_word(F) != ERR_NONE) return;                                                          \
-  const int u = tp.u;                                                                           \
-  const unsigned tmask = tp.mask;                                                               \
-  const size_t Eu = (size_t)F.E;                                                                \
-  double *xs = sh + tp.slot * T::SLOT, *zs = xs + NE, *zd = zs + U * NV;                        \
-  (void)Eu;
-
 // k_cheb: the Chebyshev mass solve (Saad Alg. 12.1, src/rhs.jl:920-939), a team of QH threads per
 // element: thread u takes row u of the point grid and J of the modal entries. Elements are visited in
 // decreasing order of their step counts (k_prep lists them by count), so the longest solves start
@@ -1053,18 +1026,16 @@ struct MassTeam {
   static constexpr int ZR = 2 * HP * NV;                // the sums and differences of row pairs
   static constexpr int SLOT = (2 * NE + ZR + QH * QH) | 1;   // d, X', the rows, G; odd: bank conflicts
 };
-__host__ __device__ constexpr int mass_tile(int nu, int nv, bool cg, int threads) {
-  const int qh = qhigh(nu, nv);
-  return (threads / 32) * (32 / (cg ? (qh + 1) / 2 : qh));
+__host__ __device__ constexpr int mass_tile(int nu, int nv, int threads) {
+  return (threads / 32) * (32 / qhigh(nu, nv));
 }
 
-// The thread's part of r -= (M/θ) d, M = I - P_h^T W G P_h, for d in xs as d 2^nd (complete, after a
-// __syncwarp) and G in Gs. The levels of the sum factorisation keep the exponents fixed by the
-// operators; 2^kd takes the last one to the integers of d 2^nd. ith: 1/θ as an integer of 2^-56.
-template <int NU, int NV>
-__device__ __forceinline__ void team_M_fx(const Basis<NU, NV> &B, const Fx2 *Gs, int kd, Fx2 ith, int nd, int u,
-                                          int lane0, unsigned mask, const Fx2 *Phs, const Fx2 *PhWs, const Fx2 *xs,
-                                          Fx2 *zs, i64 (&r)[MassTeam<NU, NV>::J]) {
+// One product with K = P_h^T W G P_h for x in xs (Fx2, below 2^61, complete, after a __syncwarp) and G in
+// Gs: use(j, k, y) for the thread's entries k = u + QH j, where K x = y 2^(sG - ng + 64) (GPack) in the
+// integers of x. The levels of the sum factorisation keep the exponents fixed by the operators.
+template <int NU, int NV, class Use>
+__device__ __forceinline__ void team_K_fx(const Basis<NU, NV> &B, const Fx2 *Gs, int u, int lane0, unsigned mask,
+                                          const Fx2 *Phs, const Fx2 *PhWs, const Fx2 *xs, Fx2 *zs, const Use &use) {
   using T = MassTeam<NU, NV>;
   constexpr int QH = T::QH, HP = T::HP, NE = T::NE, J = T::J, NP = (NV + 1) / 2;
   // The levels leave headroom for sums that K does not reach: its rows of the grid stay below
@@ -1142,8 +1113,6 @@ __device__ __forceinline__ void team_M_fx(const Basis<NU, NV> &B, const Fx2 *Gs,
     if (2 * u + 1 == QH) zs[(HP + low) * NV + b] = Fx2{0, 0};
   }
   __syncwarp(mask);
-  const int up = max(kd - nd, 0), down = min(max(nd - kd, 0), 62);
-  const i64 half = down ? (i64)1 << (down - 1) : 0;
 #pragma unroll
   for (int j = 0; j < J; ++j) {
     const int k = u + QH * j;
@@ -1161,10 +1130,7 @@ __device__ __forceinline__ void team_M_fx(const Basis<NU, NV> &B, const Fx2 *Gs,
         h = fx_mad(y.h, p.h, h);
       }
       m += l;
-      const i64 Kd = ((((h << zsh) + (m >> (32 - zsh))) << up) + half) >> down;
-      const Fx2 t = fx_split((fx_join(xs[k]) >> nd) - Kd);
-      m = fx_mad(t.h, ith.l, fx_mad(t.l, ith.h, (fx_mad(t.l, ith.l, 0) >> 32) + (1 << 23)));
-      r[j] -= (fx_mad(t.h, ith.h, 0) << 8) + (m >> 24);
+      use(j, k, (h << zsh) + (m >> (32 - zsh)));
     }
   }
 }
@@ -1254,40 +1220,45 @@ __device__ __forceinline__ i64 fx_recip(i64 D) {
   return r;
 }
 
+// The start of k_cheb and k_cg: the operators' tables, the elements by count (pref[b]: those in the bins
+// above b), and the thread's team, row u and slot of elements g; threads without one return
+#define WEDG_MASS_SETUP(g0) \
+  using T = MassTeam<NU, NV>; \
+  constexpr int QH = T::QH, NE = T::NE, J = T::J, HP = T::HP; \
+  __shared__ double sh[T::TPB * T::SLOT]; \
+  __shared__ Fx2 Phf[HP * NV], PhWf[HP * NV]; \
+  __shared__ int pref[NBIN]; \
+  for (int i = threadIdx.x; i < HP * NV; i += blockDim.x) { \
+    Phf[i] = Fx2{B.fPh[i / NV][i % NV].h, B.fPh[i / NV][i % NV].l}; \
+    PhWf[i] = Fx2{B.fPhW[i / NV][i % NV].h, B.fPhW[i / NV][i % NV].l}; \
+  } \
+  if (F.sorted && threadIdx.x < 32) { \
+    int carry = 0; \
+_Pragma("unroll") \
+    for (int b0 = 0; b0 < NBIN; b0 += 32) { \
+      const int b = NBIN - 1 - b0 - (int)threadIdx.x, own = b >= 0 ? F.bin_count[S.parity * NBIN + b] : 0; \
+      int x = own; \
+_Pragma("unroll") \
+      for (int o = 1; o < 32; o <<= 1) { \
+        const int y = __shfl_up_sync(~0u, x, o); \
+        if ((int)threadIdx.x >= o) x += y; \
+      } \
+      if (b >= 0) pref[b] = carry + x - own; \
+      carry += __shfl_sync(~0u, x, 31); \
+    } \
+  } \
+  __syncthreads(); \
+  const int lane = threadIdx.x & 31, tw = lane / QH; \
+  if (tw >= T::TPW) return; \
+  const int u = lane - tw * QH, lane0 = tw * QH, slot = (threadIdx.x >> 5) * T::TPW + tw, g = (g0) + slot; \
+  if (g >= F.E) return; \
+  if (err_word(F) != ERR_NONE) return; \
+  const unsigned mask = ((1u << QH) - 1u) << lane0; \
+  const size_t Eu = (size_t)F.E;
+
 template <int NU, int NV>
 __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &F, const StageIO &S, int g0) {
-  using T = MassTeam<NU, NV>;
-  constexpr int QH = T::QH, NE = T::NE, J = T::J, HP = T::HP;
-  __shared__ double sh[T::TPB * T::SLOT];
-  __shared__ Fx2 Phf[HP * NV], PhWf[HP * NV];
-  __shared__ int pref[NBIN];
-  for (int i = threadIdx.x; i < HP * NV; i += blockDim.x) {
-    Phf[i] = Fx2{B.fPh[i / NV][i % NV].h, B.fPh[i / NV][i % NV].l};
-    PhWf[i] = Fx2{B.fPhW[i / NV][i % NV].h, B.fPhW[i / NV][i % NV].l};
-  }
-  if (F.sorted && threadIdx.x < 32) {                    // pref[b]: the elements in the bins above b
-    int carry = 0;
-#pragma unroll
-    for (int b0 = 0; b0 < NBIN; b0 += 32) {
-      const int b = NBIN - 1 - b0 - (int)threadIdx.x, own = b >= 0 ? F.bin_count[S.parity * NBIN + b] : 0;
-      int x = own;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(~0u, x, o);
-        if ((int)threadIdx.x >= o) x += y;
-      }
-      if (b >= 0) pref[b] = carry + x - own;
-      carry += __shfl_sync(~0u, x, 31);
-    }
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, tw = lane / QH;
-  if (tw >= T::TPW) return;
-  const int u = lane - tw * QH, lane0 = tw * QH, slot = (threadIdx.x >> 5) * T::TPW + tw, g = g0 + slot;
-  if (g >= F.E) return;
-  if (err_word(F) != ERR_NONE) return;
-  const unsigned mask = ((1u << QH) - 1u) << lane0;
-  const size_t Eu = (size_t)F.E;
+  WEDG_MASS_SETUP(g0);
   const int e = mass_element(F, S, g, pref);
   double *xs = sh + slot * T::SLOT, *X = xs + NE, *zs = X + NE;
   const double th = F.th[e], de = F.de[e];
@@ -1343,8 +1314,8 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
     }
     __syncwarp(mask);
     int nd = hb;                                   // d 2^nd, just below 2^61, is what M takes
-    const int kd = max(gp.sG - gp.ng + 64, -62);   // (team_M_fx's zsh takes the levels' exponents up to this one)
-    const Fx2 ithf = fx_split(fx_scalar(ith, FX_BIAS - 56));
+    const int kd = max(gp.sG - gp.ng + 64, -62);
+    const Fx2 ithf = fx_split(fx_scalar(ith, FX_BIAS - 56));          // 1/θ as an integer of 2^-56
     // the scalars, as integers of 2^-59: with q = ρ θ/δ the recurrence ρ' = 1/(2 θ/δ - ρ) is q' = 1/(2 - ε² q),
     // and d' = ρ'ρ d + 2 (ρ'/δ) r in the scaled system is ε² q q' d + 2 q' r
     const Fx2 e2 = fx_split(fx_scalar(eps * eps, FX_BIAS - 59));
@@ -1357,7 +1328,14 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
         if (k < NE) Xf[k] += fx_join(xf[k]) >> nd;
       }
       if (step == n) break;
-      team_M_fx<NU, NV>(B, Gs, kd, ithf, nd, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs), rr);
+      // r -= (M/θ) d, M d = d - K d, with K d 2^nd = y 2^kd
+      const int up = max(kd - nd, 0), down = min(max(nd - kd, 0), 62);
+      const i64 half = down ? (i64)1 << (down - 1) : 0;
+      team_K_fx<NU, NV>(B, Gs, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs), [&](int j, int k, i64 y) {
+        const Fx2 t = fx_split((fx_join(xf[k]) >> nd) - (((y << up) + half) >> down));
+        const i64 m = fx_mad(t.h, ithf.l, fx_mad(t.l, ithf.h, (fx_mad(t.l, ithf.l, 0) >> 32) + (1 << 23)));
+        rr[j] -= (fx_mad(t.h, ithf.h, 0) << 8) + (m >> 24);
+      });
       const i64 eq = fx_mul(fx_split(q), e2) << 2;                       // ε² q
       q = fx_recip(((i64)1 << 60) - eq);
       const Fx2 qs = fx_split(q), c1 = fx_split(fx_mul(qs, fx_split(eq)) << 2), c2 = fx_split(2 * q);
@@ -1391,76 +1369,85 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
   if (S.mode == OUT_RK4_LAST && !fin) atomicOr(F.nonfinite, 1u);
 }
 
-// k_cg: the mass solve by conjugate gradients from X = R (src/rhs.jl:821-853), elements in mesh
-// order. The team first forms G = 2βv at the high-order points of its rows (each unit reads only
-// the rows it wrote), then iterates with p in its shared slot and the inner products summed over
-// the team's lanes in a fixed order, so that every lane takes the same decisions.
+// Σ over the team's QH threads of x, on every one of them: the same tree for each
+template <int QH>
+__device__ __forceinline__ double mass_sum(double x, int u, int lane0, unsigned mask) {
+  constexpr int top = QH > 8 ? 8 : QH > 4 ? 4 : QH > 2 ? 2 : 1;
+#pragma unroll
+  for (int o = top; o > 0; o >>= 1) {
+    const double y = __shfl_sync(mask, x, lane0 + (u + o < QH ? u + o : u));
+    if (u < o && u + o < QH) x += y;
+  }
+  return __shfl_sync(mask, x, lane0);
+}
+
+// k_cg: the mass solve by conjugate gradients from X = R (src/rhs.jl:821-853), elements in mesh order, on the
+// team layout of k_cheb: the products with K in fixed point on p as integers of its own exponent, the
+// vectors and inner products in FP64, summed over the team's lanes in a fixed order so that every lane
+// takes the same decisions. A chain of products and reductions bounds it, with three blocks an SM to hide
+// it. N = 97, q = 5: 405 us with FP64 products of half as many threads, 138 us so (and 11 us for the integers
+// of G, which k_prep writes).
 template <int NU, int NV>
 __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F, const StageIO &S, int g0) {
-  WEDG_TEAM_SETUP(g0);
-  constexpr int QH = T::QH;
+  WEDG_MASS_SETUP(g0);
   const int e = g;
-  {
-    // G rows u and QH-1-u of this element
-    const int r1 = u, r2 = QH - 1 - u;
-    auto vx = [&](int a, int b) { return S.xv[e + Eu * (a + NV * b)]; };
-    double Tp[NV], Tm[NV];
-    ph_row_pair<QH, NV>(B.Ph, r1, vx, Tp, Tm);
-    auto gput = [&](const double (&Tv)[NV], int r) {
-      double Y[QH];
-      ph_to_points<QH, NV>(B.Ph, Tv, Y);
+  double *xs = sh + slot * T::SLOT, *zs = xs + 2 * NE;
+  Fx2 *xf = reinterpret_cast<Fx2 *>(xs), *Gs = reinterpret_cast<Fx2 *>(zs + T::ZR);
+  const i64 *G = reinterpret_cast<const i64 *>(F.G) + e;
+  const GPack gp(G[(size_t)QH * QH * Eu]);
+  const bool g_ok = gp.sG != GPack::BAD;
 #pragma unroll
-      for (int s2 = 0; s2 < QH; ++s2) {
-        const size_t gi = (r + QH * s2) * Eu + e;
-        F.G[gi] = Y[s2] * F.beta2[gi];
-      }
-    };
-    gput(Tp, r1);
-    if (r2 != r1) gput(Tm, r2);
-  }
-  auto G = [&](int r, int s2) { return F.G[(r + QH * s2) * Eu + e]; };
+  for (int s2 = 0; s2 < QH; ++s2) Gs[u + QH * s2] = fx_split(g_ok ? G[(u + QH * s2) * Eu] << gp.ng : 0);
+  // y = K x for the threads' entries x[j]; NaN where x or G is not finite
+  auto K = [&](const double (&x)[J], double (&y)[J]) {
+    int hx = 0;
+#pragma unroll
+    for (int j = 0; j < J; ++j) hx = max(hx, fx_abs_hi(x[j]));
+    hx = __reduce_max_sync(mask, hx);
+    const int ex = fx_exp(hx);
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const int k = u + QH * j;
+      if (k < NE) xf[k] = fx_split(fx_from(x[j], ex));
+      y[j] = 0.0;
+    }
+    __syncwarp(mask);
+    const double sc = g_ok && fx_finite(hx) ? ldexp(1.0, ex - FX_BIAS + gp.sG - gp.ng + 64)
+                                            : __longlong_as_double(0x7ff8000000000000LL);
+    team_K_fx<NU, NV>(B, Gs, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs),
+                      [&](int j, int, i64 v) { y[j] = __dmul_rn((double)v, sc); });
+    __syncwarp(mask);
+  };
   double X[J], r[J], p[J], Ap[J];
   double r0 = 0;
 #pragma unroll
   for (int j = 0; j < J; ++j) {
-    const int k = u + U * j;
-    X[j] = r[j] = p[j] = 0.0;
-    if (k < NE) {
-      const double x = F.mrhs[k * Eu + e];
-      X[j] = x;
-      xs[k] = x;
-      r0 = fma(x, x, r0);
-    }
+    const int k = u + QH * j;
+    X[j] = k < NE ? F.mrhs[k * Eu + e] : 0.0;
+    r0 = fma(X[j], X[j], r0);
   }
-  r0 = sqrt(team_sum<U>(r0, tmask));
-  __syncwarp(tmask);
-  team_K<NU, NV, 1>(B, G, u, tmask, Phs, PhWs, xs, zs, zd, r);    // r = R - M X = K R for X = R
+  r0 = sqrt(mass_sum<QH>(r0, u, lane0, mask));
+  K(X, r);                                               // r = R - M X = K R for X = R
   double rr = 0;
 #pragma unroll
   for (int j = 0; j < J; ++j) {
     p[j] = r[j];
     rr = fma(r[j], r[j], rr);
   }
-  rr = team_sum<U>(rr, tmask);
+  rr = mass_sum<QH>(rr, u, lane0, mask);
   const int maxit = NV * NV + 10;
   int it = 0;
   bool bad = false;
   while (sqrt(rr) > F.mass_tol * r0 && it < maxit) {
     ++it;
-    __syncwarp(tmask);                              // the last phase 2 has read zs, zd
-#pragma unroll
-    for (int j = 0; j < J; ++j) {
-      const int k = u + U * j;
-      if (k < NE) xs[k] = p[j];
-    }
-    __syncwarp(tmask);
-#pragma unroll
-    for (int j = 0; j < J; ++j) Ap[j] = p[j];
-    team_K<NU, NV, -1>(B, G, u, tmask, Phs, PhWs, xs, zs, zd, Ap);  // A p = p - K p
+    K(p, Ap);
     double pAp = 0;
 #pragma unroll
-    for (int j = 0; j < J; ++j) pAp = fma(p[j], Ap[j], pAp);
-    pAp = team_sum<U>(pAp, tmask);
+    for (int j = 0; j < J; ++j) {
+      Ap[j] = __dsub_rn(p[j], Ap[j]);                    // A p = p - K p
+      pAp = fma(p[j], Ap[j], pAp);
+    }
+    pAp = mass_sum<QH>(pAp, u, lane0, mask);
     if (!(pAp > 0.0)) { bad = true; break; }
     const double al = rr / pAp;
     double rrn = 0;
@@ -1470,7 +1457,7 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
       r[j] = fma(-al, Ap[j], r[j]);
       rrn = fma(r[j], r[j], rrn);
     }
-    rrn = team_sum<U>(rrn, tmask);
+    rrn = mass_sum<QH>(rrn, u, lane0, mask);
     const double bt = rrn / rr;
 #pragma unroll
     for (int j = 0; j < J; ++j) p[j] = fma(bt, p[j], r[j]);
@@ -1485,13 +1472,13 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
   bool fin = true;
 #pragma unroll
   for (int j = 0; j < J; ++j) {
-    const int k = u + U * j;
+    const int k = u + QH * j;
     if (k < NE) store_v(S, e + Eu * k, X[j], fin);
   }
   if (S.mode == OUT_RK4_LAST && !fin) atomicOr(F.nonfinite, 1u);
 }
 
-#undef WEDG_TEAM_SETUP
+#undef WEDG_MASS_SETUP
 
 // The team kernels: a block of `threads` takes (threads / 32) teams per warp of elements
 template <int NU, int NV>
@@ -1503,14 +1490,14 @@ template <int NU, int NV>
 __global__ void __launch_bounds__(CHEB_THREADS, 6)
     k_cheb(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ Fields F,
            const __grid_constant__ StageIO S) {
-  cheb_body<NU, NV>(B, F, S, blockIdx.x * mass_tile(NU, NV, false, blockDim.x));
+  cheb_body<NU, NV>(B, F, S, blockIdx.x * mass_tile(NU, NV, blockDim.x));
 }
 
 template <int NU, int NV>
 __global__ void __launch_bounds__(CHEB_THREADS, 3)
     k_cg(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ Fields F,
          const __grid_constant__ StageIO S) {
-  cg_body<NU, NV>(B, F, S, blockIdx.x * team_tile<NU, NV>());
+  cg_body<NU, NV>(B, F, S, blockIdx.x * mass_tile(NU, NV, blockDim.x));
 }
 
 // tile = mass_tile elements per virtual block; CG selects k_cg's body

@@ -63,6 +63,38 @@ def test_mass_solves_over_the_spectra(gpu, q, mixed):
     assert w.size == Ph.shape[0]
 
 
+@pytest.mark.parametrize("q,mixed", [(1, True), (1, False), (4, True), (6, False), (7, False)])
+def test_cg_solves_over_the_spectra(gpu, q, mixed):
+    """The conjugate gradient solves of the same spans. They end at |r| <= 1e-14 |R|, an error of at most
+    κ 1e-14 in the Euclidean norm (NV times the largest entry); twice that, and κ NV² roundings of 1e-16
+    of the recurrence's r against the true one."""
+    from oracle.reference_rhs import dense_volume, edg_rhs_reference, reference_pre
+    N = 2
+    pp, po = _problem(q, N, mixed, mass_solver="cg")
+    nu, nv = pp["qu1"], pp["qv1"]
+    rng = np.random.default_rng(10 + q)
+    Ph = po["P_h_v"]
+    U = np.asfortranarray(rng.standard_normal((N, N, nu, nu)))
+    dense = dense_volume(reference_pre(po))
+    ws = W.Workspace(pp, N)
+    for lo, hi in SPANS[:6]:
+        V = np.zeros((N, N, nv, nv), order="F")
+        for j in range(N):
+            for k in range(N):
+                X = rng.standard_normal((nv, nv)) * np.exp(-0.5 * np.add.outer(np.arange(nv), np.arange(nv)))
+                X[0, 0] = 0.0
+                span = np.ptp(Ph @ X @ Ph.T)
+                X = X * ((hi - lo) / span) if span > 0 else X * 0.0
+                X[0, 0] = 2.0 * (hi - (Ph @ X @ Ph.T).max())
+                V[j, k] = X
+        a = edg_rhs_reference(U, V, 0.0, N, 1.0 / N, dense)
+        b = ws.rhs(U, V, 0.0)
+        g = np.einsum("ra,jkab,sb->jkrs", Ph, V, Ph)
+        kappa = float(((1 - g).max(axis=(2, 3)) / (1 - g).min(axis=(2, 3))).max())
+        tol = kappa * (2e-14 * nv + 1e-16 * nv * nv) + 1e-13
+        assert rel_max(a, b) < tol, (lo, hi, kappa, rel_max(a, b), tol)
+
+
 @pytest.mark.parametrize("q,mixed", [(2, True), (4, False), (7, False)])
 def test_rhs_scales_with_the_state(gpu, q, mixed):
     """With β = 0 and no data the right-hand side is linear: a state scaled by a power of two, as far as

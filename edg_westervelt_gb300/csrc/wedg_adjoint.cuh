@@ -21,9 +21,33 @@
 
 namespace wedg {
 
-// Threads per block of the per-element adjoint kernels: long serial work per thread, so small
-// blocks spread the elements of mid-size meshes over all SMs
-constexpr int ADJ_THREADS = 32;
+// Threads per block of k_adj_hats, a thread per element: small blocks spread mid-size meshes over the SMs
+constexpr int HATS_THREADS = 32;
+
+// k_adj_face takes a team of NU threads per element: thread r has column r of the modal blocks
+// (and, through shared memory, row r), point r of the four sides and mode r along them. With a
+// thread per element it had 512 warps at N = 128, fewer than the chip's 608 schedulers, each
+// with a chain of some 2 500 FP64 operations.
+constexpr int ADJ_THREADS = 128;
+__host__ __device__ constexpr int adj_tile(int nu) { return (ADJ_THREADS / 32) * (32 / nu); }
+template <int NU>
+struct AdjTeam {
+  static constexpr int TPW = 32 / NU;
+  static constexpr int TPB = adj_tile(NU);
+  static constexpr int SLOT = (12 * NU > 2 * NU * NU ? 12 * NU : 2 * NU * NU) | 1;   // odd: bank conflicts
+};
+// The thread's team, element e and the team's shared words s; threads without an element return
+#define WEDG_ADJ_TEAM(e0) \
+  using T = AdjTeam<NU>; \
+  __shared__ double sh[T::TPB * T::SLOT]; \
+  const int lane = threadIdx.x & 31, tw = lane / NU; \
+  if (tw >= T::TPW) return; \
+  const int r = lane - tw * NU, lane0 = tw * NU, slot = (threadIdx.x >> 5) * T::TPW + tw, e = (e0) + slot; \
+  if (e >= F.E) return; \
+  if (err_word(F) != ERR_NONE) return; \
+  const unsigned mask = (unsigned)((1ull << NU) - 1) << lane0; \
+  const size_t Eu = (size_t)F.E; \
+  double *s = sh + slot * T::SLOT;
 
 // Buffers of the adjoint kernels; every array in the state layout [e + E k] unless noted
 struct AdjIO {
@@ -68,11 +92,70 @@ __device__ __forceinline__ FaceWeights face_weights(const Fields &F, const FaceC
   return w;
 }
 
+// Traces of an n×n block X on the four sides (src/rhs.jl:388-410):
+//   oB[i] = Σ_b P[i,b] Σ_a El[a] X[a][b],  oT with Er,
+//   oL[i] = Σ_b P[i,b] Σ_a El[a] X[b][a],  oR with Er,
+// where El, Er are the values (DER false) or the derivatives (DER true) of the modes at the
+// two ends: Er[a] = ±(-1)^a El[a], so both ends come from the even and odd parts of one sum.
+// The bottom/top pair (AXIS 0) and the left/right pair (AXIS 1) are separate passes, so that
+// only one pair's end sums are live at a time. With SCALE, every output is multiplied by sc.
+template <int NQ, int NU, int n, bool DER, int AXIS, bool SCALE>
+__device__ __forceinline__ void trace2(const double (&X)[n][n], const double (&P)[NQ][NU], const double *El,
+                                       double *tr, int fam, int E, int e, double sc) {
+  double sA[n], sZ[n];   // the end sums at the low (B or L) and the high (T or R) end
+#pragma unroll
+  for (int b = 0; b < n; ++b) {
+    double xe = 0, xo = 0;
+#pragma unroll
+    for (int a = 0; a < n; a += 2) xe = fma(El[a], AXIS == 0 ? X[a][b] : X[b][a], xe);
+#pragma unroll
+    for (int a = 1; a < n; a += 2) xo = fma(El[a], AXIS == 0 ? X[a][b] : X[b][a], xo);
+    sA[b] = xe + xo;
+    sZ[b] = DER ? xo - xe : xe - xo;
+  }
+  auto put = [&](int i, double oA, double oZ) {
+    if constexpr (SCALE) { oA *= sc; oZ *= sc; }
+    tr[((fam * 4 + 2 * AXIS) * NQ + i) * (size_t)E + e] = oA;
+    tr[((fam * 4 + 2 * AXIS + 1) * NQ + i) * (size_t)E + e] = oZ;
+  };
+#pragma unroll
+  for (int i = 0; i < (NQ + 1) / 2; ++i) {
+    double eA = 0, eZ = 0, oA = 0, oZ = 0;
+#pragma unroll
+    for (int b = 0; b < n; b += 2) { eA = fma(P[i][b], sA[b], eA); eZ = fma(P[i][b], sZ[b], eZ); }
+    if (2 * i + 1 == NQ) {      // the middle point: the odd modes vanish there
+      put(i, eA, eZ);
+      continue;
+    }
+#pragma unroll
+    for (int b = 1; b < n; b += 2) { oA = fma(P[i][b], sA[b], oA); oZ = fma(P[i][b], sZ[b], oZ); }
+    put(i, eA + oA, eZ + oZ);
+    put(NQ - 1 - i, eA - oA, eZ - oZ);
+  }
+}
+
+template <int NQ, int NU, int n, bool DER, bool SCALE = false>
+__device__ __forceinline__ void trace4(const double (&X)[n][n], const double (&P)[NQ][NU], const double *El,
+                                       double *tr, int fam, int E, int e, double sc = 1.0) {
+  trace2<NQ, NU, n, DER, 0, SCALE>(X, P, El, tr, fam, E, e, sc);
+  trace2<NQ, NU, n, DER, 1, SCALE>(X, P, El, tr, fam, E, e, sc);
+}
+
+template <int n>
+__device__ __forceinline__ void load_regs(double (&X)[n][n], const double *x, int E, int e) {
+#pragma unroll
+  for (int b = 0; b < n; ++b)
+#pragma unroll
+    for (int a = 0; a < n; ++a) X[a][b] = x[e + (size_t)E * (a + n * b)];
+}
+
 // k_adj_hats: the weights of the slots A, D and F at every side point, the scaled traces of μ
 // (values and derivatives) and of ν (derivatives) (src/rhs.jl:412-473 transposed:
 // Â = (2/h) w_i tr_v(μ), D̂ = (4/h²) w_i tr_dv(μ), F̂ = -w_i tr_du(ν): the weights w_i folded
 // into the values Pw, the sign of F̂ into the end vector E1F, the mesh factors applied to the
 // traces); and nus.
+// A thread per element: its sums halve by mirrored points, which a team of NU threads would not (23 against
+// 27 us at N = 128, q = 4, cold caches).
 template <int NU, int NV>
 __device__ __forceinline__ void adj_hats_body(const Basis<NU, NV> &B, const Fields &F, const AdjIO &A, int e) {
   constexpr int NQ = NU;
@@ -96,14 +179,14 @@ __device__ __forceinline__ void adj_hats_body(const Basis<NU, NV> &B, const Fiel
 }
 
 template <int NU, int NV>
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_hats(const __grid_constant__ Basis<NU, NV> B,
+__global__ void __launch_bounds__(HATS_THREADS) k_adj_hats(const __grid_constant__ Basis<NU, NV> B,
                                                    const __grid_constant__ Fields F, const AdjIO A) {
   adj_hats_body<NU, NV>(B, F, A, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// tile = ADJ_THREADS elements per virtual block
+// tile = HATS_THREADS elements per virtual block
 template <int NU, int NV>
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_hats_m(const __grid_constant__ Basis<NU, NV> B,
+__global__ void __launch_bounds__(HATS_THREADS) k_adj_hats_m(const __grid_constant__ Basis<NU, NV> B,
                                                      const __grid_constant__ MultiAdj P) {
   for (int vb = blockIdx.x; vb < P.first[P.n]; vb += gridDim.x) {
     const int inst = multi_begin(P, vb);
@@ -111,99 +194,83 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_hats_m(const __grid_constan
   }
 }
 
-// k_adj_mass: gv += P_hᵀ (2βW ∘ vt_q ∘ μ_q) P_h on every element, by the team layout of the mass
-// solves: each unit forms the weights 2β vt_q of its two point rows (into G, which the forward
-// solve of this state no longer needs) and applies them to μ with team_K. With A.gbe, also the
-// β-derivative of μ·M(v) vt for β constant on the element, gbe[e] += Σ_q 2 W_q v_q vt_q μ_q.
+// k_adj_mass: gv += P_hᵀ (2βW ∘ vt_q ∘ μ_q) P_h on every element, on the layout of the mass solves: thread u
+// forms the weights 2β vt_q of row u of the point grid in FP64, and they are applied to μ in fixed point
+// with team_K_fx, both as integers of an exponent of their own. With A.gbe, also the β-derivative of
+// μ·M(v) vt for β constant on the element, gbe[e] += Σ_q 2 W_q v_q vt_q μ_q.
+//
+// N = 128, q = 4, cold caches: 80 us in FP64 with a thread per pair of rows, 59 us so.
 template <int NU, int NV>
 __device__ __forceinline__ void adj_mass_body(const Basis<NU, NV> &B, const Fields &F, const AdjIO &A, int e0) {
-  using T = ChebTeam<NU, NV>;
-  constexpr int QH = T::QH, U = T::U, NE = T::NE, J = T::J;
-  __shared__ double sh[T::TPB * T::SLOT];
-  __shared__ double Phs[QH * NV], PhWs[QH * NV];
-  for (int i = threadIdx.x; i < QH * NV; i += blockDim.x) {
-    Phs[i] = B.Ph[i / NV][i % NV];
-    PhWs[i] = B.PhW[i / NV][i % NV];
-  }
-  __syncthreads();
-  TeamPos tp;
-  if (!team_pos<NU, NV>(tp)) return;
-  const int e = e0 + tp.slot;
-  if (e >= F.E) return;
-  if (err_word(F) != ERR_NONE) return;
-  const int u = tp.u;
-  const unsigned tmask = tp.mask;
-  const size_t Eu = (size_t)F.E;
-  double *xs = sh + tp.slot * T::SLOT, *zs = xs + NE, *zd = zs + U * NV;
-  double db = 0.0;                                      // Σ over the unit's points of w v_q vt_q μ_q
-  {
-    const int r1 = u, r2 = QH - 1 - u;
-    auto tx = [&](int a, int b) { return A.vt[e + Eu * (a + NV * b)]; };
-    double Tp[NV], Tm[NV];
-    ph_row_pair<QH, NV>(B.Ph, r1, tx, Tp, Tm);
-    auto gput = [&](const double (&Tv)[NV], int r, double (&Y)[QH]) {
-      ph_to_points<QH, NV>(B.Ph, Tv, Y);
+  WEDG_MASS_TABLES()
+  WEDG_MASS_TEAM(e0)
+  const int e = g;
+  double *xs = sh + slot * T::SLOT, *zs = xs + 2 * NE;
+  Fx2 *xf = reinterpret_cast<Fx2 *>(xs), *Gs = reinterpret_cast<Fx2 *>(zs + T::ZR);
+  double Y[QH], Pr[NV];
+  auto row = [&](const double *x, double (&y)[QH]) {     // row u of P_h x P_h^T
+    double Tv[NV];
 #pragma unroll
-      for (int s2 = 0; s2 < QH; ++s2) {
-        const size_t gi = (r + QH * s2) * Eu + e;
-        F.G[gi] = Y[s2] * F.beta2[gi];
-      }
-    };
-    double Yp[QH], Ym[QH];
-    gput(Tp, r1, Yp);
-    if (r2 != r1) gput(Tm, r2, Ym);
-    if (A.gbe) {
-      auto vx = [&](int a, int b) { return A.xv[e + Eu * (a + NV * b)]; };
-      auto mx = [&](int a, int b) { return A.mu[e + Eu * (a + NV * b)]; };
-      double Vp[NV], Vm[NV], Mp[NV], Mm[NV];
-      ph_row_pair<QH, NV>(B.Ph, r1, vx, Vp, Vm);
-      ph_row_pair<QH, NV>(B.Ph, r1, mx, Mp, Mm);
-      auto row = [&](const double (&Y)[QH], const double (&Tv)[NV], const double (&Tmu)[NV]) {
-        double Yv[QH], Yu[QH];
-        ph_to_points<QH, NV>(B.Ph, Tv, Yv);
-        ph_to_points<QH, NV>(B.Ph, Tmu, Yu);
-        double r = 0.0;
+    for (int b = 0; b < NV; ++b) {
+      Tv[b] = 0.0;
 #pragma unroll
-        for (int s2 = 0; s2 < QH; ++s2) r = fma(B.wh[s2], Y[s2] * Yv[s2] * Yu[s2], r);
-        return r;
-      };
-      db = B.wh[r1] * row(Yp, Vp, Mp);
-      if (r2 != r1) db = fma(B.wh[r2], row(Ym, Vm, Mm), db);
+      for (int a = 0; a < NV; ++a) Tv[b] = fma(Pr[a], x[e + Eu * (a + NV * b)], Tv[b]);
     }
-  }
+    ph_to_points<QH, NV>(B.Ph, Tv, y);
+  };
+#pragma unroll
+  for (int a = 0; a < NV; ++a) Pr[a] = B.Ph[u][a];
+  row(A.vt, Y);
   if (A.gbe) {
-    db = team_sum<U>(db, tmask);
+    double Yv[QH], Yu[QH], db = 0.0;                     // Σ over the row of w v_q vt_q μ_q
+    row(A.xv, Yv);
+    row(A.mu, Yu);
+#pragma unroll
+    for (int s2 = 0; s2 < QH; ++s2) db = fma(B.wh[s2], Y[s2] * Yv[s2] * Yu[s2], db);
+    db = team_sum<QH>(B.wh[u] * db, u, lane0, mask);
     if (u == 0) A.gbe[e] += 2.0 * db;
   }
-  double acc[J];
+  double mu[J];
+  int hx = 0, hg = 0;
+#pragma unroll
+  for (int s2 = 0; s2 < QH; ++s2) {
+    Y[s2] *= F.beta2[(u + QH * s2) * Eu + e];
+    hg = max(hg, fx_abs_hi(Y[s2]));
+  }
 #pragma unroll
   for (int j = 0; j < J; ++j) {
-    const int k = u + U * j;
-    acc[j] = 0.0;
-    if (k < NE) {
-      xs[k] = A.mu[e + Eu * k];
-      acc[j] = A.gv[e + Eu * k];
-    }
+    const int k = u + QH * j;
+    mu[j] = k < NE ? A.mu[e + Eu * k] : 0.0;
+    hx = max(hx, fx_abs_hi(mu[j]));
   }
-  __syncwarp(tmask);
-  team_K<NU, NV, 1>(B, [&](int r, int s2) { return F.G[(r + QH * s2) * Eu + e]; }, u, tmask, Phs, PhWs, xs, zs, zd,
-                    acc);
+  hg = __reduce_max_sync(mask, hg);
+  hx = __reduce_max_sync(mask, hx);
+  const int eg = fx_exp(hg) + 1, ex = fx_exp(hx);        // the weights stay below 2^60
+#pragma unroll
+  for (int s2 = 0; s2 < QH; ++s2) Gs[u + QH * s2] = fx_split(fx_from(Y[s2], eg));
 #pragma unroll
   for (int j = 0; j < J; ++j) {
-    const int k = u + U * j;
-    if (k < NE) A.gv[e + Eu * k] = acc[j];
+    const int k = u + QH * j;
+    if (k < NE) xf[k] = fx_split(fx_from(mu[j], ex));
   }
+  __syncwarp(mask);
+  const double nan = __longlong_as_double(0x7ff8000000000000LL);
+  const int k2 = (ex - FX_BIAS) + (eg - FX_BIAS) + 64;   // in two factors: the exponents may add up to a subnormal
+  const double s1 = fx_finite(hg) && fx_finite(hx) ? ldexp(1.0, k2 / 2) : nan, s2 = ldexp(1.0, k2 - k2 / 2);
+  team_K_fx<NU, NV>(B, Gs, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs), [&](int j, int k, i64 y) {
+    if (k < NE) A.gv[e + Eu * k] = fma((double)y * s1, s2, A.gv[e + Eu * k]);
+  });
 }
 
 template <int NU, int NV>
-__global__ void __launch_bounds__(CHEB_THREADS, 3)
+__global__ void __launch_bounds__(CHEB_THREADS, 5)
     k_adj_mass(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ Fields F, const AdjIO A) {
-  adj_mass_body<NU, NV>(B, F, A, blockIdx.x * team_tile<NU, NV>());
+  adj_mass_body<NU, NV>(B, F, A, blockIdx.x * mass_tile(NU, NV, CHEB_THREADS));
 }
 
-// tile = team_tile elements per virtual block
+// tile = mass_tile(NU, NV, CHEB_THREADS) elements per virtual block
 template <int NU, int NV>
-__global__ void __launch_bounds__(CHEB_THREADS, 3)
+__global__ void __launch_bounds__(CHEB_THREADS, 5)
     k_adj_mass_m(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ MultiAdj P) {
   for (int vb = blockIdx.x; vb < P.first[P.n]; vb += gridDim.x) {
     const int inst = multi_begin(P, vb);
@@ -329,63 +396,58 @@ __device__ __forceinline__ void boundary_coef_partials(const Fields &F, int s, c
 //                      enters the own slots (the neighbour adds its own); on a physical side
 //                      c², α, c = √c², β enter the own slots.
 //
-// The points of a side come in mirrored pairs (i, NQ-1-i): the sums over the points are taken
-// from their sums (even modes) and differences (odd modes), and the transposes of the two
-// opposite sides (B and T, L and R) are applied together (Er = ±El, E1r = ∓E1l by mode parity).
+// The transposes of the two opposite sides (B and T, L and R) are applied together (Er = ±El, E1r = ∓E1l
+// by mode parity): those of B and T on the thread's column, those of L and R on its row.
+//
+// What bounds it: the FP64 pipe, at 12 NU operations a thread for the sums over the points, and the points'
+// own (25, with PARAMS 50, a side): 56 % of the pipe over the launch, 78 % while blocks are there (683 blocks are
+// 4.5 an SM at N = 128). N = 128, q = 4, with PARAMS, cold caches: 188 us with a thread per element, 128 us so.
 template <int NU, int NV, bool PARAMS>
 __device__ __forceinline__ void adj_face_body(const Basis<NU, NV> &B, const Fields &F, const StageIO &S,
-                                              const AdjIO &A, double *gc2, double *gal, double *gbe, int e) {
+                                              const AdjIO &A, double *gc2, double *gal, double *gbe, int e0) {
   constexpr int NQ = NU;
-  const int E = F.E, N = F.N;
-  if (e >= E) return;
-  if (err_word(F) != ERR_NONE) return;
-  const int j = e % N, k = e / N;
-  const size_t Eu = (size_t)E;
+  WEDG_ADJ_TEAM(e0)
+  const int N = F.N, j = e % N, k = e / N;
+  const bool has_v = r < NV;
   const TimeF tf = time_factors(S);
   double dc2 = 0.0, dal = 0.0, dbe = 0.0;
   if constexpr (PARAMS) {
-    // ---- volume and u-solve: ν and μ (padded to NU × NU) in registers, U, V, ut streamed
-    double Nl[NU][NU], Ml[NU][NU];
+    // ---- volume and u-solve: column r of A1 and A2 from ν and μ (padded to NU × NU)
+    double nc[NU], mc[NU], kr[(NU + 1) / 2];
+    const int o = r & 1;                                 // K1[a][c] = 0 for a + c odd
 #pragma unroll
-    for (int b = 0; b < NU; ++b)
+    for (int a = 0; a < NU; ++a) {
+      nc[a] = A.nu[e + Eu * (a + NU * r)];
+      mc[a] = has_v && a < NV ? A.mu[e + Eu * (a + NV * r)] : 0.0;
+      s[a * NU + r] = nc[a];
+      s[NU * NU + a * NU + r] = mc[a];
+    }
 #pragma unroll
-      for (int a = 0; a < NU; ++a) {
-        Nl[a][b] = A.nu[e + Eu * (a + NU * b)];
-        Ml[a][b] = (a < NV && b < NV) ? A.mu[e + Eu * (a + NV * b)] : 0.0;
+    for (int i = 0; i < (NU + 1) / 2; ++i) kr[i] = o + 2 * i < NU ? B.K1[o + 2 * i][r] : 0.0;
+    __syncwarp(mask);
+#pragma unroll
+    for (int a = 0; a < NU; ++a) {
+      double a1 = 0.0, a2 = 0.0;
+#pragma unroll
+      for (int c = a & 1; c < NU; c += 2) {
+        a1 = fma(B.K1[a][c], nc[c], a1);
+        a2 = fma(B.K1[a][c], mc[c], a2);
       }
 #pragma unroll
-    for (int b = 0; b < NU; ++b)
-#pragma unroll
-      for (int a = 0; a < NU; ++a) {
-        double a1 = 0.0, a2 = 0.0;
-#pragma unroll
-        for (int c = a & 1; c < NU; c += 2) {             // K1[a][c] = 0 for a + c odd
-          a1 = fma(B.K1[a][c], Nl[c][b], a1);
-          a2 = fma(B.K1[a][c], Ml[c][b], a2);
-        }
-#pragma unroll
-        for (int c = b & 1; c < NU; c += 2) {
-          a1 = fma(Nl[a][c], B.K1[c][b], a1);
-          a2 = fma(Ml[a][c], B.K1[c][b], a2);
-        }
-        const size_t l = e + Eu * (a + NU * b);
-        const double V = (a < NV && b < NV) ? S.xv[e + Eu * (a + NV * b)] : 0.0;
-        dc2 = fma(a1, V - S.ut[l], fma(-F.four_hh * a2, S.xu[l], dc2));
-        dal = fma(-F.four_hh * a2, V, dal);
+      for (int i = 0; i < (NU + 1) / 2; ++i) {
+        const int c = o + 2 * i < NU ? o + 2 * i : 0;
+        a1 = fma(kr[i], s[a * NU + c], a1);
+        a2 = fma(kr[i], s[NU * NU + a * NU + c], a2);
       }
+      const size_t l = e + Eu * (a + NU * r);
+      const double V = has_v && a < NV ? S.xv[e + Eu * (a + NV * r)] : 0.0;
+      dc2 = fma(a1, V - S.ut[l], fma(-F.four_hh * a2, S.xu[l], dc2));
+      dal = fma(-F.four_hh * a2, V, dal);
+    }
+    __syncwarp(mask);
   }
-  double gU[NU][NU], gV[NV][NV];
-#pragma unroll
-  for (int b = 0; b < NU; ++b)
-#pragma unroll
-    for (int a = 0; a < NU; ++a) gU[a][b] = -F.four_hh * A.gu[e + Eu * (a + NU * b)];
-#pragma unroll
-  for (int b = 0; b < NV; ++b)
-#pragma unroll
-    for (int a = 0; a < NV; ++a) gV[a][b] = A.gv[e + Eu * (a + NV * b)];
-  gV[0][0] += A.nu[e];                                  // b[0][0] += V[0][0] transposed
   const double *tr = F.tr;
-  auto T = [&](int fam, int side, int i, int el) { return tr[((fam * 4 + side) * NQ + i) * Eu + el]; };
+  auto tv_at = [&](int fam, int side, int i, int el) { return tr[((fam * 4 + side) * NQ + i) * Eu + el]; };
   auto hat = [&](int fam, int side, int i, int el) { return A.hat[((fam * 4 + side) * NQ + i) * Eu + el]; };
   // t̂ (du, v, dv) at point i of side s, and the point's parameter terms
   auto point = [&](int s, bool boundary, int i, double (&t)[3]) {
@@ -431,136 +493,120 @@ __device__ __forceinline__ void adj_face_body(const Basis<NU, NV> &B, const Fiel
     if constexpr (PARAMS) {
       const int sm = s < 2 ? 1 : 3, spp = s < 2 ? 0 : 2;
       const int em = plus ? nb : e, ep = plus ? e : nb;
-      const double vm = T(1, sm, i, em), vp = T(1, spp, i, ep);
-      const double dum = T(0, sm, i, em), dup = T(0, spp, i, ep);
-      const double dvm = T(2, sm, i, em), dvp = T(2, spp, i, ep);
-      // the weights of both roles on one-sided faces, of the own role on continuous ones
-      const FaceWeights wp = os ? w : plus ? face_weights(F, cf, ho0, ho1, ho2, 0.0, 0.0, 0.0)
-                                           : face_weights(F, cf, 0.0, 0.0, 0.0, ho0, ho1, ho2);
-      const double hP1 = plus ? ho1 : os ? hn1 : 0.0, hP2 = plus ? ho2 : os ? hn2 : 0.0;
-      const double hM1 = plus ? (os ? hn1 : 0.0) : ho1, hM2 = plus ? (os ? hn2 : 0.0) : ho2;
-      // which sides' coefficients are the element's: its own side (one-sided), both (continuous)
-      const double dp = (!os || plus) ? 1.0 : 0.0, dm = (!os || !plus) ? 1.0 : 0.0;
-      const double tau = F.tau;
+      const double vm = tv_at(1, sm, i, em), vp = tv_at(1, spp, i, ep);
+      const double dum = tv_at(0, sm, i, em), dup = tv_at(0, spp, i, ep);
+      const double dvm = tv_at(2, sm, i, em), dvp = tv_at(2, spp, i, ep);
+      const double sj = vm - vp, tau = F.tau;
+      if (!os) {
+        // own slots alone, c² and α of the face: plus or minus role by the sign of the weights
+        const double x = a * (dum - dup), y = a * (dvm - dvp), dJ = tau * (cf.c2p * x + cf.afp * y);
+        const double h0 = plus ? ho0 : -ho0, wo = cf.c2p * ho2 - cf.afp * ho1, ws = plus ? tau * wo : -tau * wo;
+        const double dv = plus ? th * sj - dJ : (1.0 - th) * sj + dJ;
+        dc2 += (F.lu * sj - (a * dum - th * x)) * h0 - x * ws + dv * ho2;
+        dal += (F.lv * sj - (a * dvm - th * y)) * h0 - y * ws - dv * ho1;
+        return;
+      }
+      // one-sided: the element's own side's coefficients enter its slots and the neighbour's
+      const double hP1 = plus ? ho1 : hn1, hP2 = plus ? ho2 : hn2, hM1 = plus ? hn1 : ho1, hM2 = plus ? hn2 : ho2;
+      const double dp = plus ? 1.0 : 0.0, dm = plus ? 0.0 : 1.0;
       const double J = a * (cf.c2m * dum - cf.c2p * dup + cf.afm * dvm - cf.afp * dvp) + cf.K;
-      const double sj = vm - vp;
       const double dvsp = th * sj - tau * J, dvsm = -(1.0 - th) * sj - tau * J;
       {
         const double dJ = a * (dm * dum - dp * dup), dG = a * ((1.0 - th) * dm * dum + th * dp * dup);
-        const double dpen = 0.5 * (dm + dp) * F.lu;
-        dc2 += (dpen * sj - dG) * wp.wA - dJ * wp.wS + dp * dvsp * hP2 - dm * dvsm * hM2;
+        dc2 += (0.5 * F.lu * sj - dG) * w.wA - dJ * w.wS + dp * dvsp * hP2 - dm * dvsm * hM2;
       }
       {
         const double dJ = a * (dm * dvm - dp * dvp), dG = a * ((1.0 - th) * dm * dvm + th * dp * dvp);
-        const double dpen = 0.5 * (dm + dp) * F.lv;
-        dal += (dpen * sj - dG) * wp.wA - dJ * wp.wS - dp * dvsp * hP1 + dm * dvsm * hM1;
+        dal += (0.5 * F.lv * sj - dG) * w.wA - dJ * w.wS - dp * dvsp * hP1 + dm * dvsm * hM1;
       }
     }
   };
-  // sides in groups of NS: opposite sides together (B and T, then L and R) while the registers
-  // allow, else one at a time
-  constexpr int NS = NU <= 5 ? 2 : 1;
+  // the thread's point of the four sides, s[(x 4 + side) NU + r]
 #pragma unroll 1
-  for (int g0 = 0; g0 < 4; g0 += NS) {
-    double qu[NS][NU], qv[NS][NV], qd[NS][NV];          // Σ_i P[i][b] t̂(s, i) per side and family
+  for (int sd = 0; sd < 4; ++sd) {
+    const bool boundary = (sd == 0 && j == 0) || (sd == 1 && j == N - 1) || (sd == 2 && k == 0) || (sd == 3 && k == N - 1);
+    double t[3];
+    point(sd, boundary, r, t);
 #pragma unroll
-    for (int h = 0; h < NS; ++h) {
-      const int s = g0 + h;
-      const bool boundary = (s == 0 && j == 0) || (s == 1 && j == N - 1) || (s == 2 && k == 0) || (s == 3 && k == N - 1);
-#pragma unroll
-      for (int b = 0; b < NU; ++b) {
-        qu[h][b] = 0.0;
-        if (b < NV) { qv[h][b] = 0.0; qd[h][b] = 0.0; }
-      }
-#pragma unroll 1
-      for (int i = 0; i < (NQ + 1) / 2; ++i) {
-        double t1[3], t2[3];
-        point(s, boundary, i, t1);
-        const bool mid = 2 * i + 1 == NQ;               // the middle point: the odd modes vanish
-        if (!mid) point(s, boundary, NQ - 1 - i, t2);
-#pragma unroll
-        for (int b = 0; b < NU; ++b) {
-          const double p = B.P[i][b];
-          const bool odd = b & 1;
-          if (mid && odd) continue;
-          const double su = mid ? t1[0] : odd ? t1[0] - t2[0] : t1[0] + t2[0];
-          qu[h][b] = fma(p, su, qu[h][b]);
-          if (b < NV) {
-            const double sv = mid ? t1[1] : odd ? t1[1] - t2[1] : t1[1] + t2[1];
-            const double sd = mid ? t1[2] : odd ? t1[2] - t2[2] : t1[2] + t2[2];
-            qv[h][b] = fma(p, sv, qv[h][b]);
-            qd[h][b] = fma(p, sd, qd[h][b]);
-          }
-        }
-      }
-    }
-    // trace transposes: B/T contract the first index with the end values, L/R the second; the
-    // far side's end vectors are Er[a] = (-1)^a El[a], E1r[a] = -(-1)^a E1l[a]
-    const bool tb = g0 < 2;
-    const bool right = NS == 1 && (g0 & 1);
-#pragma unroll
-    for (int a = 0; a < NU; ++a) {
-      const bool odd = a & 1;
-      const double e1 = B.E1l[a], e0 = B.El[a];
-#pragma unroll
-      for (int b = 0; b < NU; ++b) {
-        double cu, cv = 0.0, cd = 0.0;
-        if constexpr (NS == 2) {
-          cu = odd ? qu[0][b] + qu[1][b] : qu[0][b] - qu[1][b];
-          if (b < NV) {
-            cv = odd ? qv[0][b] - qv[1][b] : qv[0][b] + qv[1][b];
-            cd = odd ? qd[0][b] + qd[1][b] : qd[0][b] - qd[1][b];
-          }
-        } else {
-          const double s1 = right ? (odd ? 1.0 : -1.0) : 1.0, s0 = right ? (odd ? -1.0 : 1.0) : 1.0;
-          cu = s1 * qu[0][b];
-          if (b < NV) {
-            cv = s0 * qv[0][b];
-            cd = s1 * qd[0][b];
-          }
-        }
-        if (tb) gU[a][b] = fma(e1, cu, gU[a][b]);
-        else gU[b][a] = fma(e1, cu, gU[b][a]);
-        if (a < NV && b < NV) {
-          if (tb) gV[a][b] = fma(e0, cv, fma(e1, cd, gV[a][b]));
-          else gV[b][a] = fma(e0, cv, fma(e1, cd, gV[b][a]));
-        }
-      }
-    }
+    for (int x = 0; x < 3; ++x) s[(x * 4 + sd) * NU + r] = t[x];
   }
+  __syncwarp(mask);
+  double pc[NQ];                                         // P's column of mode r
 #pragma unroll
-  for (int b = 0; b < NU; ++b)
+  for (int i = 0; i < NQ; ++i) pc[i] = B.P[i][r];
+  // the sums over the points of an axis' two sides, and their combinations for even and odd modes: c[x][parity]
+  double c[3][2];
+  auto combos = [&](int ax) {
 #pragma unroll
-    for (int a = 0; a < NU; ++a) A.gu[e + Eu * (a + NU * b)] = gU[a][b];
+    for (int x = 0; x < 3; ++x) {
+      double lo = 0.0, hi = 0.0;
 #pragma unroll
-  for (int b = 0; b < NV; ++b)
+      for (int i = 0; i < NQ; ++i) {
+        lo = fma(pc[i], s[(x * 4 + 2 * ax) * NU + i], lo);
+        hi = fma(pc[i], s[(x * 4 + 2 * ax + 1) * NU + i], hi);
+      }
+      c[x][0] = x == 1 ? lo + hi : lo - hi;              // Er = ±El; E1r = ∓E1l
+      c[x][1] = x == 1 ? lo - hi : lo + hi;
+    }
+  };
+  double gU[NU], gV[NV], rU[NU], rV[NV];
+  combos(1);
 #pragma unroll
-    for (int a = 0; a < NV; ++a) A.gv[e + Eu * (a + NV * b)] = gV[a][b];
+  for (int a = 0; a < NU; ++a) rU[a] = B.E1l[a] * c[0][a & 1];
+#pragma unroll
+  for (int a = 0; a < NV; ++a) rV[a] = fma(B.El[a], c[1][a & 1], B.E1l[a] * c[2][a & 1]);
+  combos(0);
+#pragma unroll
+  for (int a = 0; a < NU; ++a) gU[a] = fma(B.E1l[a], c[0][a & 1], -F.four_hh * A.gu[e + Eu * (a + NU * r)]);
+#pragma unroll
+  for (int a = 0; a < NV; ++a)
+    gV[a] = has_v ? fma(B.El[a], c[1][a & 1], fma(B.E1l[a], c[2][a & 1], A.gv[e + Eu * (a + NV * r)])) : 0.0;
+  if (r == 0) gV[0] += A.nu[e];                          // b[0][0] += V[0][0] transposed
+  __syncwarp(mask);
+#pragma unroll
+  for (int b = 0; b < NU; ++b) s[r * NU + b] = rU[b];
+#pragma unroll
+  for (int b = 0; b < NV; ++b) s[NU * NU + r * NU + b] = rV[b];
+  __syncwarp(mask);
+#pragma unroll
+  for (int a = 0; a < NU; ++a) A.gu[e + Eu * (a + NU * r)] = gU[a] + s[a * NU + r];
+#pragma unroll
+  for (int a = 0; a < NV; ++a)
+    if (has_v) A.gv[e + Eu * (a + NV * r)] = gV[a] + s[NU * NU + a * NU + r];
   if constexpr (PARAMS) {
-    gc2[e] += dc2;
-    gal[e] += dal;
-    gbe[e] += dbe;
+    dc2 = team_sum<NU>(dc2, r, lane0, mask);
+    dal = team_sum<NU>(dal, r, lane0, mask);
+    dbe = team_sum<NU>(dbe, r, lane0, mask);
+    if (r == 0) {
+      gc2[e] += dc2;
+      gal[e] += dal;
+      gbe[e] += dbe;
+    }
   }
 }
 
 template <int NU, int NV, bool PARAMS>
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_face(const __grid_constant__ Basis<NU, NV> B,
+__global__ void __launch_bounds__(ADJ_THREADS, PARAMS ? 5 : 6) k_adj_face(const __grid_constant__ Basis<NU, NV> B,
                                                    const __grid_constant__ Fields F,
                                                    const __grid_constant__ StageIO S, const AdjIO A, double *gc2,
                                                    double *gal, double *gbe) {
-  adj_face_body<NU, NV, PARAMS>(B, F, S, A, gc2, gal, gbe, blockIdx.x * blockDim.x + threadIdx.x);
+  adj_face_body<NU, NV, PARAMS>(B, F, S, A, gc2, gal, gbe, blockIdx.x * adj_tile(NU));
 }
 
-// tile = ADJ_THREADS elements per virtual block
+// tile = adj_tile(NU) elements per virtual block
 template <int NU, int NV, bool PARAMS>
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_face_m(const __grid_constant__ Basis<NU, NV> B,
+__global__ void __launch_bounds__(ADJ_THREADS, PARAMS ? 5 : 6) k_adj_face_m(const __grid_constant__ Basis<NU, NV> B,
                                                      const __grid_constant__ MultiAdj P) {
   for (int vb = blockIdx.x; vb < P.first[P.n]; vb += gridDim.x) {
     const int inst = multi_begin(P, vb);
     const AdjArgs &a = P.a[inst];
-    adj_face_body<NU, NV, PARAMS>(B, a.F, a.S, a.A, a.gc2, a.gal, a.gbe,
-                                  (vb - P.first[inst]) * P.tile + (int)threadIdx.x);
+    adj_face_body<NU, NV, PARAMS>(B, a.F, a.S, a.A, a.gc2, a.gal, a.gbe, (vb - P.first[inst]) * P.tile);
   }
 }
+
+#undef WEDG_ADJ_TEAM
+#undef WEDG_MASS_TABLES
+#undef WEDG_MASS_BINS
+#undef WEDG_MASS_TEAM
 
 }  // namespace wedg

@@ -710,8 +710,7 @@ cudaError_t multi_stage_launch(const Launchers &L, const void *basis, int nu, in
 enum { MA_HATS = 0, MA_MASS = 1, MA_FACE = 2 };
 cudaError_t multi_adj_launch(const Launchers &L, const void *basis, int nu, int nv, int kind,
                              const std::vector<AdjArgs> &args, cudaStream_t st) {
-  const int TPW = 32 / (qhigh(nu, nv) / 2 + (qhigh(nu, nv) & 1));
-  const int tile = kind == MA_MASS ? (CHEB_THREADS / 32) * TPW : ADJ_THREADS;
+  const int tile = kind == MA_MASS ? mass_tile(nu, nv, CHEB_THREADS) : kind == MA_HATS ? HATS_THREADS : adj_tile(nu);
   const int n = (int)args.size();
   for (int c0 = 0; c0 < n; c0 += MultiAdj::cap) {
     const int m = std::min(n - c0, MultiAdj::cap);

@@ -206,15 +206,15 @@ cudaError_t launch_mass(const void *basis, const Fields &F, const StageIO &S, in
   return cudaSuccess;
 }
 
-// The adjoint kernels (wedg_adjoint.cuh): element grids of 128 threads, the mass term on the team grid
+// The adjoint kernels (wedg_adjoint.cuh)
 template <int NU, int NV>
 void launch_adj_hats(const void *basis, const Fields &F, const StageIO &, const AdjIO &A, cudaStream_t st) {
-  k_adj_hats<NU, NV><<<(F.E + ADJ_THREADS - 1) / ADJ_THREADS, ADJ_THREADS, 0, st>>>(
+  k_adj_hats<NU, NV><<<(F.E + HATS_THREADS - 1) / HATS_THREADS, HATS_THREADS, 0, st>>>(
       *static_cast<const Basis<NU, NV> *>(basis), F, A);
 }
 template <int NU, int NV>
 void launch_adj_mass(const void *basis, const Fields &F, const StageIO &, const AdjIO &A, cudaStream_t st) {
-  constexpr int tpb = ChebTeam<NU, NV>::TPB;
+  constexpr int tpb = mass_tile(NU, NV, CHEB_THREADS);
   k_adj_mass<NU, NV><<<(F.E + tpb - 1) / tpb, CHEB_THREADS, 0, st>>>(*static_cast<const Basis<NU, NV> *>(basis), F,
                                                                      A);
 }
@@ -222,7 +222,7 @@ template <int NU, int NV>
 void launch_adj_face(const void *basis, const Fields &F, const StageIO &S, const AdjIO &A, double *gc2, double *gal,
                      double *gbe, cudaStream_t st) {
   const Basis<NU, NV> &B = *static_cast<const Basis<NU, NV> *>(basis);
-  const int grid = (F.E + ADJ_THREADS - 1) / ADJ_THREADS;
+  const int grid = (F.E + adj_tile(NU) - 1) / adj_tile(NU);
   if (gc2) k_adj_face<NU, NV, true><<<grid, ADJ_THREADS, 0, st>>>(B, F, S, A, gc2, gal, gbe);
   else k_adj_face<NU, NV, false><<<grid, ADJ_THREADS, 0, st>>>(B, F, S, A, nullptr, nullptr, nullptr);
 }
@@ -266,7 +266,7 @@ template <int NU, int NV>
 cudaError_t launch_adj_hats_m(const void *basis, const MultiAdj &P, int grid, cudaStream_t st) {
   const int total = P.first[P.n];
   if (total <= 0) return cudaSuccess;
-  k_adj_hats_m<NU, NV><<<multi_grid(grid, total), ADJ_THREADS, 0, st>>>(*static_cast<const Basis<NU, NV> *>(basis),
+  k_adj_hats_m<NU, NV><<<multi_grid(grid, total), HATS_THREADS, 0, st>>>(*static_cast<const Basis<NU, NV> *>(basis),
                                                                          P);
   return cudaSuccess;
 }

@@ -213,9 +213,8 @@ __device__ __forceinline__ int multi_begin(const Multi<Args, CAP> &P, int vb) {
 // points (mirrored through the element centre) and the basis is the Legendre one,
 // so P[n-1-i][d] = (-1)^d P[i][d] for the values and the opposite sign for the
 // derivatives (the host makes these exact). A contraction over the modes is then
-// done on the first half of the points only -- its even-mode and odd-mode parts give
-// the point and its mirror as a sum and a difference -- and a contraction over the
-// points from the sums (even modes) and differences (odd modes) of mirrored points.
+// done on the first half of the points only: its even-mode and odd-mode parts give
+// the point and its mirror as a sum and a difference.
 // ----------------------------------------------------------------------------
 
 // Y[s] = Σ_b T[b] Ph[s][b] at all QH points
@@ -239,56 +238,6 @@ __device__ __forceinline__ void ph_to_points(const double (&Ph)[QH][NV], const d
   }
 }
 
-// Z[b] = Σ_s Y[s] Ph[s][b]
-template <int QH, int NV>
-__device__ __forceinline__ void ph_from_points(const double (&Ph)[QH][NV], const double (&Y)[QH], double (&Z)[NV]) {
-  double ys[QH / 2 + 1], yd[QH / 2 + 1];
-#pragma unroll
-  for (int s = 0; s < QH / 2; ++s) {
-    ys[s] = Y[s] + Y[QH - 1 - s];
-    yd[s] = Y[s] - Y[QH - 1 - s];
-  }
-#pragma unroll
-  for (int b = 0; b < NV; ++b) {
-    double z = 0.0;
-#pragma unroll
-    for (int s = 0; s < QH / 2; ++s) z = fma((b & 1) ? yd[s] : ys[s], Ph[s][b], z);
-    if constexpr ((QH & 1) != 0) {
-      if (!(b & 1)) z = fma(Y[QH / 2], Ph[QH / 2][b], z);
-    }
-    Z[b] = z;
-  }
-}
-
-// Rows r and QH-1-r (r < QH/2) of Ph X for an NV×NV block x(a, b):
-//   Tp[b] = Σ_a Ph[r][a] x(a, b),  Tm[b] = Σ_a (-1)^a Ph[r][a] x(a, b)
-template <int QH, int NV, class X>
-__device__ __forceinline__ void ph_row_pair(const double (&Ph)[QH][NV], int r, const X &x, double (&Tp)[NV],
-                                            double (&Tm)[NV]) {
-#pragma unroll
-  for (int b = 0; b < NV; ++b) {
-    double ev = 0.0, od = 0.0;
-#pragma unroll
-    for (int a = 0; a < NV; a += 2) ev = fma(Ph[r][a], x(a, b), ev);
-#pragma unroll
-    for (int a = 1; a < NV; a += 2) od = fma(Ph[r][a], x(a, b), od);
-    Tp[b] = ev + od;
-    Tm[b] = ev - od;
-  }
-}
-
-// The middle row QH/2 of Ph X when QH is odd (only the even modes are nonzero there)
-template <int QH, int NV, class X>
-__device__ __forceinline__ void ph_row_mid(const double (&Ph)[QH][NV], const X &x, double (&T)[NV]) {
-#pragma unroll
-  for (int b = 0; b < NV; ++b) {
-    double ev = 0.0;
-#pragma unroll
-    for (int a = 0; a < NV; a += 2) ev = fma(Ph[QH / 2][a], x(a, b), ev);
-    T[b] = ev;
-  }
-}
-
 // ----------------------------------------------------------------------------
 // k_prep: traces, boundary weight check, Chebyshev interval data
 // ----------------------------------------------------------------------------
@@ -306,60 +255,6 @@ struct GPack {
   __device__ i64 word() const { return (i64)sG << 32 | (unsigned)ng; }
 };
 
-// Traces of an n×n block X on the four sides (src/rhs.jl:388-410):
-//   oB[i] = Σ_b P[i,b] Σ_a El[a] X[a][b],  oT with Er,
-//   oL[i] = Σ_b P[i,b] Σ_a El[a] X[b][a],  oR with Er,
-// where El, Er are the values (DER false) or the derivatives (DER true) of the modes at the
-// two ends: Er[a] = ±(-1)^a El[a], so both ends come from the even and odd parts of one sum.
-// The bottom/top pair (AXIS 0) and the left/right pair (AXIS 1) are separate passes, so that
-// only one pair's end sums are live at a time. With SCALE, every output is multiplied by sc.
-template <int NQ, int NU, int n, bool DER, int AXIS, bool SCALE>
-__device__ __forceinline__ void trace2(const double (&X)[n][n], const double (&P)[NQ][NU], const double *El,
-                                       double *tr, int fam, int E, int e, double sc, bool modal) {
-  double sA[n], sZ[n];   // the end sums at the low (B or L) and the high (T or R) end
-#pragma unroll
-  for (int b = 0; b < n; ++b) {
-    double xe = 0, xo = 0;
-#pragma unroll
-    for (int a = 0; a < n; a += 2) xe = fma(El[a], AXIS == 0 ? X[a][b] : X[b][a], xe);
-#pragma unroll
-    for (int a = 1; a < n; a += 2) xo = fma(El[a], AXIS == 0 ? X[a][b] : X[b][a], xo);
-    sA[b] = xe + xo;
-    sZ[b] = DER ? xo - xe : xe - xo;
-  }
-  auto put = [&](int i, double oA, double oZ) {
-    if constexpr (SCALE) { oA *= sc; oZ *= sc; }
-    tr[((fam * 4 + 2 * AXIS) * NQ + i) * (size_t)E + e] = oA;
-    tr[((fam * 4 + 2 * AXIS + 1) * NQ + i) * (size_t)E + e] = oZ;
-  };
-  if (modal) {            // the end sums themselves, mode b in the slot of point b
-#pragma unroll
-    for (int b = 0; b < n; ++b) put(b, sA[b], sZ[b]);
-    return;
-  }
-#pragma unroll
-  for (int i = 0; i < (NQ + 1) / 2; ++i) {
-    double eA = 0, eZ = 0, oA = 0, oZ = 0;
-#pragma unroll
-    for (int b = 0; b < n; b += 2) { eA = fma(P[i][b], sA[b], eA); eZ = fma(P[i][b], sZ[b], eZ); }
-    if (2 * i + 1 == NQ) {      // the middle point: the odd modes vanish there
-      put(i, eA, eZ);
-      continue;
-    }
-#pragma unroll
-    for (int b = 1; b < n; b += 2) { oA = fma(P[i][b], sA[b], oA); oZ = fma(P[i][b], sZ[b], oZ); }
-    put(i, eA + oA, eZ + oZ);
-    put(NQ - 1 - i, eA - oA, eZ - oZ);
-  }
-}
-
-template <int NQ, int NU, int n, bool DER, bool SCALE = false>
-__device__ __forceinline__ void trace4(const double (&X)[n][n], const double (&P)[NQ][NU], const double *El,
-                                       double *tr, int fam, int E, int e, double sc = 1.0, bool modal = false) {
-  trace2<NQ, NU, n, DER, 0, SCALE>(X, P, El, tr, fam, E, e, sc, modal);
-  trace2<NQ, NU, n, DER, 1, SCALE>(X, P, El, tr, fam, E, e, sc, modal);
-}
-
 // The value at face point i of side `side` of trace family fam of element e held as modal end sums
 // (Fields::modal): Σ_b P[i][b] t[b] over the family's n modes
 template <int NQ, int NU, int n>
@@ -369,14 +264,6 @@ __device__ __forceinline__ double modal_at(const double (&P)[NQ][NU], const doub
 #pragma unroll
   for (int b = 0; b < n; ++b) x = fma(P[i][b], tr[((fam * 4 + side) * NQ + b) * E + e], x);
   return x;
-}
-
-template <int n>
-__device__ __forceinline__ void load_regs(double (&X)[n][n], const double *x, int E, int e) {
-#pragma unroll
-  for (int b = 0; b < n; ++b)
-#pragma unroll
-    for (int a = 0; a < n; ++a) X[a][b] = x[e + (size_t)E * (a + n * b)];
 }
 
 // ----------------------------------------------------------------------------
@@ -896,111 +783,6 @@ __device__ __forceinline__ void store_v(const StageIO &S, size_t l, double kk, b
   }
 }
 
-// The mass solves run on a team of threads per element. One step of either solver costs one
-// application of K = P_h^T diag(G W) P_h (G = 2βv at the high-order points, W = w_h w_h^T their
-// weights, folded into PhW) to a vector of NV² modal entries, and its FP64 work is cut across
-// the team by rows of the point grid: unit u of the team takes the mirrored rows u and QH-1-u
-// (the middle row alone when QH is odd), takes them to the points and back (phase 1), and leaves
-// for each mode column b the sum and the difference of the two rows' results in shared memory;
-// then every thread finishes J of the NV² modal entries from the units' rows (phase 2), for
-// which it also keeps the solver's vectors. A team lives in one warp, so its phases are ordered
-// by __syncwarp on the team's lanes. Spreading an element over the team matters because one
-// warp is tied to one SM sub-partition, whose FP64 rate is a small fraction of a lane per clock:
-// with one element per thread, the warps of the elements with the most steps ran for many times
-// the average and left the SMs idle behind them.
-template <int NU, int NV>
-struct ChebTeam {
-  static constexpr int QH = qhigh(NU, NV);
-  static constexpr int U = QH / 2 + (QH & 1);          // team size: row pairs (+ the middle row)
-  static constexpr int TPW = 32 / U;                    // teams per warp
-  static constexpr int TPB = TPW * (CHEB_THREADS / 32); // elements per block
-  static constexpr int NE = NV * NV;
-  static constexpr int J = (NE + U - 1) / U;            // modal entries per thread
-  static constexpr int SLOT = NE + 2 * U * NV;          // x, then the row sums and differences
-};
-
-// The shared setup of a team kernel: Ph and PhW in shared memory, the team of this thread, its
-// unit, its lanes. Returns false for lanes without a team.
-struct TeamPos {
-  int slot, u;
-  unsigned mask;
-};
-template <int NU, int NV>
-__device__ __forceinline__ bool team_pos(TeamPos &P) {
-  using T = ChebTeam<NU, NV>;
-  const int lane = threadIdx.x & 31, tw = lane / T::U;
-  if (tw >= T::TPW) return false;
-  P.u = lane - tw * T::U;
-  P.slot = (threadIdx.x >> 5) * T::TPW + tw;
-  P.mask = ((1u << T::U) - 1u) << (tw * T::U);
-  return true;
-}
-
-// Σ over the team's lanes of x, in the order of the units, on every lane of the team
-template <int U>
-__device__ __forceinline__ double team_sum(double x, unsigned mask) {
-  const int base = __ffs(mask) - 1;
-  double s = 0.0;
-#pragma unroll
-  for (int i = 0; i < U; ++i) s += __shfl_sync(mask, x, base + i);
-  return s;
-}
-
-// acc[j] ± (K x)[k_j] on the thread's entries k_j = u + U j (+ with SIGN = 1, - with -1), for x in
-// the team's shared slot xs (complete, after a __syncwarp). zs, zd hold the units' row results
-// until the next __syncwarp of the caller.
-// G(r, s) gives the weight at a point.
-template <int NU, int NV, int SIGN, class GAt>
-__device__ __forceinline__ void team_K(const Basis<NU, NV> &B, const GAt &G, int u, unsigned mask,
-                                       const double *Phs, const double *PhWs, const double *xs, double *zs,
-                                       double *zd, double (&acc)[ChebTeam<NU, NV>::J]) {
-  using T = ChebTeam<NU, NV>;
-  constexpr int QH = T::QH, U = T::U, NE = T::NE, J = T::J;
-  const int r1 = u, r2 = QH - 1 - u;                    // the unit's rows (r1 = r2 for the middle row)
-  auto rowZ = [&](const double (&Tv)[NV], int r, double (&Z)[NV]) {
-    double Y[QH];
-    ph_to_points<QH, NV>(B.Ph, Tv, Y);
-#pragma unroll
-    for (int s2 = 0; s2 < QH; ++s2) Y[s2] *= G(r, s2);
-    ph_from_points<QH, NV>(B.PhW, Y, Z);
-  };
-  // phase 1: rows r1, r2 of P_h x, at the points, weighted, back to the modes
-  {
-    double Tp[NV], Tm[NV], Zp[NV], Zm[NV];
-#pragma unroll
-    for (int b = 0; b < NV; ++b) {
-      double ev = 0.0, od = 0.0;
-#pragma unroll
-      for (int a = 0; a < NV; a += 2) ev = fma(Phs[r1 * NV + a], xs[a + NV * b], ev);
-#pragma unroll
-      for (int a = 1; a < NV; a += 2) od = fma(Phs[r1 * NV + a], xs[a + NV * b], od);
-      Tp[b] = ev + od;
-      Tm[b] = ev - od;
-    }
-    rowZ(Tp, r1, Zp);
-    rowZ(Tm, r2, Zm);
-#pragma unroll
-    for (int b = 0; b < NV; ++b) {
-      zs[u * NV + b] = r1 == r2 ? Zp[b] : Zp[b] + Zm[b];
-      zd[u * NV + b] = Zp[b] - Zm[b];
-    }
-  }
-  __syncwarp(mask);
-  // phase 2: the thread's entries
-#pragma unroll
-  for (int j = 0; j < J; ++j) {
-    const int k = u + U * j;
-    if (k < NE) {
-      const int a = k % NV, b = k / NV;
-      const double *z = ((a & 1) ? zd : zs) + b;
-      double x = acc[j];
-#pragma unroll
-      for (int v = 0; v < U; ++v) x = fma(SIGN * PhWs[v * NV + a], z[v * NV], x);
-      acc[j] = x;
-    }
-  }
-}
-
 // k_cheb: the Chebyshev mass solve (Saad Alg. 12.1, src/rhs.jl:920-939), a team of QH threads per
 // element: thread u takes row u of the point grid and J of the modal entries. Elements are visited in
 // decreasing order of their step counts (k_prep lists them by count), so the longest solves start
@@ -1220,18 +1002,19 @@ __device__ __forceinline__ i64 fx_recip(i64 D) {
   return r;
 }
 
-// The start of k_cheb and k_cg: the operators' tables, the elements by count (pref[b]: those in the bins
-// above b), and the thread's team, row u and slot of elements g; threads without one return
-#define WEDG_MASS_SETUP(g0) \
+// The start of the kernels on MassTeam: the operators' tables; the elements by count (pref[b]: those in the
+// bins above b); and the thread's team, row u and slot of elements g, where threads without one return
+#define WEDG_MASS_TABLES() \
   using T = MassTeam<NU, NV>; \
   constexpr int QH = T::QH, NE = T::NE, J = T::J, HP = T::HP; \
   __shared__ double sh[T::TPB * T::SLOT]; \
   __shared__ Fx2 Phf[HP * NV], PhWf[HP * NV]; \
-  __shared__ int pref[NBIN]; \
   for (int i = threadIdx.x; i < HP * NV; i += blockDim.x) { \
     Phf[i] = Fx2{B.fPh[i / NV][i % NV].h, B.fPh[i / NV][i % NV].l}; \
     PhWf[i] = Fx2{B.fPhW[i / NV][i % NV].h, B.fPhW[i / NV][i % NV].l}; \
-  } \
+  }
+#define WEDG_MASS_BINS() \
+  __shared__ int pref[NBIN]; \
   if (F.sorted && threadIdx.x < 32) { \
     int carry = 0; \
 _Pragma("unroll") \
@@ -1246,7 +1029,8 @@ _Pragma("unroll") \
       if (b >= 0) pref[b] = carry + x - own; \
       carry += __shfl_sync(~0u, x, 31); \
     } \
-  } \
+  }
+#define WEDG_MASS_TEAM(g0) \
   __syncthreads(); \
   const int lane = threadIdx.x & 31, tw = lane / QH; \
   if (tw >= T::TPW) return; \
@@ -1258,7 +1042,9 @@ _Pragma("unroll") \
 
 template <int NU, int NV>
 __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &F, const StageIO &S, int g0) {
-  WEDG_MASS_SETUP(g0);
+  WEDG_MASS_TABLES()
+  WEDG_MASS_BINS()
+  WEDG_MASS_TEAM(g0)
   const int e = mass_element(F, S, g, pref);
   double *xs = sh + slot * T::SLOT, *X = xs + NE, *zs = X + NE;
   const double th = F.th[e], de = F.de[e];
@@ -1369,14 +1155,14 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
   if (S.mode == OUT_RK4_LAST && !fin) atomicOr(F.nonfinite, 1u);
 }
 
-// Σ over the team's QH threads of x, on every one of them: the same tree for each
-template <int QH>
-__device__ __forceinline__ double mass_sum(double x, int u, int lane0, unsigned mask) {
-  constexpr int top = QH > 8 ? 8 : QH > 4 ? 4 : QH > 2 ? 2 : 1;
+// Σ over the team's W threads of x, on every one of them: the same tree for each
+template <int W>
+__device__ __forceinline__ double team_sum(double x, int u, int lane0, unsigned mask) {
+  constexpr int top = W > 8 ? 8 : W > 4 ? 4 : W > 2 ? 2 : 1;
 #pragma unroll
   for (int o = top; o > 0; o >>= 1) {
-    const double y = __shfl_sync(mask, x, lane0 + (u + o < QH ? u + o : u));
-    if (u < o && u + o < QH) x += y;
+    const double y = __shfl_sync(mask, x, lane0 + (u + o < W ? u + o : u));
+    if (u < o && u + o < W) x += y;
   }
   return __shfl_sync(mask, x, lane0);
 }
@@ -1389,7 +1175,8 @@ __device__ __forceinline__ double mass_sum(double x, int u, int lane0, unsigned 
 // of G, which k_prep writes).
 template <int NU, int NV>
 __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F, const StageIO &S, int g0) {
-  WEDG_MASS_SETUP(g0);
+  WEDG_MASS_TABLES()
+  WEDG_MASS_TEAM(g0)
   const int e = g;
   double *xs = sh + slot * T::SLOT, *zs = xs + 2 * NE;
   Fx2 *xf = reinterpret_cast<Fx2 *>(xs), *Gs = reinterpret_cast<Fx2 *>(zs + T::ZR);
@@ -1426,7 +1213,7 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
     X[j] = k < NE ? F.mrhs[k * Eu + e] : 0.0;
     r0 = fma(X[j], X[j], r0);
   }
-  r0 = sqrt(mass_sum<QH>(r0, u, lane0, mask));
+  r0 = sqrt(team_sum<QH>(r0, u, lane0, mask));
   K(X, r);                                               // r = R - M X = K R for X = R
   double rr = 0;
 #pragma unroll
@@ -1434,7 +1221,7 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
     p[j] = r[j];
     rr = fma(r[j], r[j], rr);
   }
-  rr = mass_sum<QH>(rr, u, lane0, mask);
+  rr = team_sum<QH>(rr, u, lane0, mask);
   const int maxit = NV * NV + 10;
   int it = 0;
   bool bad = false;
@@ -1447,7 +1234,7 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
       Ap[j] = __dsub_rn(p[j], Ap[j]);                    // A p = p - K p
       pAp = fma(p[j], Ap[j], pAp);
     }
-    pAp = mass_sum<QH>(pAp, u, lane0, mask);
+    pAp = team_sum<QH>(pAp, u, lane0, mask);
     if (!(pAp > 0.0)) { bad = true; break; }
     const double al = rr / pAp;
     double rrn = 0;
@@ -1457,7 +1244,7 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
       r[j] = fma(-al, Ap[j], r[j]);
       rrn = fma(r[j], r[j], rrn);
     }
-    rrn = mass_sum<QH>(rrn, u, lane0, mask);
+    rrn = team_sum<QH>(rrn, u, lane0, mask);
     const double bt = rrn / rr;
 #pragma unroll
     for (int j = 0; j < J; ++j) p[j] = fma(bt, p[j], r[j]);
@@ -1476,14 +1263,6 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
     if (k < NE) store_v(S, e + Eu * k, X[j], fin);
   }
   if (S.mode == OUT_RK4_LAST && !fin) atomicOr(F.nonfinite, 1u);
-}
-
-#undef WEDG_MASS_SETUP
-
-// The team kernels: a block of `threads` takes (threads / 32) teams per warp of elements
-template <int NU, int NV>
-__device__ __forceinline__ int team_tile() {
-  return (int)(blockDim.x >> 5) * ChebTeam<NU, NV>::TPW;
 }
 
 template <int NU, int NV>

@@ -40,6 +40,7 @@ struct AdjTeam {
 #define WEDG_ADJ_TEAM(e0) \
   using T = AdjTeam<NU>; \
   __shared__ double sh[T::TPB * T::SLOT]; \
+  after_previous(); \
   const int lane = threadIdx.x & 31, tw = lane / NU; \
   if (tw >= T::TPW) return; \
   const int r = lane - tw * NU, lane0 = tw * NU, slot = (threadIdx.x >> 5) * T::TPW + tw, e = (e0) + slot; \
@@ -160,6 +161,7 @@ template <int NU, int NV>
 __device__ __forceinline__ void adj_hats_body(const Basis<NU, NV> &B, const Fields &F, const AdjIO &A, int e) {
   constexpr int NQ = NU;
   const int E = F.E;
+  after_previous();
   if (e >= E) return;
   if (err_word(F) != ERR_NONE) return;
   const double s_nu = -1.0 / F.four_hh;

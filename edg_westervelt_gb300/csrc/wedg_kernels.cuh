@@ -185,6 +185,13 @@ struct StageArgs {
   StageIO S;
 };
 
+// Where kernels are launched early (launch_after), every thread waits here for the end of the kernel before
+// on the stream, and with it of all before that, ahead of the first read or write of memory. Without such
+// a launch it does nothing.
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 template <class Args, int CAP>
 struct Multi {
   static constexpr int cap = CAP;
@@ -404,6 +411,7 @@ __device__ __forceinline__ void bnd_body(const Basis<NU, NV> &B, const Fields &F
   constexpr int NQ = NU;
   const int N = F.N, E = F.E, lane = threadIdx.x & 31, tw = lane / NQ, i = lane - tw * NQ;
   const int x = side0 + tw;
+  after_previous();
   if (tw >= bnd_tile(NU) || x >= 4 * N) return;
   if (err_word(F) != ERR_NONE) return;
   const unsigned mask = ((1u << NQ) - 1u) << (tw * NQ);
@@ -702,6 +710,7 @@ template <int NU, int NV>
 __global__ void __launch_bounds__(128, 8) k_prep(const __grid_constant__ Basis<NU, NV> B,
                                               const __grid_constant__ Fields F,
                                               const __grid_constant__ StageIO S, int e0) {
+  after_previous();
   // elements from e0 on: a launch may cover a range of the elements (the first range clears the next
   // stage's counts)
   prep_body<NU, NV>(B, F, S, e0 + (int)blockIdx.x * prep_tile(NU, blockDim.x), blockIdx.x == 0 && e0 == 0);
@@ -1012,7 +1021,8 @@ __device__ __forceinline__ i64 fx_recip(i64 D) {
   for (int i = threadIdx.x; i < HP * NV; i += blockDim.x) { \
     Phf[i] = Fx2{B.fPh[i / NV][i % NV].h, B.fPh[i / NV][i % NV].l}; \
     PhWf[i] = Fx2{B.fPhW[i / NV][i % NV].h, B.fPhW[i / NV][i % NV].l}; \
-  }
+  } \
+  after_previous();
 #define WEDG_MASS_BINS() \
   __shared__ int pref[NBIN]; \
   if (F.sorted && threadIdx.x < 32) { \

@@ -140,6 +140,7 @@ __device__ __forceinline__ void stage_gen_body(const Basis<NU, NV> &B, const Fie
     const int i = threadIdx.x;
     ends[i] = B.El[i]; ends[NU + i] = B.E1l[i]; ends[2 * NU + i] = B.E1F[i];
   }
+  after_previous();
   __syncthreads();
   const int lane = threadIdx.x & 31, tw = lane / NU;
   if (tw >= T::TPW) return;

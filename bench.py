@@ -406,7 +406,7 @@ def run_ours(args):
     rhs_call = {"ms_per_call": t_rhs * 1e3, "value": world * dof / t_rhs, "unit": "DOF·stage/s",
                 "calls": args.steps, "cheb_steps_max": ws.stats()["cheb_steps_max"],
                 "cheb_steps_mean": ws.stats()["cheb_steps_sum"] / max(ws.stats()["element_stages"], 1),
-                "timing": "host clock around each call (wedg_rhs with device pointers: three kernels, the "
+                "timing": "host clock around each call (wedg_rhs with device pointers: four kernels, the "
                           "error word read back, synchronised); the front state after the warm-up's RK4 steps"}
     del ur, vr, utr, vtr
 
@@ -460,9 +460,9 @@ def run_ours(args):
                 "kernel": "RHS stage (k_prep + k_stage + k_cheb)", "dominant_kernel": dominant,
                 "dominant_share": kms[dominant] / stage_ms, "bytes_per_launch": bytes_stage, "launch_ms": stage_ms,
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if hbm else None,
-                "note": "the stage is bound by the FP64 pipe, not by HBM (see fp64_pipe); bytes are the "
+                "note": "the stage is bound by the FP64 and integer pipes, not by HBM (see fp64_pipe); bytes are the "
                         "reference data model's algorithmic bytes per element-stage x elements, over the time "
-                        "of one RHS stage (its three kernels); traffic is ncu's DRAM bytes of the three kernels "
+                        "of one RHS stage (its four kernels); traffic is ncu's DRAM bytes of the four kernels "
                         "per stage (profiles/stage_dram_N512_q6.txt)"}
     pipe = prof["fp64_pipe_pct"]
     fp64_pipe = None
@@ -477,7 +477,7 @@ def run_ours(args):
                      "peak_source": "cuBLAS DGEMM 4096^3 measured in this run",
                      "note": "the reference's FP64 operation count of a stage (each element's own Chebyshev "
                              "count) over the k_prep + k_stage + k_cheb time; it can exceed the DGEMM rate "
-                             "because the kernels execute fewer FP64 operations than that count (mirror "
+                             "because the kernels execute most of that count in fixed point and fewer operations (mirror "
                              "parity of the Gauss-Legendre rules, fast diagonalisation of the u-equation, "
                              "constant-coefficient volume terms)"}
 
@@ -709,7 +709,7 @@ def run_general(torch, dev, steps, warmup):
             "steps": steps, "fast_path": bool(ws.stats()["fast_path"]), "setup_s": setup_s,
             "kernel_ms": kms, "stage_alg_gbs": bytes_stage / (stage_ms / 1e3) / 1e9,
             "note": "timing covers all warm-up and timed steps' kernels; stage_alg_gbs = the reference data "
-                    "model's bytes of one stage over the three stage kernels' mean time"}
+                    "model's bytes of one stage over the stage kernels' mean time"}
 
 
 def config3_problem(precompute=None):

@@ -201,7 +201,7 @@ struct wedg_ws {
   long long *steps_done = nullptr;
   int parity = 0;   // bin-count buffer of the next stage
   // launch shapes (set by wedg_set_launch_shape or the autotuners): threads per block of k_prep
-  // (one element per thread) and of the mass solves (teams of threads per element); shape_gen
+  // and of the mass solves (teams of threads per element, so the block's warps set its elements); shape_gen
   // counts the changes, so that a captured batch graph is captured again after one
   int prep_threads = 128, mass_threads = CHEB_THREADS;
   int64_t shape_gen = 0;
@@ -401,7 +401,7 @@ void drain_events(wedg_ws *ws) {
   ws->ev_pending.clear();
 }
 
-// enqueue the three kernels of one stage (on the workspace's Fields, or on Fo); after_stage, when
+// enqueue the four kernels of one stage (on the workspace's Fields, or on Fo); after_stage, when
 // given, is recorded on the stream after the stage kernel; with prep_done the stage's k_prep has
 // been enqueued already (by ranges of elements, with this stage's bin parity)
 int enqueue_stage(wedg_ws *ws, const StageIO &S, const Fields *Fo = nullptr, cudaEvent_t after_stage = nullptr,
@@ -770,7 +770,7 @@ bool same_kernels(const wedg_ws *a, const wedg_ws *b) {
          a->basis == b->basis;
 }
 
-// One RHS evaluation (k_prep, k_stage, mass solve) of every workspace of a group, each with its
+// One RHS evaluation (k_prep, k_bnd, k_stage, mass solve) of every workspace of a group, each with its
 // own Fields and StageIO; one workspace: enqueue_stage. Advances the bin parities as enqueue_stage.
 int group_stage(const std::vector<wedg_ws *> &G, const std::vector<StageIO> &S, const std::vector<Fields> &F) {
   if (G.size() == 1) return enqueue_stage(G[0], S[0], &F[0]);

@@ -105,7 +105,7 @@ void pack_basis(const BasisHost &h, void *out) {
     for (int d = 0; d < NU; ++d) { b.P[i][d] = h.P[i][d]; b.S[i][d] = h.S[i][d]; b.Pw[i][d] = h.Pw[i][d]; }
   }
   for (int d = 0; d < NU; ++d) {
-    b.El[d] = h.El[d]; b.Er[d] = h.Er[d]; b.E1l[d] = h.E1l[d]; b.E1r[d] = h.E1r[d];
+    b.El[d] = h.El[d]; b.E1l[d] = h.E1l[d];
     b.E1F[d] = h.E1F[d];
     for (int c = 0; c < NU; ++c) { b.K1[d][c] = h.K1[d][c]; }
   }

@@ -1,31 +1,36 @@
 // Device kernels of libwedg: one RHS stage of the EDG scheme for the
-// Westervelt equation on sm_103a, FP64.
+// Westervelt equation on sm_103a, in FP64 and 64-bit fixed point.
 //
-// Design (GB300): the path is bound by the FP64 pipe (about 1.2 TFLOP/s on
-// GB300, 1/58 of FP32), not by HBM. The kernels therefore minimise FP64
-// instructions and keep all 32 lanes of a warp busy: one thread owns one
-// element, with compile-time sizes. The element's modal blocks live in shared
-// memory in a [index][thread] layout (conflict-free, and a shared load costs a
-// fraction of one 64-cycle FP64 warp instruction), small temporaries in
-// registers. Memory is spent freely where it saves arithmetic: traces and
-// Chebyshev weights are computed once per stage and re-read.
+// Design (GB300): the path is bound by arithmetic, not by HBM, and the FP64
+// pipe is slow (about 1.2 TFLOP/s on GB300, 1/58 of FP32; one operation holds
+// a scheduler's pipe for 64 cycles) while the integer pipes stand idle beside
+// it. So the contractions over modes and points, which are most of the work,
+// run in 64-bit fixed point with one exponent per element (wedg_fixed.cuh:
+// three integer multiply-adds of 4 cycles for an FP64 one, and more bits), and
+// the fluxes, sources, inner products and updates in FP64. A team of threads
+// shares an element: thread r has column or row r of its modal blocks or point
+// r of its sides, and blocks change hands through shared memory. That spreads
+// small meshes over the chip and keeps the registers low enough for 24 to 32
+// warps an SM.
 //
-// One RHS evaluation is three kernels:
+// One RHS evaluation is four kernels:
 //   k_prep   traces of the stage state on the four sides of every element
 //            (src/rhs.jl:384-410), the weight check of the boundary points
-//            (src/rhs.jl:105-110, 729-757) and the Chebyshev interval data
-//            (src/rhs.jl:889-907), so that every error of the stage is known
-//            before the second kernel starts;
-//   k_stage  face fluxes of the element's own sides (src/rhs.jl:611-700,
-//            65-103), lifts (:412-473), volume terms (:309-333), source
+//            (src/rhs.jl:105-110, 729-757), G = 2βv at the high-order points
+//            and the Chebyshev interval data (src/rhs.jl:889-907), so that every
+//            error of the stage is known before the next kernel starts;
+//   k_bnd    the flux slots of the physical sides (src/rhs.jl:65-103), projected
+//            on the face modes;
+//   k_stage  face fluxes of the element's own interior sides (src/rhs.jl:611-700),
+//            lifts (:412-473), volume terms (:309-333), source
 //            (:335-350) and u-equation (:352-382) with the u part of the RK4
 //            stage update (src/solver.jl:299-321); it leaves the right-hand
 //            side of the mass system in HBM;
 //   k_cheb   the Chebyshev mass solve (:920-939) and the v part of the RK4
-//            update, a team of threads per element. Elements are visited in
-//            decreasing order of their Chebyshev step counts (k_prep lists them
-//            by count), so the longest solves start first;
-//   k_cg     the same with conjugate gradients (:821-853), also a team per element.
+//            update. Elements are visited in decreasing order of their Chebyshev
+//            step counts (k_prep lists them by count), so the longest solves start
+//            first;
+//   k_cg     the same with conjugate gradients (:821-853).
 // Interior faces are evaluated by both neighbours, each writing only its own
 // slots, so no element writes another element's data.
 //
@@ -38,7 +43,8 @@
 //   v-faces     [j + N (kf + (N+1) i)]
 //   bnd data    [m + N i]
 //   Pi, srcP    [(a + NV b) E + e]
-//   2β, G       [(r + QH s) E + e]
+//   2β, G       [(r + QH s) E + e]                 G as integers, its exponents in rows QH² and QH² + 1
+//   bslots      [(q*4 + side) N + m]               q over the face modes of A, D, F
 //   mass rhs    [(a + NV b) E + e]
 #pragma once
 #include <cuda_runtime.h>
@@ -71,7 +77,7 @@ struct Basis {
   double w[NQ];
   double P[NQ][NU], S[NQ][NU];   // P[i][d] = P_u[i, d], S likewise; the v-basis is d < NV
   double Pw[NQ][NU];             // w[i] P[i][d]
-  double El[NU], Er[NU], E1l[NU], E1r[NU];
+  double El[NU], E1l[NU];        // the modes and their derivatives at the low end; at the high end (-1)^a El[a], -(-1)^a E1l[a]
   double E1F[NU];                // -E1l, the lift factor of the u-slots (the v-slots' factors
                                  // (2/h) El and (4/h²) E1l take the mesh size from Fields)
   double Ph[QH][NV];             // P_h_v[r, d]
@@ -101,7 +107,7 @@ struct Fields {
   const double *PiSP, *PiBSP2, *PiCdiv, *PiDdiv, *srcP;
   const double *beta2;        // 2β at the high-order points, [(r + QH s) E + e]
   // G = 2βv at the high-order points, as integers of one exponent per element, which row QH² holds with
-  // a normalising shift (GPack); k_adj_mass keeps doubles of its own there.
+  // a normalising shift (GPack).
   // Row QH² + 1: the largest high words of U and V beside the constant mode (k_stage's exponents)
   double *tr, *G, *th, *de;
   // the flux slots of the physical sides projected on the face modes: [(q 4 + s) N + m], q over the
@@ -175,9 +181,9 @@ __device__ __forceinline__ unsigned long long err_word(const Fields &F) {
 // any mesh sizes. Their arguments travel in the launch's parameter block. The launch covers
 // first[n] virtual blocks: virtual block vb belongs to the instance i with first[i] ≤ vb <
 // first[i+1] and covers `tile` elements (or element slots of the mass solves' order) of it,
-// from (vb - first[i]) tile on. Each block copies its instance's arguments into shared memory
-// and runs the single-instance kernel's body on them, so an element's arithmetic is the same
-// as in a launch of its instance alone. A grid smaller than first[n] makes the launch
+// from (vb - first[i]) tile on. Each block runs the single-instance kernel's
+// body on its instance's arguments, so an element's arithmetic is the same as in a launch of its
+// instance alone. A grid smaller than first[n] makes the launch
 // persistent: block b takes the virtual blocks b, b + gridDim.x, ...
 // ----------------------------------------------------------------------------
 struct StageArgs {
@@ -453,10 +459,11 @@ __global__ void __launch_bounds__(BND_THREADS) k_bnd_m(const __grid_constant__ B
 }
 
 // Count of Chebyshev steps for the interval θ ± δ: ceil(L / acosh(θ/δ)), from FP32 where that is not within its
-// rounding of a whole number (acosh costs some 100 FP64 operations)
+// rounding of a whole number (acosh costs some 100 FP64 operations). FP32's θ/δ is good to 2e-7, acosh of it
+// to 1e-5 from 1.01 on; closer to 1 the count is taken in FP64
 __device__ __forceinline__ int cheb_count(double L, double th, double de) {
   const float x = (float)L / acoshf((float)th / (float)de), r = rintf(x);
-  if (x < 1e6f && fabsf(x - r) > 1e-4f * x + 1e-4f) return (int)ceilf(x);
+  if (th > 1.01 * de && x < 1e6f && fabsf(x - r) > 1e-4f * x + 1e-4f) return (int)ceilf(x);
   return (int)ceil(L / acosh(th / de));
 }
 
@@ -465,6 +472,10 @@ __device__ __forceinline__ int cheb_count(double L, double th, double de) {
 // point rows r, r + NU, ... With a thread per element a warp held the chip's FP64 pipes for the
 // whole of its 378 trace operations and two blocks of state per thread; the team fills them from more
 // warps and spreads small meshes over the chip.
+//
+// What bounds it: the FP64 pipe (60 %: the traces, and a conversion per entry of V and 2β) and the latency of
+// its loads. N = 512, q = 6: 760 us as FP64 code with a thread per element; 526, 488, 458 and 442 us so at four, five,
+// six and eight blocks an SM (64 registers).
 template <int NU, int NV>
 struct PrepTeam {
   static constexpr int QH = qhigh(NU, NV), TPW = 32 / NU;
@@ -806,6 +817,9 @@ __device__ __forceinline__ void store_v(const StageIO &S, size_t l, double kk, b
 // What bounds it: one product with M costs about 1 300 multiply-adds an element at q = 6, three integer
 // ones each (4 cycles a warp), and 18 shared-memory words a thread; a thread per row keeps 24 warps an SM
 // where a thread per pair of rows (half the exchanges, 16 warps) left the pipes waiting.
+// N = 512, q = 6, a front (3.5 steps on average): 2 569 us in FP64, 1 004 us in fixed point with a thread per
+// pair of rows, 878 us so; at five and eight blocks an SM 875 and 998. N = 300, q_v = 7, 27 steps: 12 850 us
+// in FP64, 4 705 us so (4 565 and 4 908).
 template <int NU, int NV>
 struct MassTeam {
   static constexpr int QH = qhigh(NU, NV);

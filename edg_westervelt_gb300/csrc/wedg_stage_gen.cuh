@@ -7,7 +7,8 @@
 // thread per element left the chip idle below some 150 000 elements (one warp's FP64 operations are
 // a chain of 64 cycles each) and held two blocks of state per thread in shared memory; a team
 // spreads an element over NU times the warps. The teams of a warp take neighbouring elements, so
-// that a load of one entry per thread reads whole 32-byte sectors.
+// that a load of one entry per thread reads whole 32-byte sectors. N = 201, q = 6: 1 242 us with a thread per
+// element, 783 us by teams; N = 32, q = 4: 191 and 41 us.
 #pragma once
 
 namespace wedg {

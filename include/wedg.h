@@ -11,7 +11,9 @@
  * layouts and copies what the device needs.
  *
  * Conventions
- *  - All arithmetic is FP64.
+ *  - States, coefficients and results are FP64. The contractions over modes and points run in 64-bit
+ *    fixed point with one exponent per element, the rest in FP64: results are as close to 64-bit
+ *    dense algebra as FP64 sums are.
  *  - Status codes mirror the reference's exceptions (wedg_status); the exact
  *    message text of the reference is available from wedg_error_message.
  *  - State arrays u (N,N,q_u+1,q_u+1) and v (N,N,q_v+1,q_v+1) use the
@@ -211,8 +213,8 @@ int wedg_set_stream(wedg_ws *ws, void *stream);
 int wedg_rk4_steps_async(wedg_ws *ws, double *u_dev, double *v_dev, double t0, double dt, int64_t nsteps);
 int wedg_sync_status(wedg_ws *ws, int64_t *steps_done, int *finite);
 
-/* Kernel timing for benchmarks: with enable != 0, every launch of the three stage
- * kernels (k_prep, k_stage, and the mass solve k_cheb or k_cg) is bracketed by CUDA events on the workspace
+/* Kernel timing for benchmarks: with enable != 0, every launch of the stage
+ * kernels (k_prep with k_bnd, k_stage, and the mass solve k_cheb or k_cg) is bracketed by CUDA events on the workspace
  * stream and its duration accumulated; wedg_kernel_times reads (and with reset,
  * clears) the totals in milliseconds and the number of launches of each. */
 int wedg_time_kernels(wedg_ws *ws, int enable);
@@ -304,9 +306,8 @@ int wedg_rk4_adjoint_reverse_many(int n, wedg_ws *const *ws, const double *const
                                   double *const *g_beta, int where);
 
 /* Launch shapes (no counterpart in the reference, whose parallel regions are the nblocks
- * element blocks of src/rhs.jl:130-180): threads per block of k_prep (one element per thread)
- * and of the mass solves (a team of threads per element, so the block's warps set its
- * elements): 32, 64, 96 or 128 each, 128 by default. Results do not depend on them (every
+ * element blocks of src/rhs.jl:130-180): threads per block of k_prep and of the mass
+ * solves (a team of threads per element in both, so the block's warps set its elements): 32, 64, 96 or 128 each, 128 by default. Results do not depend on them (every
  * element's arithmetic is its own); only the time does. */
 int wedg_set_launch_shape(wedg_ws *ws, int prep_threads, int mass_threads);
 int wedg_get_launch_shape(const wedg_ws *ws, int *prep_threads, int *mass_threads);
@@ -335,7 +336,7 @@ int wedg_set_adjoint_memory(wedg_ws *ws, int64_t bytes);
  * any mesh sizes). A bucket runs in one of two layouts (wedg_batch_set_shape): its instances'
  * own launches, each instance on its own stream (the default, the faster on the mixed batches
  * measured), or per stage of an RK4 step k_prep, k_stage and its mass solve as one launch each
- * over all of its instances (up to 31 instances per launch; larger buckets take several), whose
+ * over all of its instances (up to 22 instances per launch; larger buckets take several), whose
  * blocks each take a tile of one instance's elements. Either way an element's arithmetic is the
  * one of a launch of its instance alone. The buckets run side by side on their own streams. One
  * RK4 step of the whole batch, and four steps in which each instance (or merged bucket) goes on
@@ -358,9 +359,8 @@ int wedg_batch_rk4_steps(wedg_batch *b, double *const *u_dev, double *const *v_d
                          const double *dt, int64_t nsteps, int stop_nonfinite, int64_t *steps_done, int *finite,
                          int *status);
 
-/* The buckets of a batch and their launch shapes: the elements per block of k_prep (its threads,
- * one element each) and of the mass solves (threads / 32 warps of teams of threads per
- * element), 32, 64, 96 or 128 threads, and `persist`: 0 launches one block per tile, p > 0 a
+/* The buckets of a batch and their launch shapes: the threads per block of k_prep and of the mass
+ * solves (threads / 32 warps of teams of threads per element), 32, 64, 96 or 128, and `persist`: 0 launches one block per tile, p > 0 a
  * persistent grid of p times the blocks the SMs hold at once, each block taking tile after
  * tile; -1 (the default) launches the bucket's instances one by one instead (the single-instance
  * kernels, each instance on its own stream). Results do not depend on the shape (every element's

@@ -406,7 +406,7 @@ def run_ours(args):
     rhs_call = {"ms_per_call": t_rhs * 1e3, "value": world * dof / t_rhs, "unit": "DOF·stage/s",
                 "calls": args.steps, "cheb_steps_max": ws.stats()["cheb_steps_max"],
                 "cheb_steps_mean": ws.stats()["cheb_steps_sum"] / max(ws.stats()["element_stages"], 1),
-                "timing": "host clock around each call (wedg_rhs with device pointers: four kernels, the "
+                "timing": "host clock around each call (wedg_rhs with device pointers: three kernels, the "
                           "error word read back, synchronised); the front state after the warm-up's RK4 steps"}
     del ur, vr, utr, vtr
 
@@ -462,7 +462,7 @@ def run_ours(args):
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if hbm else None,
                 "note": "the stage is bound by the FP64 and integer pipes, not by HBM (see fp64_pipe); bytes are the "
                         "reference data model's algorithmic bytes per element-stage x elements, over the time "
-                        "of one RHS stage (its four kernels); traffic is ncu's DRAM bytes of the four kernels "
+                        "of one RHS stage (its three kernels); traffic is ncu's DRAM bytes of the kernels "
                         "per stage (profiles/stage_dram_N512_q6.txt)"}
     pipe = prof["fp64_pipe_pct"]
     fp64_pipe = None

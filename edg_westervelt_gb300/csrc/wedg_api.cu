@@ -401,7 +401,7 @@ void drain_events(wedg_ws *ws) {
   ws->ev_pending.clear();
 }
 
-// enqueue the four kernels of one stage (on the workspace's Fields, or on Fo); after_stage, when
+// enqueue the three kernels of one stage (on the workspace's Fields, or on Fo); after_stage, when
 // given, is recorded on the stream after the stage kernel; with prep_done the stage's k_prep has
 // been enqueued already (by ranges of elements, with this stage's bin parity)
 int enqueue_stage(wedg_ws *ws, const StageIO &S, const Fields *Fo = nullptr, cudaEvent_t after_stage = nullptr,
@@ -419,7 +419,7 @@ int enqueue_stage(wedg_ws *ws, const StageIO &S, const Fields *Fo = nullptr, cud
     cudaEventRecord(e0, ws->stream);
   }
   if (!prep_done) CK(ws, ws->L.prep(ws->basis.data(), F, Sp, bp, tp, ws->stream, 0));
-  CK(ws, ws->L.bnd(ws->basis.data(), F, Sp, 1, BND_THREADS, ws->stream));
+  else CK(ws, ws->L.bnd(ws->basis.data(), F, Sp, 1, BND_THREADS, ws->stream));
   if (ws->timing) cudaEventRecord(e1, ws->stream);
   CK(ws, ws->L.stage(ws->basis.data(), F, Sp, bs, ts, ws->stream));
   if (after_stage) CK(ws, cudaEventRecord(after_stage, ws->stream));
@@ -429,7 +429,7 @@ int enqueue_stage(wedg_ws *ws, const StageIO &S, const Fields *Fo = nullptr, cud
     cudaEventRecord(e3, ws->stream);
     ws->ev_pending.push_back({e0, e1, e2, e3});
   }
-  ws->stats.kernel_launches += prep_done ? 3 : 4;
+  ws->stats.kernel_launches += 3;
   ws->stats.element_stages += ws->E;
   CK(ws, cudaGetLastError());
   return WEDG_OK;
@@ -770,7 +770,7 @@ bool same_kernels(const wedg_ws *a, const wedg_ws *b) {
          a->basis == b->basis;
 }
 
-// One RHS evaluation (k_prep, k_bnd, k_stage, mass solve) of every workspace of a group, each with its
+// One RHS evaluation (k_prep, k_stage, mass solve) of every workspace of a group, each with its
 // own Fields and StageIO; one workspace: enqueue_stage. Advances the bin parities as enqueue_stage.
 int group_stage(const std::vector<wedg_ws *> &G, const std::vector<StageIO> &S, const std::vector<Fields> &F) {
   if (G.size() == 1) return enqueue_stage(G[0], S[0], &F[0]);

@@ -201,10 +201,12 @@ cudaError_t launch_prep(const void *basis, const Fields &F, const StageIO &S, in
                         cudaStream_t st, int e0) {
   // (ranges of elements also wait for their copies to the device, and are launched after those)
   const bool all = blocks * prep_tile(NU, threads) >= F.E;
-  return launch_after(k_prep<NU, NV>, all ? F.E : INT_MAX, blocks, threads, st, basis_of<NU, NV>(basis), F, S, e0);
+  const int sides = (threads / 32) * bnd_tile(NU), nb = all ? (4 * F.N + sides - 1) / sides : 0;
+  return launch_after(k_prep<NU, NV>, all ? F.E : INT_MAX, nb + blocks, threads, st, basis_of<NU, NV>(basis), F, S,
+                      e0, nb);
 }
 
-// k_bnd over the 4N physical sides (the grid follows from F.N)
+// k_bnd over the 4N physical sides (the grid follows from F.N), after a k_prep by ranges
 template <int NU, int NV>
 cudaError_t launch_bnd(const void *basis, const Fields &F, const StageIO &S, int, int, cudaStream_t st) {
   return launch_after(k_bnd<NU, NV>, F.E, (4 * F.N + bnd_tile(NU) - 1) / bnd_tile(NU), BND_THREADS, st,

@@ -13,14 +13,14 @@
 // small meshes over the chip and keeps the registers low enough for 24 to 32
 // warps an SM.
 //
-// One RHS evaluation is four kernels:
+// One RHS evaluation is three kernels:
 //   k_prep   traces of the stage state on the four sides of every element
 //            (src/rhs.jl:384-410), the weight check of the boundary points
 //            (src/rhs.jl:105-110, 729-757), G = 2βv at the high-order points
 //            and the Chebyshev interval data (src/rhs.jl:889-907), so that every
 //            error of the stage is known before the next kernel starts;
-//   k_bnd    the flux slots of the physical sides (src/rhs.jl:65-103), projected
-//            on the face modes;
+//            Its first blocks, or k_bnd, take the flux slots of the physical sides
+//            (src/rhs.jl:65-103), projected on the face modes;
 //   k_stage  face fluxes of the element's own interior sides (src/rhs.jl:611-700),
 //            lifts (:412-473), volume terms (:309-333), source
 //            (:335-350) and u-equation (:352-382) with the u part of the RK4
@@ -268,17 +268,6 @@ struct GPack {
   __device__ i64 word() const { return (i64)sG << 32 | (unsigned)ng; }
 };
 
-// The value at face point i of side `side` of trace family fam of element e held as modal end sums
-// (Fields::modal): Σ_b P[i][b] t[b] over the family's n modes
-template <int NQ, int NU, int n>
-__device__ __forceinline__ double modal_at(const double (&P)[NQ][NU], const double *tr, int fam, int side, int i,
-                                           size_t E, int e) {
-  double x = 0.0;
-#pragma unroll
-  for (int b = 0; b < n; ++b) x = fma(P[i][b], tr[((fam * 4 + side) * NQ + b) * E + e], x);
-  return x;
-}
-
 // ----------------------------------------------------------------------------
 // k_stage helpers
 // ----------------------------------------------------------------------------
@@ -333,12 +322,10 @@ __device__ __forceinline__ void interior_flux(const Fields &F, const FaceCoef &c
 
 // Numerical flux slots A, D, F at point i of physical side s of the element (src/rhs.jl:65-103, 738-763)
 template <int NU, int NV>
-__device__ __forceinline__ void boundary_point(const Basis<NU, NV> &B, const Fields &F, const TimeF &S, int s, int j,
-                                               int k, int e, int i, double &A, double &D, double &Fs) {
-  constexpr int NQ = NU;
-  const int N = F.N, E = F.E;
-  const double *tr = F.tr;
-  auto T = [&](int fam, int side, int el) { return tr[((fam * 4 + side) * NQ + i) * (size_t)E + el]; };
+__device__ __forceinline__ void boundary_point(const Fields &F, const TimeF &S, int s, int j,
+                                               int k, int i, double du, double v_fp, double dv_fp, double &A,
+                                               double &D, double &Fs) {
+  const int N = F.N;
   const int m = s < 2 ? k : j;
   const double sgn = (s == 0 || s == 2) ? -1.0 : 1.0;
   size_t fi;
@@ -346,10 +333,7 @@ __device__ __forceinline__ void boundary_point(const Basis<NU, NV> &B, const Fie
   if (s < 2) { fi = (s == 0 ? 0 : N) + (size_t)(N + 1) * (k + (size_t)N * i); c2a = F.hc2; afa = F.haf; cfa = F.hcf; bfa = F.hbf; }
   else { fi = j + (size_t)N * ((s == 2 ? 0 : N) + (size_t)(N + 1) * i); c2a = F.vc2; afa = F.vaf; cfa = F.vcf; bfa = F.vbf; }
   const double c2f = c2a[fi], af = afa[fi], cf = cfa[fi];
-  const bool modal = F.modal != 0;
-  const double v_fp = modal ? modal_at<NQ, NU, NV>(B.P, tr, 1, s, i, E, e) : T(1, s, e);
-  const double gun = sgn * (F.two_h * (modal ? modal_at<NQ, NU, NU>(B.P, tr, 0, s, i, E, e) : T(0, s, e)));
-  const double gvn = sgn * (F.two_h * (modal ? modal_at<NQ, NU, NV>(B.P, tr, 2, s, i, E, e) : T(2, s, e)));
+  const double gun = sgn * (F.two_h * du), gvn = sgn * (F.two_h * dv_fp);
   const double spn = F.bspn[s][m + (size_t)N * i], sp = F.bsp[s][m + (size_t)N * i];
   const double gu_ex = sgn * (S.ct * spn - spn);
   const double gv_ex = sgn * (-F.omega * S.st * spn);
@@ -404,12 +388,15 @@ __device__ __forceinline__ void side_point(const Fields &F, int s, int j, int k,
   interior_flux(F, cf, plus, dum, dup, vm, vp, dvm, dvp, A, D, Fs);
 }
 
-// k_bnd: the physical sides, a team of NQ lanes per side: lane i evaluates the flux slots at
-// point i, then projects them on mode i (Y[b] = Σ_q w_q P[q][b] (.)_q), and k_stage reads the
+// The physical sides, a team of NQ lanes per side: lane i takes the side's traces at mode i from the state,
+// evaluates the flux slots at point i, then projects them on mode i (Y[b] = Σ_q w_q P[q][b] (.)_q), and k_stage reads the
 // projections. A point costs about 150 FP64 operations (two square roots and the divisions); in its
 // element's thread of k_stage a side held the 31 others of the warp up for 7 points on end, in every
 // fourth warp at N = 256 and in every one below N = 64, and the columns of the left and right sides
-// were whole warps of it. Spread over the chip the 4N sides take some 6 us.
+// were whole warps of it. With traces of their own (6 NU operations a lane) the sides need nothing of k_prep,
+// so a launch of it over all elements has them as its first blocks; after k_prep, as a kernel of their own
+// (k_bnd: after a k_prep by ranges of elements, and k_bnd_m), they take 6 to 9 us of a stage: N = 64 31 -> 23 us with
+// k_prep, N = 512 445 -> 436.
 constexpr int BND_THREADS = 32;
 __host__ __device__ constexpr int bnd_tile(int nu) { return BND_THREADS / nu; }
 template <int NU, int NV>
@@ -417,15 +404,40 @@ __device__ __forceinline__ void bnd_body(const Basis<NU, NV> &B, const Fields &F
   constexpr int NQ = NU;
   const int N = F.N, E = F.E, lane = threadIdx.x & 31, tw = lane / NQ, i = lane - tw * NQ;
   const int x = side0 + tw;
-  after_previous();
   if (tw >= bnd_tile(NU) || x >= 4 * N) return;
-  if (err_word(F) != ERR_NONE) return;
   const unsigned mask = ((1u << NQ) - 1u) << (tw * NQ);
   const TimeF tf = time_factors(S);
   const int s = x / N, m = x - s * N;
   const int j = s == 0 ? 0 : s == 1 ? N - 1 : m, k = s == 2 ? 0 : s == 3 ? N - 1 : m, e = j + N * k;
+  // the side's traces: the sums over the normal modes at mode i along the side, then at point i
+  const size_t Eu = (size_t)E;
+  const bool hi = s & 1, along = s < 2, has_v = i < NV;
+  double xe = 0, xo = 0, ve = 0, vo = 0, de = 0, dd = 0;
+#pragma unroll
+  for (int a = 0; a < NU; ++a) {
+    const double x = S.xu[e + Eu * (along ? a + NU * i : i + NU * a)];
+    if (a & 1) xo = fma(B.E1l[a], x, xo);
+    else xe = fma(B.E1l[a], x, xe);
+  }
+#pragma unroll
+  for (int a = 0; a < NV; ++a) {
+    const double x = has_v ? S.xv[e + Eu * (along ? a + NV * i : i + NV * a)] : 0.0;
+    if (a & 1) { vo = fma(B.El[a], x, vo); dd = fma(B.E1l[a], x, dd); }
+    else { ve = fma(B.El[a], x, ve); de = fma(B.E1l[a], x, de); }
+  }
+  const double mu = hi ? xo - xe : xe + xo, mv = hi ? ve - vo : ve + vo, md = hi ? dd - de : de + dd;
+  double du = 0.0, v = 0.0, dv = 0.0;
+#pragma unroll
+  for (int b = 0; b < NU; ++b) {
+    const double p = B.P[i][b];
+    du = fma(p, __shfl_sync(mask, mu, tw * NQ + b), du);
+    if (b < NV) {
+      v = fma(p, __shfl_sync(mask, mv, tw * NQ + b), v);
+      dv = fma(p, __shfl_sync(mask, md, tw * NQ + b), dv);
+    }
+  }
   double A, D, Fs;
-  boundary_point<NU, NV>(B, F, tf, s, j, k, e, i, A, D, Fs);
+  boundary_point<NU, NV>(F, tf, s, j, k, i, du, v, dv, A, D, Fs);
   double ya = 0.0, yd = 0.0, yf = 0.0;
 #pragma unroll
   for (int q = 0; q < NQ; ++q) {
@@ -446,6 +458,7 @@ template <int NU, int NV>
 __global__ void __launch_bounds__(BND_THREADS) k_bnd(const __grid_constant__ Basis<NU, NV> B,
                                                      const __grid_constant__ Fields F,
                                                      const __grid_constant__ StageIO S) {
+  after_previous();
   bnd_body<NU, NV>(B, F, S, blockIdx.x * bnd_tile(NU));
 }
 // tile = bnd_tile(NU) sides per virtual block, of the 4N of an instance
@@ -475,7 +488,7 @@ __device__ __forceinline__ int cheb_count(double L, double th, double de) {
 //
 // What bounds it: the FP64 pipe (60 %: the traces, and a conversion per entry of V and 2β) and the latency of
 // its loads. N = 512, q = 6: 760 us as FP64 code with a thread per element; 526, 488, 458 and 442 us so at four, five,
-// six and eight blocks an SM (64 registers).
+// six and eight blocks an SM (64 registers), the last with the physical sides 445, and 436 with them in its own blocks.
 template <int NU, int NV>
 struct PrepTeam {
   static constexpr int QH = qhigh(NU, NV), TPW = 32 / NU;
@@ -720,11 +733,16 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
 template <int NU, int NV>
 __global__ void __launch_bounds__(128, 8) k_prep(const __grid_constant__ Basis<NU, NV> B,
                                               const __grid_constant__ Fields F,
-                                              const __grid_constant__ StageIO S, int e0) {
+                                              const __grid_constant__ StageIO S, int e0, int nb) {
   after_previous();
+  const int vb = (int)blockIdx.x - nb;
+  if (vb < 0) {                                          // the first nb blocks take the physical sides
+    bnd_body<NU, NV>(B, F, S, (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * bnd_tile(NU));
+    return;
+  }
   // elements from e0 on: a launch may cover a range of the elements (the first range clears the next
   // stage's counts)
-  prep_body<NU, NV>(B, F, S, e0 + (int)blockIdx.x * prep_tile(NU, blockDim.x), blockIdx.x == 0 && e0 == 0);
+  prep_body<NU, NV>(B, F, S, e0 + vb * prep_tile(NU, blockDim.x), vb == 0 && e0 == 0);
 }
 
 // tile = prep_tile(NU, threads) elements per virtual block

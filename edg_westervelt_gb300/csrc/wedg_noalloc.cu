@@ -306,7 +306,6 @@ extern "C" int wedg_rhs_noalloc(const wedg_config *cfg, const wedg_pre *pre, con
   unsigned long long err = 0;
   unsigned int cgf = 0;
   if ((ce = Lch.prep(basis, F, S, (iE + ep - 1) / ep, tp, st, 0)) != cudaSuccess ||
-      (ce = Lch.bnd(basis, F, S, 1, BND_THREADS, st)) != cudaSuccess ||
       (ce = Lch.stage(basis, F, S, (iE + tile - 1) / tile, ts, st)) != cudaSuccess ||
       (ce = Lch.mass(basis, F, S, 1, CHEB_THREADS, st)) != cudaSuccess ||
       (ce = cudaGetLastError()) != cudaSuccess ||

@@ -174,6 +174,10 @@ __device__ __forceinline__ TimeF time_factors(const StageIO &S) {
 __device__ __forceinline__ unsigned long long err_word(const Fields &F) {
   return *(volatile unsigned long long *)F.err;
 }
+// Whether an error is known, the same answer for all threads of a team (the kernel may be recording one meanwhile)
+__device__ __forceinline__ bool team_stopped(const Fields &F, unsigned mask) {
+  return __any_sync(mask, err_word(F) != ERR_NONE);
+}
 
 // ----------------------------------------------------------------------------
 // Multi-instance launches (the batched form): one launch runs one kernel of a stage for up to
@@ -517,8 +521,8 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
   if (tw >= T::TPW) return;
   const int r = lane - tw * NU, slot = (threadIdx.x >> 5) * T::TPW + tw, e = e0 + slot;
   if (e >= E) return;
-  if (err_word(F) != ERR_NONE) return;
   const unsigned mask = ((1u << NU) - 1u) << (tw * NU);
+  if (team_stopped(F, mask)) return;
   const size_t Eu = (size_t)E;
   const bool has_v = r < NV, modal = F.modal != 0;
   double *Us = sh + slot * T::SLOT, *Vs = Us + NU * NU;
@@ -1078,8 +1082,8 @@ _Pragma("unroll") \
   if (tw >= T::TPW) return; \
   const int u = lane - tw * QH, lane0 = tw * QH, slot = (threadIdx.x >> 5) * T::TPW + tw, g = (g0) + slot; \
   if (g >= F.E) return; \
-  if (err_word(F) != ERR_NONE) return; \
   const unsigned mask = ((1u << QH) - 1u) << lane0; \
+  if (team_stopped(F, mask)) return; \
   const size_t Eu = (size_t)F.E;
 
 template <int NU, int NV>

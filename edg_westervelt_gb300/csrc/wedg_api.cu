@@ -45,12 +45,20 @@ __global__ void k_rk4_final(int n_u, int n_v, double *u, double *v, const double
   if (!fin) atomicOr(nonfinite, 1u);
 }
 
+// The bookkeeping at the end of a step: a known error stops the steps after it (latch_error)
+__device__ __forceinline__ void step_done(unsigned long long *err, const unsigned int *nonfinite, int stop_nonfinite,
+                                          long long *steps_done) {
+  if (*err == ERR_NONE) {
+    *steps_done += 1;
+    if (stop_nonfinite && *nonfinite) *err = (3ull << ERR_CLASS_SHIFT);
+  }
+  err[1] = *err;
+}
+
 __global__ void k_step_done(unsigned long long *err, const unsigned int *nonfinite, int stop_nonfinite,
                             long long *steps_done) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (*err != ERR_NONE) return;
-  *steps_done += 1;
-  if (stop_nonfinite && *nonfinite) *err = (3ull << ERR_CLASS_SHIFT);
+  step_done(err, nonfinite, stop_nonfinite, steps_done);
 }
 
 // out = a x + b y (+ z), elementwise; y, z may be null
@@ -100,9 +108,7 @@ __global__ void k_step_done_p(const __grid_constant__ StepMulti P) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.n) return;
   const StepFlagsP &x = P.f[i];
-  if (*x.err != ERR_NONE) return;
-  *x.steps_done += 1;
-  if (P.stop_nonfinite && *x.nonfinite) *x.err = (3ull << ERR_CLASS_SHIFT);
+  step_done(x.err, x.nonfinite, P.stop_nonfinite, x.steps_done);
 }
 
 // The candidates of the autotuners, tried one coordinate at a time (k_prep's block, then the
@@ -157,7 +163,7 @@ __global__ void k_batch_reset(const BatchFlagPtrs *p, int n) {
   const BatchFlagPtrs f = p[blockIdx.x];
   for (int t = threadIdx.x; t < 2 * NBIN; t += blockDim.x) f.bin_count[t] = 0;
   if (threadIdx.x == 0) {
-    *f.err = ERR_NONE;
+    f.err[0] = f.err[1] = ERR_NONE;
     *f.nsum = 0;
     *f.cg_nfail = 0;
     *f.nonfinite = 0;
@@ -541,6 +547,12 @@ int adjoint_buffers(wedg_ws *ws) {
 int enqueue_adjoint_core(wedg_ws *ws, const Fields &Fs, const StageIO &S, const double *lam_u, const double *lam_v,
                          double *gu, double *gv, double *gpar) {
   const int ts = STAGE_THREADS, tile = stage_tile(ws->nu), bs = (ws->E + tile - 1) / tile;
+  // ν = A_e⁻¹ λ_u (first: k_stage stops the mass solve on an error of the forward one)
+  StageIO Su = S;
+  Su.mode = OUT_ADJ_USOLVE;
+  Su.xu = lam_u;
+  Su.ut = ws->adj_nu;
+  CK(ws, ws->L.stage(ws->basis.data(), Fs, Su, bs, ts, ws->stream));
   // μ = M(v)⁻¹ λ_v, on the Chebyshev data of the state
   Fields Fm = Fs;
   Fm.mrhs = const_cast<double *>(lam_v);
@@ -548,12 +560,6 @@ int enqueue_adjoint_core(wedg_ws *ws, const Fields &Fs, const StageIO &S, const 
   Sm.mode = OUT_RHS;
   Sm.vt = ws->adj_mu;
   CK(ws, ws->L.mass(ws->basis.data(), Fm, Sm, 1, ws->mass_threads, ws->stream));
-  // ν = A_e⁻¹ λ_u
-  StageIO Su = S;
-  Su.mode = OUT_ADJ_USOLVE;
-  Su.xu = lam_u;
-  Su.ut = ws->adj_nu;
-  CK(ws, ws->L.stage(ws->basis.data(), Fs, Su, bs, ts, ws->stream));
   const AdjIO A{ws->adj_mu, ws->adj_nu, ws->adj_nus, S.vt, ws->adj_hat, gu, gv, S.xv,
                 gpar ? gpar + 2 * (size_t)ws->E : nullptr};
   ws->L.adj_hats(ws->basis.data(), Fs, S, A, ws->stream);
@@ -846,6 +852,17 @@ int group_adjoint_core(const std::vector<wedg_ws *> &G, const std::vector<Fields
   std::vector<StageArgs> sa(n);
   std::vector<AdjArgs> aa(n);
   cudaError_t e;
+  // ν = A_e⁻¹ λ_u (first, as in enqueue_adjoint_core)
+  for (int i = 0; i < n; ++i) {
+    sa[i].F = Fs[i];
+    sa[i].S = S[i];
+    sa[i].S.mode = OUT_ADJ_USOLVE;
+    sa[i].S.xu = lam_u[i];
+    sa[i].S.ut = G[i]->adj_nu;
+  }
+  if ((e = multi_stage_launch(w->L, w->basis.data(), w->nu, w->nv, w->fast, MK_STAGE, sa, 0, w->stream, all)) !=
+      cudaSuccess)
+    return cuda_fail(w, e, "multi-instance launch");
   // μ = M(v)⁻¹ λ_v on the Chebyshev data of the states
   for (int i = 0; i < n; ++i) {
     sa[i].F = Fs[i];
@@ -856,17 +873,6 @@ int group_adjoint_core(const std::vector<wedg_ws *> &G, const std::vector<Fields
   }
   if ((e = multi_stage_launch(w->L, w->basis.data(), w->nu, w->nv, w->fast, MK_MASS, sa, w->mass_threads, w->stream,
                               all)) != cudaSuccess)
-    return cuda_fail(w, e, "multi-instance launch");
-  // ν = A_e⁻¹ λ_u
-  for (int i = 0; i < n; ++i) {
-    sa[i].F = Fs[i];
-    sa[i].S = S[i];
-    sa[i].S.mode = OUT_ADJ_USOLVE;
-    sa[i].S.xu = lam_u[i];
-    sa[i].S.ut = G[i]->adj_nu;
-  }
-  if ((e = multi_stage_launch(w->L, w->basis.data(), w->nu, w->nv, w->fast, MK_STAGE, sa, 0, w->stream, all)) !=
-      cudaSuccess)
     return cuda_fail(w, e, "multi-instance launch");
   for (int i = 0; i < n; ++i) {
     wedg_ws *g = G[i];
@@ -1336,9 +1342,7 @@ __global__ void k_step_done_m(int n, const StepFlags *f, int stop_nonfinite) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const StepFlags x = f[i];
-  if (*x.err != ERR_NONE) return;
-  *x.steps_done += 1;
-  if (stop_nonfinite && *x.nonfinite) *x.err = (3ull << ERR_CLASS_SHIFT);
+  step_done(x.err, x.nonfinite, stop_nonfinite, x.steps_done);
 }
 
 // k_rk4_final of many CG instances in one launch: blockIdx.y is the instance
@@ -1737,7 +1741,7 @@ int create_finish(wedg_ws *ws) {
   const size_t nU = (size_t)nu * nu * E, nV = (size_t)nv * nv * E;
   if ((rc = dalloc(ws, &F.tr, (size_t)12 * nq * E)) || (rc = dalloc(ws, &F.G, ((size_t)qh * qh + 2) * E)) ||
       (rc = dalloc(ws, &F.bslots, (size_t)4 * N * (2 * nv + nu))) || (rc = dalloc(ws, &F.th, Es)) || (rc = dalloc(ws, &F.de, Es)) || (rc = dalloc(ws, &F.nst, Es)) ||
-      (rc = dalloc(ws, &F.nmax, 3)) || (rc = dalloc(ws, &F.nsum, 1)) || (rc = dalloc(ws, &F.err, 1)) ||
+      (rc = dalloc(ws, &F.nmax, 3)) || (rc = dalloc(ws, &F.nsum, 1)) || (rc = dalloc(ws, &F.err, 2)) ||
       (rc = dalloc(ws, &F.cg_nfail, 1)) ||
       (rc = dalloc(ws, &F.nonfinite, 1)) || (rc = dalloc(ws, &ws->steps_done, 1)) ||
       (rc = dalloc(ws, &ws->d_u, nU)) || (rc = dalloc(ws, &ws->d_v, nV)) || (rc = dalloc(ws, &ws->d_ut, nU)) ||

@@ -119,7 +119,7 @@ struct Fields {
                               // src/rhs.jl:911-918), [2] of the whole call (statistics)
   int *bins, *bin_count;      // elements by Chebyshev count: bins[b E + i], two count buffers of NBIN
   unsigned long long *nsum;   // Σ of the per-element Chebyshev step counts
-  unsigned long long *err;
+  unsigned long long *err;    // [0] the error recorded, [1] the same once later kernels stop for it
   unsigned int *cg_nfail, *nonfinite;
   double theta, tau, lu, lv, omega, two_h, four_hh, mass_tol, Lcheb;
   int one_sided, mms_on, src_on, cg, cheb_common, sorted;
@@ -174,9 +174,25 @@ __device__ __forceinline__ TimeF time_factors(const StageIO &S) {
 __device__ __forceinline__ unsigned long long err_word(const Fields &F) {
   return *(volatile unsigned long long *)F.err;
 }
-// Whether an error is known, the same answer for all threads of a team (the kernel may be recording one meanwhile)
+// Errors are recorded by k_prep and k_cg (F.err[0], the smallest by atomicMin), and which one is reported must
+// not depend on the order of their blocks. So these kernels and k_cheb stop on errors of earlier kernels alone:
+// those which the last k_stage or the end of a step found (F.err[1], latch_error). Between k_cg and the next
+// k_prep there may be neither, but with k_cg k_prep records boundary weights only, so any other error is
+// an earlier one. One answer for all threads of a team (several streams may share the words).
 __device__ __forceinline__ bool team_stopped(const Fields &F, unsigned mask) {
-  return __any_sync(mask, err_word(F) != ERR_NONE);
+  return __any_sync(mask, *(volatile unsigned long long *)(F.err + 1) != ERR_NONE);
+}
+__device__ __forceinline__ bool prep_stopped(const Fields &F, unsigned mask) {
+  bool stop = *(volatile unsigned long long *)(F.err + 1) != ERR_NONE;
+  if (F.cg) {
+    const unsigned long long w = err_word(F);
+    stop = stop || (w != ERR_NONE && (w >> ERR_CLASS_SHIFT) > 0);
+  }
+  return __any_sync(mask, stop);
+}
+__device__ __forceinline__ void latch_error(const Fields &F) {
+  const unsigned long long w = err_word(F);
+  if (w != ERR_NONE) F.err[1] = w;
 }
 
 // ----------------------------------------------------------------------------
@@ -522,7 +538,7 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
   const int r = lane - tw * NU, slot = (threadIdx.x >> 5) * T::TPW + tw, e = e0 + slot;
   if (e >= E) return;
   const unsigned mask = ((1u << NU) - 1u) << (tw * NU);
-  if (team_stopped(F, mask)) return;
+  if (prep_stopped(F, mask)) return;
   const size_t Eu = (size_t)E;
   const bool has_v = r < NV, modal = F.modal != 0;
   double *Us = sh + slot * T::SLOT, *Vs = Us + NU * NU;

@@ -250,9 +250,9 @@ extern "C" int wedg_rhs_noalloc(const wedg_config *cfg, const wedg_pre *pre, con
   F.mrhs = base + o_mrhs;
   F.bins = reinterpret_cast<int *>(base + o_bins);
   F.bin_count = reinterpret_cast<int *>(base + o_bcnt);
-  double *flags = base + o_flags;   // err (u64), nsum (u64), cg_nfail, nonfinite (u32), nmax (3 ints)
+  double *flags = base + o_flags;   // err (2 u64), nsum (u64), cg_nfail, nonfinite (u32), nmax (3 ints)
   F.err = reinterpret_cast<unsigned long long *>(flags);
-  F.nsum = reinterpret_cast<unsigned long long *>(flags + 1);
+  F.nsum = reinterpret_cast<unsigned long long *>(flags + 2);
   F.nmax = reinterpret_cast<int *>(flags + 5);
   F.cg_nfail = reinterpret_cast<unsigned int *>(flags + 3);
   F.nonfinite = reinterpret_cast<unsigned int *>(flags + 4);
@@ -298,7 +298,7 @@ extern "C" int wedg_rhs_noalloc(const wedg_config *cfg, const wedg_pre *pre, con
   // ---- clear what must start at zero (the array keeps the last call's contents), then run
   if ((ce = cudaMemsetAsync(flags, 0, 8 * sizeof(double), st)) != cudaSuccess ||
       (ce = cudaMemsetAsync(F.bin_count, 0, 2 * NBIN * sizeof(int), st)) != cudaSuccess ||
-      (ce = cudaMemsetAsync(F.err, 0xFF, sizeof(unsigned long long), st)) != cudaSuccess) {
+      (ce = cudaMemsetAsync(F.err, 0xFF, 2 * sizeof(unsigned long long), st)) != cudaSuccess) {
     if (msg && msg_len) snprintf(msg, msg_len, "CUDA error: %s", cudaGetErrorString(ce));
     return WEDG_ERR_CUDA;
   }

@@ -137,6 +137,7 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
   }
   if (threadIdx.x < NU) { tE[threadIdx.x] = B.fEl[threadIdx.x]; tE[NU + threadIdx.x] = B.fE1[threadIdx.x]; }
   after_previous();
+  if (e0 == 0 && threadIdx.x == 0) latch_error(F);
   __syncthreads();
   const int lane = threadIdx.x & 31, tw = lane / NU;
   if (tw >= T::TPW) return;

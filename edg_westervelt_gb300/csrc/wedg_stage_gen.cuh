@@ -142,6 +142,7 @@ __device__ __forceinline__ void stage_gen_body(const Basis<NU, NV> &B, const Fie
     ends[i] = B.El[i]; ends[NU + i] = B.E1l[i]; ends[2 * NU + i] = B.E1F[i];
   }
   after_previous();
+  if (e0 == 0 && threadIdx.x == 0) latch_error(F);
   __syncthreads();
   const int lane = threadIdx.x & 31, tw = lane / NU;
   if (tw >= T::TPW) return;

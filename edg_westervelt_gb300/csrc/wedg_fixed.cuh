@@ -68,6 +68,16 @@ __device__ __forceinline__ int fx_hi(i64 x) {
   return h ^ (h >> 31);
 }
 
+// x 2^-n for n ≥ 0 (toward -∞; n from 64 on as 63) and x 2^n for any n, modulo 2^64
+__device__ __forceinline__ i64 fx_sar(i64 x, int n) {
+  asm("shr.s64 %0, %0, %1;" : "+l"(x) : "r"(n));
+  return x;
+}
+__device__ __forceinline__ i64 fx_shift(i64 x, int n) {
+  asm("shl.b64 %0, %0, %1;" : "+l"(x) : "r"(max(n, 0)));     // 0 from 64 on
+  return fx_sar(x, max(-n, 0));
+}
+
 // 2^k for -1022 ≤ k ≤ 1023
 __device__ __forceinline__ double fx_pow2(int k) { return __hiloint2double((k + 1023) << 20, 0); }
 

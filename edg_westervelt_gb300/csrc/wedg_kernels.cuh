@@ -847,10 +847,11 @@ __device__ __forceinline__ void store_v(const StageIO &S, size_t l, double kk, b
 // first.
 //
 // The iteration runs in fixed point on the system scaled by the middle θ of the spectral interval,
-// (M/θ) X' = R with X' = θX, whose spectrum is 1 ± ε, ε = δ/θ: the integers of r, X' and d keep the
-// exponent of R through all steps (the solution grows by at most 1/(1 - ε), for which R gets
-// headroom), and d goes into the products with M as d 2^nd, at the top of its range. Elements with
-// ε > 31/32, θ < 1/8 or max|G| > 7 and right-hand sides that are not finite take it in FP64.
+// (M/θ) X' = R with X' = θX, whose spectrum is 1 ± ε, ε = δ/θ. r, X' and d are integers r 2^nr, X' 2^nX and
+// d 2^nd of the exponent of R, each brought to the top of its range by its own shift after every step, so
+// that each keeps some 55 bits of its own size or more, however far the residual falls and whatever ε, θ and
+// G are. (With one exponent for r and X' over all steps, and the headroom that the solution may need,
+// 49 bits were left at ε close to 1, and systems beyond ε = 31/32 took a form in FP64.)
 //
 // What bounds it: one product with M costs about 1 300 multiply-adds an element at q = 6, three integer
 // ones each (4 cycles a warp), and 18 shared-memory words a thread; a thread per row keeps 24 warps an SM
@@ -978,78 +979,6 @@ __device__ __forceinline__ void team_K_fx(const Basis<NU, NV> &B, const Fx2 *Gs,
   }
 }
 
-// k_cheb's iteration in FP64, for the elements beyond the limits of the fixed-point form
-template <int NU, int NV>
-__device__ __noinline__ void cheb_fp64(const Basis<NU, NV> &B, const StageIO &S, const i64 *G, int sG,
-                                       const double (&R)[MassTeam<NU, NV>::J], double th, double de, int n, int u,
-                                       unsigned mask, size_t Eu, int e, double *xs, double *X, double *zs,
-                                       bool &fin) {
-  using T = MassTeam<NU, NV>;
-  constexpr int QH = T::QH, NE = T::NE, J = T::J;
-  const double gs = ldexp(1.0, sG), s1 = th / de, ith = 1.0 / th;
-  double rr[J];
-#pragma unroll 1
-  for (int j = 0; j < J; ++j) {
-    const int k = u + QH * j;
-    rr[j] = R[j];
-    if (k < NE) {
-      X[k] = 0.0;
-      xs[k] = R[j] * ith;
-    }
-  }
-  __syncwarp(mask);
-  double rho = 1.0 / s1;
-#pragma unroll 1
-  for (int step = 1; step <= n; ++step) {
-#pragma unroll 1
-    for (int j = 0; j < J; ++j) {
-      const int k = u + QH * j;
-      if (k < NE) {
-        X[k] += xs[k];
-        rr[j] -= xs[k];
-      }
-    }
-    if (step == n) break;
-    // r += K d: row u at the points, weighted, and back (zs holds QH rows of NV)
-    double t[NV], z[NV];
-#pragma unroll
-    for (int b = 0; b < NV; ++b) {
-      t[b] = z[b] = 0.0;
-#pragma unroll
-      for (int a = 0; a < NV; ++a) t[b] = fma(B.Ph[u][a], xs[a + NV * b], t[b]);
-    }
-#pragma unroll 1
-    for (int s2 = 0; s2 < QH; ++s2) {
-      double y = 0.0;
-#pragma unroll
-      for (int b = 0; b < NV; ++b) y = fma(t[b], B.Ph[s2][b], y);
-      y *= (double)G[(u + QH * s2) * Eu] * gs;
-#pragma unroll
-      for (int b = 0; b < NV; ++b) z[b] = fma(y, B.PhW[s2][b], z[b]);
-    }
-#pragma unroll
-    for (int b = 0; b < NV; ++b) zs[u * NV + b] = z[b];
-    __syncwarp(mask);
-    const double rhon = 1.0 / (2.0 * s1 - rho);
-    const double c1 = rhon * rho, c2 = 2.0 * rhon / de;
-#pragma unroll 1
-    for (int j = 0; j < J; ++j) {
-      const int k = u + QH * j;
-      if (k < NE) {
-        for (int v = 0; v < QH; ++v) rr[j] = fma(B.PhW[v][k % NV], zs[v * NV + k / NV], rr[j]);
-        xs[k] = fma(c1, xs[k], c2 * rr[j]);
-      }
-    }
-    rho = rhon;
-    __syncwarp(mask);
-  }
-#pragma unroll 1
-  for (int j = 0; j < J; ++j) {
-    const int k = u + QH * j;
-    if (k < NE) store_v(S, e + Eu * k, X[k], fin);
-  }
-}
-
 // 1/D for 1 ≤ D ≤ 2 as integers of 2^-59: FP32's reciprocal and two steps of Newton's method
 __device__ __forceinline__ i64 fx_recip(i64 D) {
   const float f = __uint_as_float((unsigned)(D >> 36) - (1u << 23) + (127u << 23));   // D ≥ 2^59: its top 24 bits
@@ -1128,26 +1057,16 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
     for (int s2 = 0; s2 < QH; ++s2) Gs[u + QH * s2] = fx_split(G[(u + QH * s2) * Eu] << gp.ng);
   hr = __reduce_max_sync(mask, hr);
   bool fin = true;
-  const double ith = 1.0 / th, eps = de * ith;
-  // max|G| from the ends of the interval
-  const double gmax = fmax(fabs(1.0 - (th + de)), fabs(1.0 - (th - de)));
-  if (fx_finite(hr) && eps <= 31.0 / 32.0 && th >= 0.125 && gmax <= 7.0) {
-    // R with headroom: the entries of X' and d stay below |R|max + 2 ε/(1 - ε) |R| and those of M d below
-    // that with |R| (1 + max|G|) (the Euclidean norm, from the entries' high words in FP32, with a
-    // little to spare)
-    float r2 = 0.0f;
+  const double ith = 1.0 / th;
+  if (!fx_finite(hr)) {
 #pragma unroll
     for (int j = 0; j < J; ++j) {
-      const int x = fx_abs_hi(R[j]) - (hr & 0x7ff00000) + (127 << 20);   // |R| over the largest's power of two
-      const float f = x > 0 ? __int_as_float(x << 3) : 0.0f;
-      r2 = fmaf(f, f, r2);
+      const int k = u + QH * j;
+      if (k < NE) store_v(S, e + Eu * k, n > 1 ? __longlong_as_double(0x7ff8000000000000LL) : R[j] * ith, fin);
     }
-    r2 = (float)__reduce_add_sync(mask, (unsigned)(r2 * 1024.0f) + 1) * (1.0f / 1024.0f);
-    const float ef = (float)eps;
-    const float grow = 1.0f + 0.51f * (1.0f + (float)gmax) * fmaxf(1.0f, 2.0f * ef / (1.0f - ef)) * sqrtf(r2);
-    const int hb = (__float_as_int(grow) >> 23) - 126;
-    const int er = fx_exp(hr) + hb;
-    // r in registers, X' and d (as d 2^nd, what M takes) in shared memory
+  } else {
+    const int er = fx_exp(hr);
+    // r in registers, X' and d in shared memory
     Fx2 *xf = reinterpret_cast<Fx2 *>(xs);
     i64 *Xf = reinterpret_cast<i64 *>(X);
     i64 rr[J];
@@ -1156,63 +1075,112 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
       const int k = u + QH * j;
       rr[j] = fx_from(R[j], er);
       if (k < NE) {
-        Xf[k] = 0;
-        xf[k] = fx_split(rr[j] << hb);
+        Xf[k] = rr[j];
+        xf[k] = fx_split(rr[j]);
       }
     }
     __syncwarp(mask);
-    int nd = hb;                                   // d 2^nd, just below 2^61, is what M takes
-    const int kd = max(gp.sG - gp.ng + 64, -62);
-    const Fx2 ithf = fx_split(fx_scalar(ith, FX_BIAS - 56));          // 1/θ as an integer of 2^-56
+    // r = rr 2^-nr with room for ur bits more, d = (Xf's thread entries) 2^-nd at the top of its range, X' with
+    // high words below bX
+    int nr = 0, ur = 0, nX = 0, nd = 0;
+    unsigned bX = (1u << 29) + 1;
+    const int kd = gp.sG - gp.ng + 64;             // K d 2^nd = y 2^kd
+    // 1/θ = (integer 2^-60) 2^(fi - 1022), the integer in [2^59, 2^60). The entries of (M/θ) d are below
+    // (1 + ε) NV times the largest of d (Euclidean norms), that is below 2^LG times it
+    constexpr int LG = NV <= 1 ? 1 : NV <= 2 ? 2 : NV <= 4 ? 3 : 4;
+    static_assert(2 * NV <= 1 << LG, "the bound of a step");
+    const int fi = (__double2hiint(ith) >> 20) & 0x7ff;
+    const Fx2 ithf = fx_split(fx_from(ith, fi + 1));
     // the scalars, as integers of 2^-59: with q = ρ θ/δ the recurrence ρ' = 1/(2 θ/δ - ρ) is q' = 1/(2 - ε² q),
     // and d' = ρ'ρ d + 2 (ρ'/δ) r in the scaled system is ε² q q' d + 2 q' r
+    const double eps = de * ith;
     const Fx2 e2 = fx_split(fx_scalar(eps * eps, FX_BIAS - 59));
     i64 q = (i64)1 << 59;                          // ρ = δ/θ: q = 1
 #pragma unroll 1
-    for (int step = 1; step <= n; ++step) {
-#pragma unroll
-      for (int j = 0; j < J; ++j) {
-        const int k = u + QH * j;
-        if (k < NE) Xf[k] += fx_join(xf[k]) >> nd;
-      }
-      if (step == n) break;
-      // r -= (M/θ) d, M d = d - K d, with K d 2^nd = y 2^kd
-      const int up = max(kd - nd, 0), down = min(max(nd - kd, 0), 62);
-      const i64 half = down ? (i64)1 << (down - 1) : 0;
+    for (int step = 1; step < n; ++step) {
+      // r -= (M/θ) d, M d = d - K d, at the exponent n1 that leaves both below 2^60. The difference, times
+      // 2^(fi - 1022) for 1/θ, is below 2^61 and is taken modulo 2^64
+      const int n1 = min(nr + ur, nd - LG) - 1, sd = fi - 1022 + n1 - nd, sy = kd + sd, sr = n1 - nr;
+      // (a half unit of bias a step would add up: r moved down goes toward -∞, and so does what is taken from it)
+      const int half_p = sr < 0 ? 0 : 1 << 27;
+      int hr1 = 0;
       team_K_fx<NU, NV>(B, Gs, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs), [&](int j, int k, i64 y) {
-        const Fx2 t = fx_split((fx_join(xf[k]) >> nd) - (((y << up) + half) >> down));
-        const i64 m = fx_mad(t.h, ithf.l, fx_mad(t.l, ithf.h, (fx_mad(t.l, ithf.l, 0) >> 32) + (1 << 23)));
-        rr[j] -= (fx_mad(t.h, ithf.h, 0) << 8) + (m >> 24);
+        const Fx2 t = fx_split((i64)((u64)fx_shift(fx_join(xf[k]), sd) - (u64)fx_shift(y, sy)));
+        const i64 m = fx_mad(t.h, ithf.l, fx_mad(t.l, ithf.h, half_p));
+        rr[j] = fx_shift(rr[j], sr) - ((fx_mad(t.h, ithf.h, 0) << 4) + (m >> 28));
+        hr1 |= fx_hi(rr[j]);
       });
       const i64 eq = fx_mul(fx_split(q), e2) << 2;                       // ε² q
       q = fx_recip(((i64)1 << 60) - eq);
-      const Fx2 qs = fx_split(q), c1 = fx_split(fx_mul(qs, fx_split(eq)) << 2), c2 = fx_split(2 * q);
+      const Fx2 qs = fx_split(q), c2 = fx_split(2 * q);
+      const Fx2 c1 = fx_split(fx_sar(fx_mul(qs, fx_split(eq)) << 2, nd - n1));   // d's part at the exponent n1
       int hd = 0;
       i64 dd[J];
 #pragma unroll
       for (int j = 0; j < J; ++j) {
         const int k = u + QH * j;
-        const Fx2 d = fx_split(k < NE ? fx_join(xf[k]) >> nd : 0), r = fx_split(rr[j]);
+        const Fx2 d = k < NE ? xf[k] : Fx2{0, 0}, r = fx_split(rr[j]);
         const i64 m = fx_mad(d.h, c1.l, fx_mad(d.l, c1.h, fx_mad(r.h, c2.l, fx_mad(r.l, c2.h, 1 << 26))));
         dd[j] = (fx_mad(d.h, c1.h, fx_mad(r.h, c2.h, 0)) << 5) + (m >> 27);
-        hd = max(hd, fx_hi(dd[j]));
+        hd |= fx_hi(dd[j]);
       }
-      nd = fx_room(__reduce_max_sync(mask, hd));
+      // the room of both (|r| ≤ 2^61, |d'| < 2^63), as far as 14 bits, from the ors of the high words' upper halves
+      const unsigned w = __reduce_or_sync(mask, (unsigned)hd >> 15 | (unsigned)hr1 >> 15 << 16);
+      const int ud = __clz(w & 0xffff) - 18;
+      ur = __clz(w >> 16) - 18;
+      nr = n1;
+      nd = n1 + ud;
+      // X' += d', to nearest
+      int sX = nd - nX;
+      if (sX < 0) {
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+          if (u + QH * j < NE) Xf[u + QH * j] = fx_sar(Xf[u + QH * j], -sX);
+        bX = (bX >> min(-sX, 31)) + 1;
+        nX = nd;
+        sX = 0;
+      }
+      sX = min(sX, 62);
+      const i64 half = ((i64)1 << sX) >> 1;
 #pragma unroll
       for (int j = 0; j < J; ++j) {
         const int k = u + QH * j;
-        if (k < NE) xf[k] = fx_split(dd[j] << nd);
+        const i64 d = fx_shift(dd[j], ud);
+        if (k < NE) {
+          xf[k] = fx_split(d);
+          Xf[k] += fx_sar(d + half, sX);
+        }
+      }
+      bX += ((1u << 29) >> min(sX, 31)) + 1;
+      if (bX > 0x50000000u) {                      // the next d' may not fit: the actual size, and down by one if needed
+        int hX = 0;
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+          if (u + QH * j < NE) hX = max(hX, fx_hi(Xf[u + QH * j]));
+        bX = __reduce_max_sync(mask, hX) + 1;
+        if (bX > 1u << 29) {
+#pragma unroll
+          for (int j = 0; j < J; ++j)
+            if (u + QH * j < NE) Xf[u + QH * j] >>= 1;
+          bX = (bX >> 1) + 1;
+          --nX;
+        }
       }
       __syncwarp(mask);
     }
-    const double sc = fx_pow2(er - FX_BIAS) * ith;
+    // X = X' / θ; in two factors where 2^kk or the product of both is beyond the normal numbers
+    const int kk = er - FX_BIAS - nX, ei = fi - 1023;
+    const bool wide = kk > 1023 || abs(kk + ei) > 1000;
+    const double sc = wide ? fx_pow2(-ei) * ith : fx_pow2(kk) * ith;
 #pragma unroll
     for (int j = 0; j < J; ++j) {
       const int k = u + QH * j;
-      if (k < NE) store_v(S, e + Eu * k, __dmul_rn((double)Xf[k], sc), fin);
+      if (k < NE) {
+        double x = __dmul_rn((double)Xf[k], sc);
+        if (wide) x = ldexp(x, kk + ei);
+        store_v(S, e + Eu * k, x, fin);
+      }
     }
-  } else {
-    cheb_fp64<NU, NV>(B, S, G, gp.sG, R, th, de, n, u, mask, Eu, e, xs, X, zs, fin);
   }
   if (S.mode == OUT_RK4_LAST && !fin) atomicOr(F.nonfinite, 1u);
 }

@@ -256,12 +256,12 @@ __device__ __forceinline__ void adj_mass_body(const Basis<NU, NV> &B, const Fiel
     if (k < NE) xf[k] = fx_split(fx_from(mu[j], ex));
   }
   __syncwarp(mask);
-  const double nan = __longlong_as_double(0x7ff8000000000000LL);
-  const int k2 = (ex - FX_BIAS) + (eg - FX_BIAS) + 64;   // in two factors: the exponents may add up to a subnormal
-  const double s1 = fx_finite(hg) && fx_finite(hx) ? ldexp(1.0, k2 / 2) : nan, s2 = ldexp(1.0, k2 - k2 / 2);
-  team_K_fx<NU, NV>(B, Gs, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs), [&](int j, int k, i64 y) {
-    if (k < NE) A.gv[e + Eu * k] = fma((double)y * s1, s2, A.gv[e + Eu * k]);
-  });
+  const double one = fx_finite(hg) && fx_finite(hx) ? 1.0 : __longlong_as_double(0x7ff8000000000000LL);
+  const int k0 = (ex - FX_BIAS) + (eg - FX_BIAS);
+  team_K_fx<NU, NV>(B, Gs, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs),
+                    [&](int j, int k, i64 y, int ey) {
+                      if (k < NE) A.gv[e + Eu * k] = fx_scale((double)y * one, k0 + ey) + A.gv[e + Eu * k];
+                    });
 }
 
 template <int NU, int NV>

@@ -134,7 +134,8 @@ void pack_basis(const BasisHost &h, void *out) {
     b.cPh[d] = (int)ceil(ldexp(c, 8));
   }
   {
-    double c = 0;                  // the largest Euclidean norm of a row of Ph
+    // rows of the grid of K d stay below max|G| |d| max_r |Ph[r]| (Euclidean norms)
+    double c = 0;
     for (int r = 0; r < QH; ++r) {
       double s = 0;
       for (int d = 0; d < NV; ++d) s += b.Ph[r][d] * b.Ph[r][d];

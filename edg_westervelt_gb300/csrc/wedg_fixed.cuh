@@ -78,8 +78,12 @@ __device__ __forceinline__ i64 fx_shift(i64 x, int n) {
   return fx_sar(x, max(-n, 0));
 }
 
-// 2^k for -1022 ≤ k ≤ 1023
+// 2^k for -1022 ≤ k ≤ 1023, and x 2^k for any k (rounded where that is subnormal)
 __device__ __forceinline__ double fx_pow2(int k) { return __hiloint2double((k + 1023) << 20, 0); }
+__device__ __forceinline__ double fx_scale(double x, int k) {
+  k = min(max(k, -2044), 2046);
+  return __dmul_rn(__dmul_rn(x, fx_pow2(k >> 1)), fx_pow2(k - (k >> 1)));
+}
 
 __device__ __forceinline__ i64 fx_mad(int a, int b, i64 c) {
   i64 d;

@@ -91,7 +91,7 @@ struct Basis {
   FxC fPh[QH][NV], fPhW[QH][NV], fEl[NU], fE1[NU], fK1[NU][NU], fQ[NU][NU], fL[NU][NU], fM[NU][NU][2];
   int gPh, gPhW, gEl, gE1, gK1, gQ, gL, gM;   // their exponents
   int kK1[NU];
-  int nrow;                      // bits that team_K_fx shifts the grid rows up by
+  int nrow;                      // bits that the grid rows of team_K_fx have room for in every case
   int cPh[NV];                   // 2^8 max|Ph[.][a]|, rounded up
 };
 
@@ -875,18 +875,20 @@ __host__ __device__ constexpr int mass_tile(int nu, int nv, int threads) {
 }
 
 // One product with K = P_h^T W G P_h for x in xs (Fx2, below 2^61, complete, after a __syncwarp) and G in
-// Gs: use(j, k, y) for the thread's entries k = u + QH j, where K x = y 2^(sG - ng + 64) (GPack) in the
-// integers of x. The levels of the sum factorisation keep the exponents fixed by the operators.
+// Gs: use(j, k, y, ey) for the thread's entries k = u + QH j, where K x = y 2^(sG - ng + ey) (GPack) in the
+// integers of x. The operators' exponents leave headroom at every level for the largest sums that are
+// possible, up to four bits more than sums usually take. So each level's numbers go up to the top of their
+// range by what room they have: the thread's row T and its weighted points by nt, the rows of the team by nz.
+// Without the second and third shift the error of a product was 2 to 5e-16 of its largest entry from n_v = 4
+// on, as in FP64 or twice that, and is 0.3 to 1e-16 so. Up to n_v = 3 (0.5 to 1.6e-16) the rows go up by
+// what the norms leave in every case (nrow), and the last level takes the products of the low halves too: the
+// shifts would cost a tenth of such a product.
 template <int NU, int NV, class Use>
 __device__ __forceinline__ void team_K_fx(const Basis<NU, NV> &B, const Fx2 *Gs, int u, int lane0, unsigned mask,
                                           const Fx2 *Phs, const Fx2 *PhWs, const Fx2 *xs, Fx2 *zs, const Use &use) {
   using T = MassTeam<NU, NV>;
   constexpr int QH = T::QH, HP = T::HP, NE = T::NE, J = T::J, NP = (NV + 1) / 2;
-  // The levels leave headroom for sums that K does not reach: its rows of the grid stay below
-  // max|G| |d| max_r |Ph[r]| (Euclidean norms) and K d below max|G| |d|. The rows go up by nrow bits, and
-  // the modes by the rest, so that little is lost to the rounding of the levels; T goes up to the top
-  // of its range for the points, by the thread's own nt.
-  const int nrow = B.nrow, zsh = 2 * (61 - B.gPh) + 2 * (61 - B.gPhW) - nrow;
+  constexpr bool RISE = NV >= 4;
   const bool high = u >= HP;                             // the mirror of a lower row
   const int low = high ? QH - 1 - u : u, mate = lane0 + (QH - 1 - u);
   // row u of P_h d: the thread of the lower row sums the even modes, its mirror the odd ones
@@ -915,37 +917,46 @@ __device__ __forceinline__ void team_K_fx(const Basis<NU, NV> &B, const Fx2 *Gs,
   nt = fx_room(nt);
   // the points of the row, weighted, and back to the modes
   i64 Z[NV];
+  int nz;
   {
     Fx2 t[NV];
 #pragma unroll
     for (int b = 0; b < NV; ++b) t[b] = fx_split(Tv[b] << nt);
     auto tv = [&](int b) { return t[b]; };
-    Fx2 ys[QH / 2 + 1], yd[QH / 2 + 1];
+    i64 ys[QH / 2 + 1], yd[QH / 2 + 1];
     auto weigh = [&](i64 y0, int s2) {
       const Fx2 y = fx_split(y0), g = Gs[u + QH * s2];
       const i64 m = fx_mad(y.h, g.l, fx_mad(y.l, g.h, 1 << 28));
       return (fx_mad(y.h, g.h, 0) << 3) + (m >> 29);
     };
+    int top = 0;
 #pragma unroll
     for (int s2 = 0; s2 < QH / 2; ++s2) {
       auto c = [&](int b) -> const FxC & { return B.fPh[s2][b]; };
       const i64 e0 = fx_dot<0, 2, NV>(tv, c), o0 = fx_dot<1, 2, NV>(tv, c);
       const i64 p = weigh(e0 + o0, s2), m = weigh(e0 - o0, QH - 1 - s2);
-      ys[s2] = fx_split(p + m);
-      yd[s2] = fx_split(p - m);
+      ys[s2] = p + m;
+      yd[s2] = p - m;
+      if constexpr (RISE) top |= fx_hi(p + m) | fx_hi(p - m);
     }
-    if constexpr ((QH & 1) != 0)
-      ys[QH / 2] = fx_split(
-          weigh(fx_dot<0, 2, NV>(tv, [&](int b) -> const FxC & { return B.fPh[QH / 2][b]; }), QH / 2));
-    const int dn = nt - nrow;
+    if constexpr ((QH & 1) != 0) {
+      ys[QH / 2] = weigh(fx_dot<0, 2, NV>(tv, [&](int b) -> const FxC & { return B.fPh[QH / 2][b]; }), QH / 2);
+      if constexpr (RISE) top |= fx_hi(ys[QH / 2]);
+    }
+    const int nw = RISE ? fx_room(top) : 0;
+    nt += nw;
+    int hz = 0;
 #pragma unroll
     for (int b = 0; b < NV; ++b) {
       auto c = [&](int s2) -> const FxC & { return B.fPhW[s2][b]; };
-      i64 z;
-      if (b & 1) z = fx_dot<0, 1, QH / 2>([&](int s2) { return yd[s2]; }, c);
-      else z = fx_dot<0, 1, (QH + 1) / 2>([&](int s2) { return ys[s2]; }, c);
-      Z[b] = dn > 0 ? (z + ((i64)1 << (dn - 1))) >> dn : z << -dn;
+      if (b & 1) Z[b] = fx_dot<0, 1, QH / 2>([&](int s2) { return fx_split(yd[s2] << nw); }, c);
+      else Z[b] = fx_dot<0, 1, (QH + 1) / 2>([&](int s2) { return fx_split(ys[s2] << nw); }, c);
+      hz |= fx_hi(Z[b]);
     }
+    // the rows' common exponent, below 2^60 for the sums of pairs
+    nz = RISE ? __reduce_min_sync(mask, nt + fx_room(hz)) - 1 : B.nrow;
+#pragma unroll
+    for (int b = 0; b < NV; ++b) Z[b] = fx_shift(Z[b], nz - nt);
   }
   // the sums (lower row's thread) and differences (its mirror) of the row pairs, [row NV + b] each; the
   // middle row is its own sum, and its difference is not read for anything (P_h's odd modes vanish there)
@@ -957,24 +968,22 @@ __device__ __forceinline__ void team_K_fx(const Basis<NU, NV> &B, const Fx2 *Gs,
     if (2 * u + 1 == QH) zs[(HP + low) * NV + b] = Fx2{0, 0};
   }
   __syncwarp(mask);
+  const int zsh = 2 * (61 - B.gPh) + 2 * (61 - B.gPhW) - nz, ey = RISE ? 61 + zsh : 64;
 #pragma unroll
   for (int j = 0; j < J; ++j) {
     const int k = u + QH * j;
     if (k < NE) {
       const int a = k % NV, b = k / NV;
       const Fx2 *z = zs + ((a & 1) ? HP * NV : 0) + b;
-      // (with the products of the low halves: the result goes up by zsh)
-      i64 m = 0, h = 0, l = 0;
+      i64 m = RISE ? 1 << 28 : 0, h = 0;
 #pragma unroll
       for (int v = 0; v < HP; ++v) {
         const Fx2 p = PhWs[v * NV + a], y = z[v * NV];
-        l += fx_mad(y.l, p.l, 0) >> 32;
-        m = fx_mad(y.h, p.l, m);
-        m = fx_mad(y.l, p.h, m);
+        if constexpr (!RISE) m += fx_mad(y.l, p.l, 0) >> 32;
+        m = fx_mad(y.h, p.l, fx_mad(y.l, p.h, m));
         h = fx_mad(y.h, p.h, h);
       }
-      m += l;
-      use(j, k, (h << zsh) + (m >> (32 - zsh)));
+      use(j, k, RISE ? (h << 3) + (m >> 29) : (h << zsh) + (m >> (32 - zsh)), ey);
     }
   }
 }
@@ -1084,7 +1093,6 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
     // high words below bX
     int nr = 0, ur = 0, nX = 0, nd = 0;
     unsigned bX = (1u << 29) + 1;
-    const int kd = gp.sG - gp.ng + 64;             // K d 2^nd = y 2^kd
     // 1/θ = (integer 2^-60) 2^(fi - 1022), the integer in [2^59, 2^60). The entries of (M/θ) d are below
     // (1 + ε) NV times the largest of d (Euclidean norms), that is below 2^LG times it
     constexpr int LG = NV <= 1 ? 1 : NV <= 2 ? 2 : NV <= 4 ? 3 : 4;
@@ -1100,11 +1108,12 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
     for (int step = 1; step < n; ++step) {
       // r -= (M/θ) d, M d = d - K d, at the exponent n1 that leaves both below 2^60. The difference, times
       // 2^(fi - 1022) for 1/θ, is below 2^61 and is taken modulo 2^64
-      const int n1 = min(nr + ur, nd - LG) - 1, sd = fi - 1022 + n1 - nd, sy = kd + sd, sr = n1 - nr;
+      const int n1 = min(nr + ur, nd - LG) - 1, sd = fi - 1022 + n1 - nd, sr = n1 - nr;
       // (a half unit of bias a step would add up: r moved down goes toward -∞, and so does what is taken from it)
       const int half_p = sr < 0 ? 0 : 1 << 27;
       int hr1 = 0;
-      team_K_fx<NU, NV>(B, Gs, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs), [&](int j, int k, i64 y) {
+      team_K_fx<NU, NV>(B, Gs, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs), [&](int j, int k, i64 y, int ey) {
+        const int sy = gp.sG - gp.ng + ey + sd;
         const Fx2 t = fx_split((i64)((u64)fx_shift(fx_join(xf[k]), sd) - (u64)fx_shift(y, sy)));
         const i64 m = fx_mad(t.h, ithf.l, fx_mad(t.l, ithf.h, half_p));
         rr[j] = fx_shift(rr[j], sr) - ((fx_mad(t.h, ithf.h, 0) << 4) + (m >> 28));
@@ -1120,16 +1129,17 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
       for (int j = 0; j < J; ++j) {
         const int k = u + QH * j;
         const Fx2 d = k < NE ? xf[k] : Fx2{0, 0}, r = fx_split(rr[j]);
-        const i64 m = fx_mad(d.h, c1.l, fx_mad(d.l, c1.h, fx_mad(r.h, c2.l, fx_mad(r.l, c2.h, 1 << 26))));
-        dd[j] = (fx_mad(d.h, c1.h, fx_mad(r.h, c2.h, 0)) << 5) + (m >> 27);
+        const i64 m = fx_mad(d.h, c1.l, fx_mad(d.l, c1.h, fx_mad(r.h, c2.l, fx_mad(r.l, c2.h, 1 << 28))));
+        dd[j] = (fx_mad(d.h, c1.h, fx_mad(r.h, c2.h, 0)) << 3) + (m >> 29);
         hd |= fx_hi(dd[j]);
       }
-      // the room of both (|r| ≤ 2^61, |d'| < 2^63), as far as 14 bits, from the ors of the high words' upper halves
+      // the room of both (|r| ≤ 2^61, |d'| < 2^61 at the exponent n1 - 2), as far as 14 bits, from the ors of the
+      // high words' upper halves
       const unsigned w = __reduce_or_sync(mask, (unsigned)hd >> 15 | (unsigned)hr1 >> 15 << 16);
-      const int ud = __clz(w & 0xffff) - 18;
+      const int ud = max(__clz(w & 0xffff) - 18, 0);
       ur = __clz(w >> 16) - 18;
       nr = n1;
-      nd = n1 + ud;
+      nd = n1 - 2 + ud;
       // X' += d', to nearest
       int sX = nd - nX;
       if (sX < 0) {
@@ -1145,7 +1155,7 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
 #pragma unroll
       for (int j = 0; j < J; ++j) {
         const int k = u + QH * j;
-        const i64 d = fx_shift(dd[j], ud);
+        const i64 d = dd[j] << ud;
         if (k < NE) {
           xf[k] = fx_split(d);
           Xf[k] += fx_sar(d + half, sX);
@@ -1229,10 +1239,10 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
       y[j] = 0.0;
     }
     __syncwarp(mask);
-    const double sc = g_ok && fx_finite(hx) ? ldexp(1.0, ex - FX_BIAS + gp.sG - gp.ng + 64)
-                                            : __longlong_as_double(0x7ff8000000000000LL);
+    const double one = g_ok && fx_finite(hx) ? 1.0 : __longlong_as_double(0x7ff8000000000000LL);
+    const int k0 = ex - FX_BIAS + (g_ok ? gp.sG - gp.ng : 0);
     team_K_fx<NU, NV>(B, Gs, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs),
-                      [&](int j, int, i64 v) { y[j] = __dmul_rn((double)v, sc); });
+                      [&](int j, int, i64 v, int ey) { y[j] = fx_scale((double)v * one, k0 + ey); });
     __syncwarp(mask);
   };
   double X[J], r[J], p[J], Ap[J];

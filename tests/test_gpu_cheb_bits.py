@@ -13,10 +13,10 @@ from oracle.precompute import precompute as opre
 pytestmark = pytest.mark.gpu
 
 # (lowest, highest) 2βv: ε = δ/θ of 0.025, 0.58, 0.80, 0.959, 0.9678, 0.9692, 0.9656, 0.958, 0.9676, 0.9685, 0.995; θ
-# of 0.126 and 0.124; a matrix far from and one close to zero everywhere
+# of 0.126 and 0.124; a matrix far from and one close to zero everywhere; a spread of three orders
 SPANS = [(-0.02, 0.03), (-0.58, 0.58), (-6.0, 0.2), (-0.9, 0.96), (-0.9, 0.969), (-0.9, 0.9703), (-3.0, 0.93),
          (-6.0, 0.85), (-6.9, 0.87), (-7.1, 0.87), (-1.0, 0.995), (0.868, 0.88), (0.87, 0.882), (-40.0, -3.0),
-         (0.999, 0.9995)]
+         (0.999, 0.9995), (-300.0, 0.9)]
 
 
 def _operators(po):

@@ -148,7 +148,8 @@ void pack_basis(const BasisHost &h, void *out) {
   }
   // the constant-coefficient kernels' operators: the end values two to a sum (A and D of a side), K1
   // by its rows (columns in one sum with them), Q by rows or columns beside the constant mode
-  double eL = 0, e1 = 0, sK = 0, bK = 0, sQ = 0, bQ = 0, bL = 0, bE = 0, QE[NU];
+  double eL = 0, e1 = 0, sK = 0, bK = 0, sQ = 0, bQ = 0, bL = 0, bE = 0;
+  double QE[NU];
   for (int i = 0; i < NU; ++i) {
     big(eL, fabs(h.El[i]));
     big(e1, fabs(h.E1l[i]));
@@ -186,8 +187,8 @@ void pack_basis(const BasisHost &h, void *out) {
       b.fK1[i][a] = fx_const(ldexp(h.K1[i][a], -k1_bits<NU>(a)), b.gK1);
       b.fQ[i][a] = fx_const(i == 0 || a == 0 ? 0.0 : h.Q[i][a], b.gQ);
       b.fL[i][a] = fx_const(i + a == 0 ? 0.0 : h.ilam2[i][a], b.gL);
-      b.fM[i][a][0] = fx_const(i + a == 0 ? 0.0 : QE[i] * h.ilam2[i][a], b.gM);
-      b.fM[i][a][1] = fx_const(i + a == 0 ? 0.0 : QE[a] * h.ilam2[i][a], b.gM);
+      b.fM[i][a][0] = fx_const(i + a == 0 ? 0.0L : (long double)QE[i] * h.ilam2[i][a], b.gM);
+      b.fM[i][a][1] = fx_const(i + a == 0 ? 0.0L : (long double)QE[a] * h.ilam2[i][a], b.gM);
     }
   }
   for (int r = 0; r < QH; ++r)

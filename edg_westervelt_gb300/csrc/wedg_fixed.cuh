@@ -122,8 +122,8 @@ inline int fx_exponent(double sum, double big) {
   frexp(big * (1 + 1e-6), &b);
   return (61 - a < 60 - b) ? 61 - a : 60 - b;
 }
-inline FxC fx_const(double x, int g) {
-  const Fx2 p = fx_split((i64)llrint(ldexp(x, g)));
+inline FxC fx_const(long double x, int g) {
+  const Fx2 p = fx_split((i64)llrintl(ldexpl(x, g)));
   return FxC{p.h, p.l, 8 * p.h};
 }
 

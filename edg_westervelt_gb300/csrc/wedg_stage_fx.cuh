@@ -431,6 +431,7 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
   sX = usolve ? sV + 61 - B.gL : max(sV, sB) + 1;
   const int nV = sX - sV, nB = sX - sB;
   const Fx2 g1[2] = {fx_split(f1[0]), fx_split(f1[1])};
+  int top = 0;                                           // the largest high word of the row
 #pragma unroll
   for (int b = 0; b < NU; ++b) {
     auto q = [&](int m) -> const FxC & { return B.fQ[m][b]; };
@@ -439,7 +440,7 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
     else y = (b & 1) ? fx_dot<1, 2, NU>(xs, q) : fx_dot<2, 2, NU>(xs, q);
     if (usolve) {
       const FxC l = B.fL[c][b];
-      X[c + NU * b] = fx_mul(fx_split(y), Fx2{l.h, l.l});
+      y = fx_mul(fx_split(y), Fx2{l.h, l.l});
     } else {
       const Fx2 f0 = fx_split(FQ[(c & 1) * NU + b]), g = g1[b & 1];
       const FxC c0 = tM[c * NU + b][0], c1 = tM[c * NU + b][1];
@@ -447,12 +448,18 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
       m = fx_mad(g.h, c1.l, fx_mad(g.l, c1.h, m));
       m = fx_mad(f0.h, c0.h8, m >> 29);
       m = fx_mad(g.h, c1.h8, m);
-      X[c + NU * b] = fx_down(y, nV) + fx_down(m, nB);
+      y = fx_down(y, nV) + fx_down(m, nB);
     }
+    X[c + NU * b] = y;
+    top |= fx_hi(y);
   }
+  // Each product leaves dQ bits of headroom for sums that an orthonormal Q seldom has: over the four of them eight
+  // bits, so that 52 were left. The room there is after two is taken back (2^sX stays far from subnormal)
+  const int up = min(fx_room(__reduce_or_sync(mask, top)), max(sX + 960, 0));
+  sX -= up;
   __syncwarp(mask);
 #pragma unroll
-  for (int i = 0; i < NU; ++i) x[i] = fx_split(X[i + NU * c]);
+  for (int i = 0; i < NU; ++i) x[i] = fx_split(X[i + NU * c] << up);
   X[NU * c] = fx_down(fx_join(x[0]), dQ);                // Q X, column c
 #pragma unroll
   for (int a = 1; a < NU; ++a) {

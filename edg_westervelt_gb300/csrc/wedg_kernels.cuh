@@ -1305,15 +1305,20 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
   if (S.mode == OUT_RK4_LAST && !fin) atomicOr(F.nonfinite, 1u);
 }
 
+// Blocks per SM asked of the mass solves. k_cheb: five from n_v = 6 on, where six (80 registers) spill 92 bytes a
+// thread and more (a stage's solves at N = 512, q = 6: 935 us at six, 888 at five; N = 300, q = 7 4 690 and 4 636 us), and
+// six below (n_v = 5, N = 256: 132 and 138 us; n_v = 3, N = 333: 314 and 322 us). k_cg: three
+__host__ __device__ constexpr int mass_blocks(int nv, bool cg) { return cg ? 3 : nv >= 6 ? 5 : 6; }
+
 template <int NU, int NV>
-__global__ void __launch_bounds__(CHEB_THREADS, 6)
+__global__ void __launch_bounds__(CHEB_THREADS, mass_blocks(NV, false))
     k_cheb(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ Fields F,
            const __grid_constant__ StageIO S) {
   cheb_body<NU, NV>(B, F, S, blockIdx.x * mass_tile(NU, NV, blockDim.x));
 }
 
 template <int NU, int NV>
-__global__ void __launch_bounds__(CHEB_THREADS, 3)
+__global__ void __launch_bounds__(CHEB_THREADS, mass_blocks(NV, true))
     k_cg(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ Fields F,
          const __grid_constant__ StageIO S) {
   cg_body<NU, NV>(B, F, S, blockIdx.x * mass_tile(NU, NV, blockDim.x));
@@ -1321,7 +1326,7 @@ __global__ void __launch_bounds__(CHEB_THREADS, 3)
 
 // tile = mass_tile elements per virtual block; CG selects k_cg's body
 template <int NU, int NV, bool CG>
-__global__ void __launch_bounds__(CHEB_THREADS, CG ? 3 : 6)
+__global__ void __launch_bounds__(CHEB_THREADS, mass_blocks(NV, CG))
     k_mass_m(const __grid_constant__ Basis<NU, NV> B, const __grid_constant__ MultiStage P) {
   for (int vb = blockIdx.x; vb < P.first[P.n]; vb += gridDim.x) {
     const int inst = multi_begin(P, vb);

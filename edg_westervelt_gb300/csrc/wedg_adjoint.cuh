@@ -45,8 +45,8 @@ struct AdjTeam {
   if (tw >= T::TPW) return; \
   const int r = lane - tw * NU, lane0 = tw * NU, slot = (threadIdx.x >> 5) * T::TPW + tw, e = (e0) + slot; \
   if (e >= F.E) return; \
-  if (err_word(F) != ERR_NONE) return; \
   const unsigned mask = (unsigned)((1ull << NU) - 1) << lane0; \
+  if (team_failed(F, mask)) return; \
   const size_t Eu = (size_t)F.E; \
   double *s = sh + slot * T::SLOT;
 

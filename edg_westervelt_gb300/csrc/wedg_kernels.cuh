@@ -190,6 +190,12 @@ __device__ __forceinline__ bool prep_stopped(const Fields &F, unsigned mask) {
   }
   return __any_sync(mask, stop);
 }
+// k_stage and the adjoint's kernels stop on any error: none is recorded on their stream while they run, but another
+// stream's k_prep may record one for the same words (the adjoint's recompute beside its reverse sweep), and a team
+// must leave as a whole
+__device__ __forceinline__ bool team_failed(const Fields &F, unsigned mask) {
+  return __any_sync(mask, err_word(F) != ERR_NONE);
+}
 __device__ __forceinline__ void latch_error(const Fields &F) {
   const unsigned long long w = err_word(F);
   if (w != ERR_NONE) F.err[1] = w;

@@ -144,8 +144,8 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
   const int c = lane - tw * NU, slot = (threadIdx.x >> 5) * T::TPW + tw;
   const int e = e0 + slot, E = F.E, N = F.N;
   if (e >= E) return;
-  if (err_word(F) != ERR_NONE) return;
   const unsigned mask = ((1u << NU) - 1u) << (tw * NU);
+  if (team_failed(F, mask)) return;
   const size_t Eu = (size_t)E;
   const bool usolve = S.mode == OUT_ADJ_USOLVE, volume = S.mode == OUT_ADJ_VOLUME;
   const double nan = __longlong_as_double(0x7ff8000000000000LL);

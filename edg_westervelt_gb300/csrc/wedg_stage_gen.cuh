@@ -149,8 +149,8 @@ __device__ __forceinline__ void stage_gen_body(const Basis<NU, NV> &B, const Fie
   const int r = lane - tw * NU, slot = (threadIdx.x >> 5) * T::TPW + tw;
   const int e = e0 + slot, E = F.E, N = F.N;
   if (e >= E) return;
-  if (err_word(F) != ERR_NONE) return;
   const unsigned mask = (NU == 32 ? ~0u : ((1u << NU) - 1u)) << (tw * NU);
+  if (team_failed(F, mask)) return;
   const size_t Eu = (size_t)E;
   const bool adjoint = S.mode >= OUT_ADJ_USOLVE;
   const bool has_v = r < NV;                              // the thread's column of the v-blocks

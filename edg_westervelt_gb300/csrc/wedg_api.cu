@@ -683,7 +683,6 @@ int argument_error(wedg_ws *ws, const std::string &msg) {
 //      launch's capacity (wedg_kernels.cuh): k_prep (tile = prep_tile), k_bnd (tile = bnd_tile of the
 //      4N sides), k_stage (tile = stage_tile), the mass solve (tile = mass_tile). grid_of
 //      maps the virtual blocks of a chunk to its physical grid (persistent launches).
-enum { MK_PREP = 0, MK_BND = 1, MK_STAGE = 2, MK_MASS = 3 };
 template <class GridOf>
 cudaError_t multi_stage_launch(const Launchers &L, const void *basis, int nu, int nv, bool fast, int kind,
                                const std::vector<StageArgs> &args, int threads, cudaStream_t st, GridOf grid_of) {
@@ -1456,12 +1455,10 @@ struct wedg_batch {
 namespace {
 
 // Physical blocks of a multi-instance launch of `total` virtual blocks: all of them, or with
-// persist > 0 that many times the blocks the SMs hold at once (resident blocks per SM at 128
-// threads, scaled for smaller blocks)
-int bucket_grid(const wedg_batch *b, const BatchBucket &k, int total, int resident128, int threads) {
-  if (k.persist <= 0) return total;
-  const int cap = k.persist * b->nsm * resident128 * (128 / std::max(32, std::min(128, threads)));
-  return std::min(total, std::max(cap, 1));
+// persist > 0 that many times the blocks the SMs hold at once
+int bucket_grid(const wedg_batch *b, const BatchBucket &k, int total, int kind, int threads) {
+  if (k.persist <= 0 || kind == MK_BND) return total;
+  return std::min(total, k.persist * b->nsm * k.L.resident(kind, threads, k.cg));
 }
 
 int enqueue_merged_step(wedg_batch *b, BatchBucket &k, double *const *u, double *const *v, const double *t,
@@ -1531,9 +1528,7 @@ int enqueue_merged_step(wedg_batch *b, BatchBucket &k, double *const *u, double 
     }
     for (int kind : {MK_PREP, MK_BND, MK_STAGE, MK_MASS}) {
       const int threads = kind == MK_PREP ? k.prep_threads : kind == MK_MASS ? k.mass_threads : STAGE_THREADS;
-      auto grid = [&](int kd, int total) {
-        return kd == MK_BND ? total : bucket_grid(b, k, total, kd == MK_STAGE ? 2 : 3, threads);
-      };
+      auto grid = [&](int kd, int total) { return bucket_grid(b, k, total, kd, threads); };
       const cudaError_t e =
           multi_stage_launch(k.L, k.basis.data(), k.nu, k.nv, k.fast, kind, args, threads, k.st, grid);
       if (e != cudaSuccess) return cuda_fail(b->ws[k.ids[0]], e, "multi-instance launch");

@@ -45,6 +45,9 @@ typedef void (*adj_face_fn)(const void *basis, const Fields &F, const StageIO &S
 typedef cudaError_t (*multi_fn)(const void *basis, const MultiStage &P, int grid, int threads,
                                 cudaStream_t st);
 typedef cudaError_t (*multi_adj_fn)(const void *basis, const MultiAdj &P, int grid, cudaStream_t st);
+enum { MK_PREP = 0, MK_BND = 1, MK_STAGE = 2, MK_MASS = 3 };
+// Blocks of `threads` threads of a multi-instance kernel that an SM of the current device holds at once
+typedef int (*resident_fn)(int kind, int threads, bool cg);
 
 // k_prep over the elements [e0, e0 + blocks × prep_tile) (clipped to the mesh)
 typedef cudaError_t (*prep_fn)(const void *basis, const Fields &F, const StageIO &S, int blocks, int threads,
@@ -56,6 +59,7 @@ struct Launchers {
   adj_fn adj_hats = nullptr, adj_mass = nullptr;
   adj_face_fn adj_face = nullptr;
   multi_fn prep_m = nullptr, bnd_m = nullptr, stage_m = nullptr, mass_m = nullptr;
+  resident_fn resident = nullptr;
   multi_adj_fn adj_hats_m = nullptr, adj_mass_m = nullptr, adj_face_m = nullptr;
   pack_fn pack = nullptr;
   size_t basis_size = 0;
@@ -293,6 +297,17 @@ cudaError_t launch_mass_m(const void *basis, const MultiStage &P, int grid, int 
   return cudaSuccess;
 }
 
+template <int NU, int NV, bool FAST>
+int resident_m(int kind, int threads, bool cg) {
+  const void *k = kind == MK_PREP    ? (const void *)k_prep_m<NU, NV>
+                  : kind == MK_BND   ? (const void *)k_bnd_m<NU, NV>
+                  : kind == MK_STAGE ? (const void *)k_stage_m<NU, NV, FAST>
+                  : cg               ? (const void *)k_mass_m<NU, NV, true>
+                                     : (const void *)k_mass_m<NU, NV, false>;
+  int n = 0;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads, 0) == cudaSuccess && n > 0 ? n : 1;
+}
+
 template <int NU, int NV>
 cudaError_t launch_adj_hats_m(const void *basis, const MultiAdj &P, int grid, cudaStream_t st) {
   const int total = P.first[P.n];
@@ -329,6 +344,7 @@ Launchers make_launchers(bool fast) {
   L.bnd_m = launch_bnd_m<NU, NV>;
   L.stage_m = fast ? launch_stage_m<NU, NV, true> : launch_stage_m<NU, NV, false>;
   L.mass_m = launch_mass_m<NU, NV>;
+  L.resident = fast ? resident_m<NU, NV, true> : resident_m<NU, NV, false>;
   L.adj_hats_m = launch_adj_hats_m<NU, NV>;
   L.adj_mass_m = launch_adj_mass_m<NU, NV>;
   L.adj_face_m = launch_adj_face_m<NU, NV>;

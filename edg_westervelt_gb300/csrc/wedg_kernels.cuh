@@ -724,15 +724,17 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
   if (F.cg) return;                                      // (k_cg finds a matrix that is not positive definite)
   const double gmin = ldexp((double)kmin, sG), gmax = ldexp((double)kmax, sG);
   const double amin = 1.0 - gmax, amax = 1.0 - gmin;
-  if (nan || !(amin > 0.0)) {
+  const double th = 0.5 * (amax + amin);
+  const double de = fmax(0.5 * (amax - amin), 1e-15 * th);
+  const int n = cheb_count(F.Lcheb, th, de);
+  // (no count: θ = δ to the last bit, a matrix that is singular to rounding. The conversion of an infinite
+  // count gives INT_MAX, steps for an hour)
+  if (nan || !(amin > 0.0) || n == INT_MAX) {
     atomicMin(F.err, (1ull << ERR_CLASS_SHIFT) | (unsigned long long)(e + 1));
     return;
   }
-  const double th = 0.5 * (amax + amin);
-  const double de = fmax(0.5 * (amax - amin), 1e-15 * th);
   F.th[e] = th;
   F.de[e] = de;
-  const int n = cheb_count(F.Lcheb, th, de);
   F.nst[e] = n;
   // largest count and the sum of the counts: one atomic each per warp
   const unsigned am = __activemask();

@@ -73,3 +73,23 @@ def test_errors_of_one_stage_only(gpu):
                 ws.rk4_steps(u, v, 10.0, 1e-4, n)
             assert ws.error_key == 9 + N * 3 + 1
             assert np.array_equal(u, u0) and np.array_equal(v, v0)
+
+
+def test_a_matrix_singular_to_rounding_is_refused(gpu):
+    """1 - 2βv from some 0.1 to 1e18: θ and δ of the Chebyshev interval are the same double, and no number of steps is
+    enough (the reference's ceil(Int, Inf) throws)."""
+    N = 3
+    co = W.constant_coefficients(c=1.0, alpha=1e-6, beta=0.5)
+    pre, _ = W.precompute(3, N, coefficients=co, mixed=False, flux="upwind", mode="source", boundary="wall", kappa=0.5)
+    P = np.asarray(pre["P_h_v"])
+    u = np.zeros((N, N, 4, 4), order="F")
+    v = np.zeros_like(u, order="F")
+    X = np.zeros((4, 4))
+    X[1, 0] = 1.0
+    g = P @ X @ P.T
+    X *= 1e18 / np.ptp(g)
+    X[0, 0] = 2.0 * (0.9 - (P @ X @ P.T).max())
+    v[1, 1] = X
+    ws = W.Workspace(pre, N)
+    with pytest.raises(W.ErrorException, match="mass matrix not positive definite on element 5"):
+        ws.rhs(u, v, 10.0)

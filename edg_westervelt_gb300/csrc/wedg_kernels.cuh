@@ -522,6 +522,9 @@ struct PrepTeam {
   static constexpr int SLOT = (S0 > S1 ? (S0 > S2 ? S0 : S2) : S1 > S2 ? S1 : S2) | 1;   // odd: bank conflicts
 };
 __host__ __device__ constexpr int prep_tile(int nu, int threads) { return (threads / 32) * (32 / nu); }
+// Blocks per SM asked of k_prep: eight (64 registers), and twelve up to q_u = 2, where a thread needs fewer (N = 1024,
+// q_u = 1: 231 and 208 us)
+__host__ __device__ constexpr int prep_blocks(int nu) { return nu <= 3 ? 12 : 8; }
 
 // The block's elements from e0 on (first: the instance's first block, which clears the bin counts)
 template <int NU, int NV>
@@ -759,7 +762,7 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
 }
 
 template <int NU, int NV>
-__global__ void __launch_bounds__(128, 8) k_prep(const __grid_constant__ Basis<NU, NV> B,
+__global__ void __launch_bounds__(128, prep_blocks(NU)) k_prep(const __grid_constant__ Basis<NU, NV> B,
                                               const __grid_constant__ Fields F,
                                               const __grid_constant__ StageIO S, int e0, int nb) {
   after_previous();
@@ -775,7 +778,7 @@ __global__ void __launch_bounds__(128, 8) k_prep(const __grid_constant__ Basis<N
 
 // tile = prep_tile(NU, threads) elements per virtual block
 template <int NU, int NV>
-__global__ void __launch_bounds__(128, 8) k_prep_m(const __grid_constant__ Basis<NU, NV> B,
+__global__ void __launch_bounds__(128, prep_blocks(NU)) k_prep_m(const __grid_constant__ Basis<NU, NV> B,
                                                 const __grid_constant__ MultiStage P) {
   for (int vb = blockIdx.x; vb < P.first[P.n]; vb += gridDim.x) {
     const int inst = multi_begin(P, vb);
@@ -1075,7 +1078,7 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
   hr = __reduce_max_sync(mask, hr);
   bool fin = true;
   const double ith = 1.0 / th;
-  if (!fx_finite(hr)) {
+  if (n == 1 || !fx_finite(hr)) {                  // (one step is R/θ)
 #pragma unroll
     for (int j = 0; j < J; ++j) {
       const int k = u + QH * j;

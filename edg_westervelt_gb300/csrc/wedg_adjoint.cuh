@@ -41,12 +41,12 @@ struct AdjTeam {
   using T = AdjTeam<NU>; \
   __shared__ double sh[T::TPB * T::SLOT]; \
   after_previous(); \
+  if (warp_failed(F)) return; \
   const int lane = threadIdx.x & 31, tw = lane / NU; \
   if (tw >= T::TPW) return; \
   const int r = lane - tw * NU, lane0 = tw * NU, slot = (threadIdx.x >> 5) * T::TPW + tw, e = (e0) + slot; \
   if (e >= F.E) return; \
   const unsigned mask = (unsigned)((1ull << NU) - 1) << lane0; \
-  if (team_failed(F, mask)) return; \
   const size_t Eu = (size_t)F.E; \
   double *s = sh + slot * T::SLOT;
 

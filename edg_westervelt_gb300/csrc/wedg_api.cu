@@ -45,7 +45,7 @@ __global__ void k_rk4_final(int n_u, int n_v, double *u, double *v, const double
   if (!fin) atomicOr(nonfinite, 1u);
 }
 
-// The bookkeeping at the end of a step: a known error stops the steps after it (latch_error)
+// The bookkeeping at the end of a step: a known error stops the steps after it (warp_stopped)
 __device__ __forceinline__ void step_done(unsigned long long *err, const unsigned int *nonfinite, int stop_nonfinite,
                                           long long *steps_done) {
   if (*err == ERR_NONE) {

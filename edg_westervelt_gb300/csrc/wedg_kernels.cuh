@@ -176,29 +176,31 @@ __device__ __forceinline__ unsigned long long err_word(const Fields &F) {
 }
 // Errors are recorded by k_prep and k_cg (F.err[0], the smallest by atomicMin), and which one is reported must
 // not depend on the order of their blocks. So these kernels and k_cheb stop on errors of earlier kernels alone:
-// those which the last k_stage or the end of a step found (F.err[1], latch_error). Between k_cg and the next
+// those which the last k_stage or the end of a step found (F.err[1], stage_failed). Between k_cg and the next
 // k_prep there may be neither, but with k_cg k_prep records boundary weights only, so any other error is
-// an earlier one. One answer for all threads of a team (several streams may share the words).
-__device__ __forceinline__ bool team_stopped(const Fields &F, unsigned mask) {
-  return __any_sync(mask, *(volatile unsigned long long *)(F.err + 1) != ERR_NONE);
+// an earlier one. One answer for all threads of a warp (several streams may share the words, and a team leaves as a
+// whole), before any of them returns: a vote of each team by itself takes 150 to 600 cycles of its warp, one of
+// the warp some 20.
+__device__ __forceinline__ bool warp_stopped(const Fields &F) {
+  return __any_sync(~0u, *(volatile unsigned long long *)(F.err + 1) != ERR_NONE);
 }
-__device__ __forceinline__ bool prep_stopped(const Fields &F, unsigned mask) {
+__device__ __forceinline__ bool prep_stopped(const Fields &F) {
   bool stop = *(volatile unsigned long long *)(F.err + 1) != ERR_NONE;
   if (F.cg) {
     const unsigned long long w = err_word(F);
     stop = stop || (w != ERR_NONE && (w >> ERR_CLASS_SHIFT) > 0);
   }
-  return __any_sync(mask, stop);
+  return __any_sync(~0u, stop);
 }
 // k_stage and the adjoint's kernels stop on any error: none is recorded on their stream while they run, but another
-// stream's k_prep may record one for the same words (the adjoint's recompute beside its reverse sweep), and a team
-// must leave as a whole
-__device__ __forceinline__ bool team_failed(const Fields &F, unsigned mask) {
-  return __any_sync(mask, err_word(F) != ERR_NONE);
-}
-__device__ __forceinline__ void latch_error(const Fields &F) {
+// stream's k_prep may record one for the same words (the adjoint's recompute beside its reverse sweep)
+__device__ __forceinline__ bool warp_failed(const Fields &F) { return __any_sync(~0u, err_word(F) != ERR_NONE); }
+// The same in k_stage, where one thread of a launch (latch) hands the error on to the kernels that stop on earlier
+// errors alone, with the word it has read: a read of its own before the block's barrier was 0.4 us of every stage
+__device__ __forceinline__ bool stage_failed(const Fields &F, bool latch) {
   const unsigned long long w = err_word(F);
-  if (w != ERR_NONE) F.err[1] = w;
+  if (latch && w != ERR_NONE) F.err[1] = w;
+  return __any_sync(~0u, w != ERR_NONE);
 }
 
 // ----------------------------------------------------------------------------
@@ -542,12 +544,12 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
   if (first && threadIdx.x == 0) F.nmax[1 - S.parity] = 0;
   for (int i = threadIdx.x; i < NQ * NU; i += blockDim.x) Ps[i] = B.P[i / NU][i % NU];
   __syncthreads();
+  if (prep_stopped(F)) return;
   const int lane = threadIdx.x & 31, tw = lane / NU;
   if (tw >= T::TPW) return;
   const int r = lane - tw * NU, slot = (threadIdx.x >> 5) * T::TPW + tw, e = e0 + slot;
   if (e >= E) return;
   const unsigned mask = ((1u << NU) - 1u) << (tw * NU);
-  if (prep_stopped(F, mask)) return;
   const size_t Eu = (size_t)E;
   const bool has_v = r < NV, modal = F.modal != 0;
   double *Us = sh + slot * T::SLOT, *Vs = Us + NU * NU;
@@ -1043,12 +1045,12 @@ _Pragma("unroll") \
   }
 #define WEDG_MASS_TEAM(g0) \
   __syncthreads(); \
+  if (warp_stopped(F)) return; \
   const int lane = threadIdx.x & 31, tw = lane / QH; \
   if (tw >= T::TPW) return; \
   const int u = lane - tw * QH, lane0 = tw * QH, slot = (threadIdx.x >> 5) * T::TPW + tw, g = (g0) + slot; \
   if (g >= F.E) return; \
   const unsigned mask = ((1u << QH) - 1u) << lane0; \
-  if (team_stopped(F, mask)) return; \
   const size_t Eu = (size_t)F.E;
 
 template <int NU, int NV>

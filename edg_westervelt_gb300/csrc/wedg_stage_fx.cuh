@@ -149,15 +149,14 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
   }
   if (threadIdx.x < NU) { tE[threadIdx.x] = B.fEl[threadIdx.x]; tE[NU + threadIdx.x] = B.fE1[threadIdx.x]; }
   after_previous();
-  if (e0 == 0 && threadIdx.x == 0) latch_error(F);
   __syncthreads();
+  if (stage_failed(F, e0 == 0 && threadIdx.x == 0)) return;
   const int lane = threadIdx.x & 31, tw = lane / NU;
   if (tw >= T::TPW) return;
   const int c = lane - tw * NU, slot = (threadIdx.x >> 5) * T::TPW + tw;
   const int e = e0 + slot, E = F.E, N = F.N;
   if (e >= E) return;
   const unsigned mask = ((1u << NU) - 1u) << (tw * NU);
-  if (team_failed(F, mask)) return;
   const size_t Eu = (size_t)E;
   const bool usolve = S.mode == OUT_ADJ_USOLVE, volume = S.mode == OUT_ADJ_VOLUME;
   const double nan = __longlong_as_double(0x7ff8000000000000LL);

@@ -142,15 +142,14 @@ __device__ __forceinline__ void stage_gen_body(const Basis<NU, NV> &B, const Fie
     ends[i] = B.El[i]; ends[NU + i] = B.E1l[i]; ends[2 * NU + i] = B.E1F[i];
   }
   after_previous();
-  if (e0 == 0 && threadIdx.x == 0) latch_error(F);
   __syncthreads();
+  if (stage_failed(F, e0 == 0 && threadIdx.x == 0)) return;
   const int lane = threadIdx.x & 31, tw = lane / NU;
   if (tw >= T::TPW) return;
   const int r = lane - tw * NU, slot = (threadIdx.x >> 5) * T::TPW + tw;
   const int e = e0 + slot, E = F.E, N = F.N;
   if (e >= E) return;
   const unsigned mask = (NU == 32 ? ~0u : ((1u << NU) - 1u)) << (tw * NU);
-  if (team_failed(F, mask)) return;
   const size_t Eu = (size_t)E;
   const bool adjoint = S.mode >= OUT_ADJ_USOLVE;
   const bool has_v = r < NV;                              // the thread's column of the v-blocks

@@ -245,8 +245,8 @@ __device__ __forceinline__ void adj_mass_body(const Basis<NU, NV> &B, const Fiel
     mu[j] = k < NE ? A.mu[e + Eu * k] : 0.0;
     hx = max(hx, fx_abs_hi(mu[j]));
   }
-  hg = __reduce_max_sync(mask, hg);
-  hx = __reduce_max_sync(mask, hx);
+  hg = team_max<QH>(team, hg);
+  hx = team_max<QH>(team, hx);
   const int eg = fx_exp(hg) + 1, ex = fx_exp(hx);        // the weights stay below 2^60
 #pragma unroll
   for (int s2 = 0; s2 < QH; ++s2) Gs[u + QH * s2] = fx_split(fx_from(Y[s2], eg));
@@ -258,7 +258,7 @@ __device__ __forceinline__ void adj_mass_body(const Basis<NU, NV> &B, const Fiel
   __syncwarp(mask);
   const double one = fx_finite(hg) && fx_finite(hx) ? 1.0 : __longlong_as_double(0x7ff8000000000000LL);
   const int k0 = (ex - FX_BIAS) + (eg - FX_BIAS);
-  team_K_fx<NU, NV>(B, Gs, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs),
+  team_K_fx<NU, NV>(B, Gs, team, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs),
                     [&](int j, int k, i64 y, int ey) {
                       if (k < NE) A.gv[e + Eu * k] = fx_scale((double)y * one, k0 + ey) + A.gv[e + Eu * k];
                     });

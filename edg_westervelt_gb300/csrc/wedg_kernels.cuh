@@ -550,6 +550,7 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
   const int r = lane - tw * NU, slot = (threadIdx.x >> 5) * T::TPW + tw, e = e0 + slot;
   if (e >= E) return;
   const unsigned mask = ((1u << NU) - 1u) << (tw * NU);
+  const Team team{mask, tw * NU, r};
   const size_t Eu = (size_t)E;
   const bool has_v = r < NV, modal = F.modal != 0;
   double *Us = sh + slot * T::SLOT, *Vs = Us + NU * NU;
@@ -596,8 +597,8 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
       ends(de, d_o, true, lo[2][ax], hi[2][ax]);
     }
   }
-  hu = __reduce_max_sync(mask, hu);
-  hv = __reduce_max_sync(mask, hv);
+  hu = team_max<NU>(team, hu);
+  hv = team_max<NU>(team, hv);
   i64 *Gi = reinterpret_cast<i64 *>(F.G);
   if (r == 0) Gi[(size_t)(QH * QH + 1) * E + e] = (i64)hu << 32 | hv;
   const int N = F.N, j = e % N, k = e / N;
@@ -662,8 +663,8 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
   for (int q = r; q < QH; q += NU)
 #pragma unroll
     for (int s2 = 0; s2 < QH; ++s2) hb = max(hb, fx_abs_hi(F.beta2[(q + QH * s2) * Eu + e]));
-  hb = __reduce_max_sync(mask, hb);
-  hv = max(hv, __reduce_max_sync(mask, r == 0 ? fx_abs_hi(V[0]) : 0));
+  hb = team_max<NU>(team, hb);
+  hv = max(hv, __shfl_sync(mask, fx_abs_hi(V[0]), team.lane0));   // with the constant mode
   const bool nan = !fx_finite(hv) || !fx_finite(hb);
   const int ev = fx_exp(hv), eb = fx_exp(hb) + 2;
   Fx2 x[NV];
@@ -677,7 +678,7 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
   // the rows T = Ph V go up by nt, the room that Σ_a max|Ph[.][a]| |V[a][b]| leaves in every column, so that
   // v_q has the bits which the levels' headroom for any V would take (top 2^12 bounds the high words
   // of T 2^(61 - gPh))
-  const int nt = max(__clz(__reduce_max_sync(mask, top)) - 3 - 12 + (61 - B.gPh), 0);
+  const int nt = max(__clz(team_max<NU>(team, top)) - 3 - 12 + (61 - B.gPh), 0);
   const int sG = (ev - FX_BIAS) + 2 * (61 - B.gPh) - nt + (eb - FX_BIAS) + 61;   // G = (integer) 2^sG
   Fx2 *Ts = reinterpret_cast<Fx2 *>(Us);                 // T[q][b] at Ts[q NV + b]
   __syncwarp(mask);                                      // the sums are spent
@@ -716,14 +717,8 @@ __device__ __forceinline__ void prep_body(const Basis<NU, NV> &B, const Fields &
     if constexpr ((QH & 1) != 0)
       point(fx_dot<0, 2, NV>(tb, [&](int b) -> const FxC & { return B.fPh[QH / 2][b]; }), QH / 2);
   }
-  // the extrema over the team: the high words, then the low words of those that have it
-  {
-    const int h1 = __reduce_max_sync(mask, (int)(kmax >> 32)), h0 = __reduce_min_sync(mask, (int)(kmin >> 32));
-    const unsigned l1 = __reduce_max_sync(mask, (int)(kmax >> 32) == h1 ? (unsigned)kmax : 0u);
-    const unsigned l0 = __reduce_min_sync(mask, (int)(kmin >> 32) == h0 ? (unsigned)kmin : ~0u);
-    kmax = (i64)((u64)(unsigned)h1 << 32 | l1);
-    kmin = (i64)((u64)(unsigned)h0 << 32 | l0);
-  }
+  kmax = team_max<NU>(team, kmax);
+  kmin = team_min<NU>(team, kmin);
   if (r != 0) return;
   Gi[(size_t)QH * QH * E + e] = GPack(nan ? GPack::BAD : sG, kmin, kmax).word();
   if (F.cg) return;                                      // (k_cg finds a matrix that is not positive definite)
@@ -897,13 +892,15 @@ __host__ __device__ constexpr int mass_tile(int nu, int nv, int threads) {
 // what the norms leave in every case (nrow), and the last level takes the products of the low halves too: the
 // shifts would cost a tenth of such a product.
 template <int NU, int NV, class Use>
-__device__ __forceinline__ void team_K_fx(const Basis<NU, NV> &B, const Fx2 *Gs, int u, int lane0, unsigned mask,
-                                          const Fx2 *Phs, const Fx2 *PhWs, const Fx2 *xs, Fx2 *zs, const Use &use) {
+__device__ __forceinline__ void team_K_fx(const Basis<NU, NV> &B, const Fx2 *Gs, const Team &team, const Fx2 *Phs,
+                                           const Fx2 *PhWs, const Fx2 *xs, Fx2 *zs, const Use &use) {
   using T = MassTeam<NU, NV>;
   constexpr int QH = T::QH, HP = T::HP, NE = T::NE, J = T::J, NP = (NV + 1) / 2;
   constexpr bool RISE = NV >= 4;
+  const int u = team.u;
+  const unsigned mask = team.mask;
   const bool high = u >= HP;                             // the mirror of a lower row
-  const int low = high ? QH - 1 - u : u, mate = lane0 + (QH - 1 - u);
+  const int low = high ? QH - 1 - u : u, mate = team.lane0 + (QH - 1 - u);
   // row u of P_h d: the thread of the lower row sums the even modes, its mirror the odd ones
   i64 Tv[NV];
   {
@@ -967,7 +964,7 @@ __device__ __forceinline__ void team_K_fx(const Basis<NU, NV> &B, const Fx2 *Gs,
       hz |= fx_hi(Z[b]);
     }
     // the rows' common exponent, below 2^60 for the sums of pairs
-    nz = RISE ? __reduce_min_sync(mask, nt + fx_room(hz)) - 1 : B.nrow;
+    nz = RISE ? team_min<QH>(team, nt + fx_room(hz)) - 1 : B.nrow;
 #pragma unroll
     for (int b = 0; b < NV; ++b) Z[b] = fx_shift(Z[b], nz - nt);
   }
@@ -1051,6 +1048,7 @@ _Pragma("unroll") \
   const int u = lane - tw * QH, lane0 = tw * QH, slot = (threadIdx.x >> 5) * T::TPW + tw, g = (g0) + slot; \
   if (g >= F.E) return; \
   const unsigned mask = ((1u << QH) - 1u) << lane0; \
+  const Team team{mask, lane0, u}; \
   const size_t Eu = (size_t)F.E;
 
 template <int NU, int NV>
@@ -1077,7 +1075,7 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
   if (n > 1)
 #pragma unroll
     for (int s2 = 0; s2 < QH; ++s2) Gs[u + QH * s2] = fx_split(G[(u + QH * s2) * Eu] << gp.ng);
-  hr = __reduce_max_sync(mask, hr);
+  hr = team_max<QH>(team, hr);
   bool fin = true;
   const double ith = 1.0 / th;
   if (n == 1 || !fx_finite(hr)) {                  // (one step is R/θ)
@@ -1125,7 +1123,7 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
       // (a half unit of bias a step would add up: r moved down goes toward -∞, and so does what is taken from it)
       const int half_p = sr < 0 ? 0 : 1 << 27;
       int hr1 = 0;
-      team_K_fx<NU, NV>(B, Gs, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs), [&](int j, int k, i64 y, int ey) {
+      team_K_fx<NU, NV>(B, Gs, team, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs), [&](int j, int k, i64 y, int ey) {
         const int sy = gp.sG - gp.ng + ey + sd;
         const Fx2 t = fx_split((i64)((u64)fx_shift(fx_join(xf[k]), sd) - (u64)fx_shift(y, sy)));
         const i64 m = fx_mad(t.h, ithf.l, fx_mad(t.l, ithf.h, half_p));
@@ -1148,7 +1146,7 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
       }
       // the room of both (|r| ≤ 2^61, |d'| < 2^61 at the exponent n1 - 2), as far as 14 bits, from the ors of the
       // high words' upper halves
-      const unsigned w = __reduce_or_sync(mask, (unsigned)hd >> 15 | (unsigned)hr1 >> 15 << 16);
+      const unsigned w = team_or<QH>(team, (unsigned)hd >> 15 | (unsigned)hr1 >> 15 << 16);
       const int ud = max(__clz(w & 0xffff) - 18, 0);
       ur = __clz(w >> 16) - 18;
       nr = n1;
@@ -1180,7 +1178,7 @@ __device__ __forceinline__ void cheb_body(const Basis<NU, NV> &B, const Fields &
 #pragma unroll
         for (int j = 0; j < J; ++j)
           if (u + QH * j < NE) hX = max(hX, fx_hi(Xf[u + QH * j]));
-        bX = __reduce_max_sync(mask, hX) + 1;
+        bX = team_max<QH>(team, hX) + 1;
         if (bX > 1u << 29) {
 #pragma unroll
           for (int j = 0; j < J; ++j)
@@ -1243,7 +1241,7 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
     int hx = 0;
 #pragma unroll
     for (int j = 0; j < J; ++j) hx = max(hx, fx_abs_hi(x[j]));
-    hx = __reduce_max_sync(mask, hx);
+    hx = team_max<QH>(team, hx);
     const int ex = fx_exp(hx);
 #pragma unroll
     for (int j = 0; j < J; ++j) {
@@ -1254,7 +1252,7 @@ __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F,
     __syncwarp(mask);
     const double one = g_ok && fx_finite(hx) ? 1.0 : __longlong_as_double(0x7ff8000000000000LL);
     const int k0 = ex - FX_BIAS + (g_ok ? gp.sG - gp.ng : 0);
-    team_K_fx<NU, NV>(B, Gs, u, lane0, mask, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs),
+    team_K_fx<NU, NV>(B, Gs, team, Phf, PhWf, xf, reinterpret_cast<Fx2 *>(zs),
                       [&](int j, int, i64 v, int ey) { y[j] = fx_scale((double)v * one, k0 + ey); });
     __syncwarp(mask);
   };

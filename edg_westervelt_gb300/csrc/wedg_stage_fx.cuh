@@ -157,6 +157,7 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
   const int e = e0 + slot, E = F.E, N = F.N;
   if (e >= E) return;
   const unsigned mask = ((1u << NU) - 1u) << (tw * NU);
+  const Team team{mask, tw * NU, c};
   const size_t Eu = (size_t)E;
   const bool usolve = S.mode == OUT_ADJ_USOLVE, volume = S.mode == OUT_ADJ_VOLUME;
   const double nan = __longlong_as_double(0x7ff8000000000000LL);
@@ -182,7 +183,7 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
     const int kc = B.kK1[c];
 #pragma unroll
     for (int a = 0; a < NU; ++a) top = max(top, fx_hi(w[a]) >> (kmax - max(k1_bits<NU>(a), kc)));
-    const int room = fx_room(__reduce_max_sync(mask, top) + 1);
+    const int room = fx_room(team_max<NU>(team, top) + 1);
     s += kmax - room + 61 - B.gK1;
     // the entry of a contraction over its mode m: W 2^(k_m - kmax + room)
     auto scaled = [&](i64 v, int m) {
@@ -227,7 +228,7 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
       d[a] = a + c > 0 ? S.xu[e + Eu * (a + NU * c)] : 0.0;
       hx = max(hx, fx_abs_hi(d[a]));
     }
-    hx = __reduce_max_sync(mask, hx);
+    hx = team_max<NU>(team, hx);
     ok = fx_finite(hx);
     const int ex = fx_exp(hx);
     sX = ex - FX_BIAS;
@@ -251,8 +252,8 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
     } else {
 #pragma unroll
       for (int a = 0; a < NU; ++a) { hu = max(hu, fx_abs_hi(du[a])); hv = max(hv, fx_abs_hi(dv[a])); }
-      hu = __reduce_max_sync(mask, hu);
-      hv = __reduce_max_sync(mask, hv);
+      hu = team_max<NU>(team, hu);
+      hv = team_max<NU>(team, hv);
     }
     ok = fx_finite(hu) && fx_finite(hv);
     const int eu = fx_exp(hu), ev = fx_exp(hv);
@@ -349,9 +350,9 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
       hd = max(hd, fx_abs_hi(D[s]));
       hf = max(hf, fx_abs_hi(Fo[s]));
     }
-    ha = __reduce_max_sync(mask, ha);
-    hd = __reduce_max_sync(mask, hd);
-    hf = __reduce_max_sync(mask, hf);
+    ha = team_max<NU>(team, ha);
+    hd = team_max<NU>(team, hd);
+    hf = team_max<NU>(team, hf);
     ok = ok && fx_finite(ha) && fx_finite(hd) && fx_finite(hf);
     const int ea = fx_exp(ha) + 1, ed = fx_exp(hd) + 1, ef = fx_exp(hf) + 1;
     // ---- lifts (src/rhs.jl:421-473). The two sides of an axis are lifted together: with σ_a = (-1)^a the
@@ -467,7 +468,7 @@ __device__ __forceinline__ void stage_fast_body(const Basis<NU, NV> &B, const Fi
   }
   // Each product leaves dQ bits of headroom for sums that an orthonormal Q seldom has: over the four of them eight
   // bits, so that 52 were left. The room there is after two is taken back (2^sX stays far from subnormal)
-  const int up = min(fx_room(__reduce_or_sync(mask, top)), max(sX + 960, 0));
+  const int up = min(fx_room(team_or<NU>(team, top)), max(sX + 960, 0));
   sX -= up;
   __syncwarp(mask);
 #pragma unroll

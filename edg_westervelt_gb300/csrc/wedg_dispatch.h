@@ -40,7 +40,7 @@ typedef void (*adj_face_fn)(const void *basis, const Fields &F, const StageIO &S
                             double *gal, double *gbe, cudaStream_t st);
 
 // Multi-instance launches (wedg_kernels.cuh): `grid` blocks (0: one per virtual block) of
-// `threads` threads; the caller sets P.tile to the kernel's elements per block (k_prep: threads,
+// `threads` threads; the caller sets P.tile to the kernel's elements per block (k_prep: prep_tile,
 // k_bnd: bnd_tile sides, k_stage: stage_tile, the mass solves: (threads / 32) teams per warp)
 typedef cudaError_t (*multi_fn)(const void *basis, const MultiStage &P, int grid, int threads,
                                 cudaStream_t st);
@@ -76,16 +76,15 @@ const Basis<NU, NV> &basis_of(const void *basis) {
   return *static_cast<const Basis<NU, NV> *>(basis);
 }
 
-// Launches k after the kernel before it on the stream. Up to LAUNCH_EARLY elements the launch itself is
-// already under way while that kernel runs, and k's threads wait for its end on the device (after_previous),
-// which saves most of the gap between two kernels: N = 32 2.71 -> 2.40 ms and N = 64 25.1 -> 22.9 ms for their
-// runs, 1-2 % at N = 256 to 333. At N = 512 the gaps are below 1 % and it measured 0.5 % slower; the kernels of
+// Launches k after the kernel before it on the stream. With `early` the launch itself is already under way while that
+// kernel runs, and k's threads wait for its end on the device (after_previous), which saves most of the gap between
+// two kernels, at every size: two RK4 steps at q = 2 and 6, N = 364 2 198 -> 2 141 and 9 360 -> 9 300 us, N = 512 3 950
+// -> 3 895 and 17 720 -> 17 662 us; N = 32 2.71 -> 2.40 ms and N = 64 25.1 -> 22.9 ms for their runs. The kernels of
 // several instances, which fill the chip, gained nothing.
 // (Letting k's blocks onto the SMs as well, before the kernel before it has ended, was better at N = 32 alone:
 // they spread unevenly over the SMs that happen to have room; N = 128 adjoint 4 % slower.)
-constexpr int LAUNCH_EARLY = 1 << 17;
 template <class... P, class... A>
-cudaError_t launch_after(void (*k)(P...), int E, int grid, int threads, cudaStream_t st, const A &...a) {
+cudaError_t launch_after(void (*k)(P...), bool early, int grid, int threads, cudaStream_t st, const A &...a) {
   static_assert((std::is_same<P, A>::value && ...), "the arguments are passed by address");
   void *args[] = {const_cast<void *>(static_cast<const void *>(&a))...};
   cudaLaunchAttribute at{};
@@ -96,7 +95,7 @@ cudaError_t launch_after(void (*k)(P...), int E, int grid, int threads, cudaStre
   c.blockDim = dim3(threads);
   c.stream = st;
   c.attrs = &at;
-  c.numAttrs = E <= LAUNCH_EARLY ? 1 : 0;
+  c.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelExC(&c, reinterpret_cast<const void *>(k), args);
 }
 
@@ -208,14 +207,14 @@ cudaError_t launch_prep(const void *basis, const Fields &F, const StageIO &S, in
   // (ranges of elements also wait for their copies to the device, and are launched after those)
   const bool all = blocks * prep_tile(NU, threads) >= F.E;
   const int sides = (threads / 32) * bnd_tile(NU), nb = all ? (4 * F.N + sides - 1) / sides : 0;
-  return launch_after(k_prep<NU, NV>, all ? F.E : INT_MAX, nb + blocks, threads, st, basis_of<NU, NV>(basis), F, S,
+  return launch_after(k_prep<NU, NV>, all, nb + blocks, threads, st, basis_of<NU, NV>(basis), F, S,
                       e0, nb);
 }
 
 // k_bnd over the 4N physical sides (the grid follows from F.N), after a k_prep by ranges
 template <int NU, int NV>
 cudaError_t launch_bnd(const void *basis, const Fields &F, const StageIO &S, int, int, cudaStream_t st) {
-  return launch_after(k_bnd<NU, NV>, F.E, (4 * F.N + bnd_tile(NU) - 1) / bnd_tile(NU), BND_THREADS, st,
+  return launch_after(k_bnd<NU, NV>, true, (4 * F.N + bnd_tile(NU) - 1) / bnd_tile(NU), BND_THREADS, st,
                       basis_of<NU, NV>(basis), F, S);
 }
 
@@ -224,7 +223,7 @@ template <int NU, int NV, bool FAST>
 cudaError_t launch_stage(const void *basis, const Fields &F, const StageIO &S, int blocks, int threads,
                          cudaStream_t st) {
   if (blocks <= 0) return cudaSuccess;
-  return launch_after(k_stage<NU, NV, FAST>, F.E, blocks, threads, st, basis_of<NU, NV>(basis), F, S);
+  return launch_after(k_stage<NU, NV, FAST>, true, blocks, threads, st, basis_of<NU, NV>(basis), F, S);
 }
 
 // The mass solve: k_cheb or k_cg, a team of threads per element (static shared memory sized
@@ -238,28 +237,28 @@ cudaError_t launch_mass(const void *basis, const Fields &F, const StageIO &S, in
   threads = (threads >= 32 && threads <= CHEB_THREADS && threads % 32 == 0) ? threads : CHEB_THREADS;
   const int tpb = mass_tile(NU, NV, threads);
   const int grid = (F.E + tpb - 1) / tpb;
-  if (F.cg) return launch_after(k_cg<NU, NV>, F.E, grid, threads, st, B, F, S);
-  return launch_after(k_cheb<NU, NV>, F.E, grid, threads, st, B, F, S);
+  if (F.cg) return launch_after(k_cg<NU, NV>, true, grid, threads, st, B, F, S);
+  return launch_after(k_cheb<NU, NV>, true, grid, threads, st, B, F, S);
 }
 
 // The adjoint kernels (wedg_adjoint.cuh)
 template <int NU, int NV>
 void launch_adj_hats(const void *basis, const Fields &F, const StageIO &, const AdjIO &A, cudaStream_t st) {
-  launch_after(k_adj_hats<NU, NV>, F.E, (F.E + HATS_THREADS - 1) / HATS_THREADS, HATS_THREADS, st,
+  launch_after(k_adj_hats<NU, NV>, true, (F.E + HATS_THREADS - 1) / HATS_THREADS, HATS_THREADS, st,
                basis_of<NU, NV>(basis), F, A);
 }
 template <int NU, int NV>
 void launch_adj_mass(const void *basis, const Fields &F, const StageIO &, const AdjIO &A, cudaStream_t st) {
   constexpr int tpb = mass_tile(NU, NV, CHEB_THREADS);
-  launch_after(k_adj_mass<NU, NV>, F.E, (F.E + tpb - 1) / tpb, CHEB_THREADS, st, basis_of<NU, NV>(basis), F, A);
+  launch_after(k_adj_mass<NU, NV>, true, (F.E + tpb - 1) / tpb, CHEB_THREADS, st, basis_of<NU, NV>(basis), F, A);
 }
 template <int NU, int NV>
 void launch_adj_face(const void *basis, const Fields &F, const StageIO &S, const AdjIO &A, double *gc2, double *gal,
                      double *gbe, cudaStream_t st) {
   const Basis<NU, NV> &B = *static_cast<const Basis<NU, NV> *>(basis);
   const int grid = (F.E + adj_tile(NU) - 1) / adj_tile(NU);
-  if (gc2) launch_after(k_adj_face<NU, NV, true>, F.E, grid, ADJ_THREADS, st, B, F, S, A, gc2, gal, gbe);
-  else launch_after(k_adj_face<NU, NV, false>, F.E, grid, ADJ_THREADS, st, B, F, S, A, gc2, gal, gbe);
+  if (gc2) launch_after(k_adj_face<NU, NV, true>, true, grid, ADJ_THREADS, st, B, F, S, A, gc2, gal, gbe);
+  else launch_after(k_adj_face<NU, NV, false>, true, grid, ADJ_THREADS, st, B, F, S, A, gc2, gal, gbe);
 }
 
 template <int NU, int NV>

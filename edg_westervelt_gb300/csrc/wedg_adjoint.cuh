@@ -402,7 +402,7 @@ __device__ __forceinline__ void boundary_coef_partials(const Fields &F, int s, c
 // by mode parity): those of B and T on the thread's column, those of L and R on its row.
 //
 // What bounds it: the FP64 pipe, at 12 NU operations a thread for the sums over the points, and the points'
-// own (25, with PARAMS 50, a side): 56 % of the pipe over the launch, 78 % while blocks are there (683 blocks are
+// own (25, with PARAMS 50, a side): 55 % of the pipe over the launch, 78 % while blocks are there (683 blocks are
 // 4.5 an SM at N = 128). N = 128, q = 4, with PARAMS, cold caches: 188 us with a thread per element, 128 us so.
 template <int NU, int NV, bool PARAMS>
 __device__ __forceinline__ void adj_face_body(const Basis<NU, NV> &B, const Fields &F, const StageIO &S,

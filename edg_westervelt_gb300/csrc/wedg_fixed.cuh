@@ -1,10 +1,11 @@
 // 64-bit fixed-point arithmetic for the contractions of the stage kernels.
 //
-// The FP64 pipe of sm_103a issues 1.9 lanes per clock and SM (585 G DFMA/s measured over the chip);
-// the integer multiply-add with a 64-bit sum (mad.wide.s32) runs at 16 200 G/s beside it, at the
-// same time. A product of two 62-bit integers costs three of them, so a contraction with constants
-// runs about six times faster here, the combination of the partial sums included, and carries 60
-// bits where a double carries 53.
+// The FP64 pipe of sm_103a issues 2 lanes per clock and SM (628 G DFMA/s measured over the chip: eight chains
+// a thread, 64 warps an SM, 2 070 MHz), 64 cycles a warp and scheduler; the integer multiply-add with a 64-bit sum
+// (mad.wide.s32) takes 2.04 (19 780 G/s, the same probe), at the same time. A product of two 62-bit
+// integers costs three of them, a tenth of an FP64 one; the sums, shifts and splits around it are work of the
+// ALU. A block keeps 61 bits of its largest number where doubles keep 53 of each: a number 2^-k of the largest
+// has 61 - k.
 //
 // A block of numbers shares one exponent: x = X 2^s with |X| < 2^61, from the largest number of the
 // block (fx_from). Numbers and constants are used in balanced halves, X = h 2^32 + l with l in

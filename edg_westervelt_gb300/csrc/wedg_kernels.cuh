@@ -6,11 +6,11 @@
 // a scheduler's pipe for 64 cycles) while the integer pipes stand idle beside
 // it. So the contractions over modes and points, which are most of the work,
 // run in 64-bit fixed point with one exponent per element (wedg_fixed.cuh:
-// three integer multiply-adds of 4 cycles for an FP64 one, and more bits), and
+// three integer multiply-adds of 2 cycles for an FP64 one), and
 // the fluxes, sources, inner products and updates in FP64. A team of threads
 // shares an element: thread r has column or row r of its modal blocks or point
 // r of its sides, and blocks change hands through shared memory. That spreads
-// small meshes over the chip and keeps the registers low enough for 24 to 32
+// small meshes over the chip and keeps the registers low enough for 20 to 48
 // warps an SM.
 //
 // One RHS evaluation is three kernels:
@@ -516,7 +516,7 @@ __device__ __forceinline__ int cheb_count(double L, double th, double de) {
 //
 // What bounds it: the FP64 pipe (60 %: the traces, and a conversion per entry of V and 2β) and the latency of
 // its loads. N = 512, q = 6: 760 us as FP64 code with a thread per element; 526, 488, 458 and 442 us so at four, five,
-// six and eight blocks an SM (64 registers), the last with the physical sides 445, and 436 with them in its own blocks.
+// six and eight blocks an SM (64 registers), the last with the physical sides 445, and 435 with them in its own blocks.
 template <int NU, int NV>
 struct PrepTeam {
   static constexpr int QH = qhigh(NU, NV), TPW = 32 / NU;
@@ -862,11 +862,11 @@ __device__ __forceinline__ void store_v(const StageIO &S, size_t l, double kk, b
 // 49 bits were left at ε close to 1, and systems beyond ε = 31/32 took a form in FP64.)
 //
 // What bounds it: one product with M costs about 1 300 multiply-adds an element at q = 6, three integer
-// ones each (4 cycles a warp), and 18 shared-memory words a thread; a thread per row keeps 24 warps an SM
+// ones each (2 cycles a warp) and as much again on the ALU, and 18 shared-memory words a thread: both pipes are 57 to
+// 60 % busy where every element takes 29 steps. A thread per row keeps 20 to 24 warps an SM
 // where a thread per pair of rows (half the exchanges, 16 warps) left the pipes waiting.
-// N = 512, q = 6, a front (3.5 steps on average): 2 569 us in FP64, 1 004 us in fixed point with a thread per
-// pair of rows, 878 us so; at five and eight blocks an SM 875 and 998. N = 300, q_v = 7, 27 steps: 12 850 us
-// in FP64, 4 705 us so (4 565 and 4 908).
+// N = 512, q = 6, a front (3.6 steps on average): 2 569 us in FP64, 890 us so (1 004 us with a thread per
+// pair of rows). N = 300, q_v = 7, 27 steps: 12 850 us in FP64, 4 620 us so. N = 333, q = 2, 19 steps: 282 us.
 template <int NU, int NV>
 struct MassTeam {
   static constexpr int QH = qhigh(NU, NV);
@@ -1222,7 +1222,7 @@ __device__ __forceinline__ double team_sum(double x, int u, int lane0, unsigned 
 // team layout of k_cheb: the products with K in fixed point on p as integers of its own exponent, the
 // vectors and inner products in FP64, summed over the team's lanes in a fixed order so that every lane
 // takes the same decisions. A chain of products and reductions bounds it, with three blocks an SM to hide
-// it. N = 97, q = 5: 405 us with FP64 products of half as many threads, 138 us so (and 11 us for the integers
+// it. N = 97, q = 5: 405 us with FP64 products of half as many threads, 137 us so (and 11 us for the integers
 // of G, which k_prep writes).
 template <int NU, int NV>
 __device__ __forceinline__ void cg_body(const Basis<NU, NV> &B, const Fields &F, const StageIO &S, int g0) {

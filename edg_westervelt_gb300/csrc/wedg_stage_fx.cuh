@@ -10,7 +10,8 @@
 // which keeps about 700 operations: the slots, one conversion per output and the updates. The team
 // keeps the registers low enough for 24 warps an SM and spreads small meshes over the chip.
 // N = 512, q = 6: 1 499 us as FP64 code with a thread per element, 1 108 us in fixed point so, 844 us by teams at
-// six blocks an SM (980 and 878 at four and five); N = 64, q = 4: 87 and 26 us.
+// six blocks an SM (980 and 878 at four and five), 852 us with the room taken back in the u-solve; N = 64, q = 4: 87
+// and 26 us.
 //
 // With Cw = c²W, Aw = αW, the 1D stiffness K1 = S^T diag(w) S and the orthonormal basis
 //   (c²∇φ_v,∇u_h) + (α∇φ_v,∇v_h) = (K1 W + W K1)[v-block] / (-4/h²),  W = -(4/h²)(c² U + α V),

@@ -12,8 +12,9 @@
  *
  * Conventions
  *  - States, coefficients and results are FP64. The contractions over modes and points run in 64-bit
- *    fixed point with one exponent per element, the rest in FP64: results are as close to 64-bit
- *    dense algebra as FP64 sums are.
+ *    fixed point with one exponent per block of an element, the rest in FP64. In the norm of a block, results
+ *    are as close to 64-bit dense algebra as FP64 sums are; entries far below the largest of their block
+ *    (2^-8 and less) have fewer bits than a double.
  *  - Status codes mirror the reference's exceptions (wedg_status); the exact
  *    message text of the reference is available from wedg_error_message.
  *  - State arrays u (N,N,q_u+1,q_u+1) and v (N,N,q_v+1,q_v+1) use the
